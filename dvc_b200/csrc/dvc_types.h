@@ -10,9 +10,8 @@ namespace dvc {
 // Derived from the reference's ladder tables (ReadLdpcaLadderFile_LdpcaDecoder.cpp:150-201):
 // per code c the syndrome length m_c = (n/period)*bpp[c], its rate m_c/n, the
 // row of every edge, plus layouts this decoder adds for parallel BP: per code
-// the row-order positions of the edges (each row's edges contiguous, in
-// increasing edge order, so that row sums keep the reference's summation
-// order), the CRC-8 contribution of each single source bit, and the GF(2)
+// the storage position and row slot of every edge (below), the CRC-8
+// contribution of each single source bit, and the GF(2)
 // inverse of the full-rate matrix with bit i of row j at word i/32, bit i%32.
 struct LadderDev {
   int n, e, period, num_codes, invh_words;
@@ -21,12 +20,16 @@ struct LadderDev {
   const int *idx;         // [num_codes*period]
   const int *synd_len;    // [num_codes]
   const float *code_rate; // [num_codes]
-  const int *row_ptr;     // [num_codes*(n+1)] first row-order position of each row
-  // Edges are numbered column-major (edge e = 3k + i is the i-th edge of column
-  // k, every column has degree 3); row-order position p lists each row's edges
-  // in increasing e, rows in order.
-  const uint16_t *pos;       // [num_codes*e] row-order position of edge e
-  const uint16_t *rid;       // [num_codes*e] row of row-order position p
+  // Rows of a code are decoded in slot order: sorted by degree, largest first
+  // (ties in row order), 32 slots to a group, one group to a warp.  The edge
+  // messages of group g are stored transposed: edge i (in increasing edge
+  // order) of the row in lane l at position base + i * width + l, width = the
+  // rows of the group (32 but for the last), so a warp reads its rows without
+  // bank conflicts.  Rows shorter than the group's first are padded.
+  int pos_max;               // positions of the largest code, padding included (multiple of 4)
+  const uint32_t *edge;      // [num_codes*3*n] edge 3k + i of column k at [(3*code + i)*n + k]: position | slot << 16
+  const uint32_t *grp;       // [num_codes*ceil(n/32)] base | edges of its longest row << 16
+  const uint16_t *slot_row;  // [num_codes*n] row of each slot
   const uint16_t *ir_full;   // [e] row of edge e in the full-rate code (the encoder's matrix)
   const uint8_t *crc_tab;    // [n]
   const uint32_t *invh;      // [n*invh_words]

@@ -59,14 +59,13 @@ __device__ void pack_bits(const G &g, const uint8_t *dec, int n, uint32_t *out) 
 // every thread of the group
 template <class G, int MAXC>
 __device__ void finalise(const G &g, const LdpcaBatch &A, const LadderDev &L, int j, int acc, const LdSmem &S,
-                         uint32_t *s_ured, int *s_flag, const uint4 *pdesc) {
+                         uint32_t *s_ured, LdCtl *ctl, const uint4 *pdesc) {
   const LdpcaBatchCw &C = A.cw[j];
   LdpcaBatchState &st = A.state[j];
   const int n = L.n, last = L.num_codes - 1, start = st.start;
+  int *s_flag = &ctl->flag;
   if (acc == last) {
-    ld_build_syndrome(g, L, last, S.accs, S.rpar);
-    g.sync();
-    ld_invh_decode(g, L, S.rpar, S.dec, reinterpret_cast<uint32_t *>(S.msg));
+    ld_full_rate(g, L, S);
   } else {
     if (g.t == 0) {
       int slot = -1;
@@ -87,7 +86,8 @@ __device__ void finalise(const G &g, const LdpcaBatch &A, const LadderDev &L, in
       float llr[MAXC];
       ld_llr(g, n, A.lr + C.lr_off, A.xt, xs, llr, nullptr, nullptr);
       int it = 0;
-      ld_try_code(g, L, acc, llr, C.crc, A.xt, pdesc, A.max_iter, nullptr, S, s_ured, s_flag, it);
+      uint32_t dm = 0;
+      ld_try_code(g, L, acc, llr, C.crc, A.xt, pdesc, A.max_iter, nullptr, S, s_ured, ctl, it, dm);
     }
     g.sync();
   }
@@ -108,10 +108,11 @@ __device__ void finalise(const G &g, const LdpcaBatch &A, const LadderDev &L, in
 // one (codeword, code) item
 template <class G, int MAXC>
 __device__ void run_item(const G &g, const LdpcaBatch &A, const LadderDev &L, int j, int code,
-                         const LdSmem &S, uint32_t *s_ured, int *s_flag, const uint4 *pdesc) {
+                         const LdSmem &S, uint32_t *s_ured, LdCtl *ctl, const uint4 *pdesc) {
   const LdpcaBatchCw &C = A.cw[j];
   LdpcaBatchState &st = A.state[j];
   const int n = L.n, last = L.num_codes - 1;
+  int *s_flag = &ctl->flag;
   const int start = st.start;
   const XlSmall xs = xl_small_global(A.xt);
   float llr[MAXC];
@@ -119,7 +120,8 @@ __device__ void run_item(const G &g, const LdpcaBatch &A, const LadderDev &L, in
   ld_stage_acc(g, A.acc + C.acc_off, n, S.accs);
   g.sync();
   int it = 0;
-  const int ok = ld_try_code(g, L, code, llr, C.crc, A.xt, pdesc, A.max_iter, &st.best, S, s_ured, s_flag, it);
+  uint32_t dm = 0;
+  const int ok = ld_try_code(g, L, code, llr, C.crc, A.xt, pdesc, A.max_iter, &st.best, S, s_ured, ctl, it, dm);
   if (g.t == 0) {
     st.iters[code - start] = it;
     atomicAdd(A.work, (unsigned long long)it);
@@ -157,7 +159,7 @@ __device__ void run_item(const G &g, const LdpcaBatch &A, const LadderDev &L, in
   g.sync();
   const int acc = *s_flag;
   g.sync();
-  if (acc >= 0) finalise<G, MAXC>(g, A, L, j, acc, S, s_ured, s_flag, pdesc);
+  if (acc >= 0) finalise<G, MAXC>(g, A, L, j, acc, S, s_ured, ctl, pdesc);
 }
 
 // next valid item of a queue (one thread): codeword index in the high bits, code in the low 8; -1 when empty
@@ -214,7 +216,7 @@ __global__ void __launch_bounds__(256) ldpca_batch_prep_kernel(LdpcaBatch A) {
     uint8_t *synd = smem;
     uint32_t *sw = reinterpret_cast<uint32_t *>(smem + ((n + 15) & ~15));
     uint8_t *dec = smem + ((n + 15) & ~15) + 4 * ((n + 31) / 32) + 16;
-    const LdGroup<256, true> g{(int)threadIdx.x, 0};
+    const LdGroup<256, true> g{(int)threadIdx.x, 0, 0};
     ld_build_syndrome(g, L, L.num_codes - 1, A.acc + C.acc_off, synd);
     g.sync();
     ld_invh_decode(g, L, synd, dec, sw);
@@ -236,34 +238,35 @@ __global__ void __launch_bounds__(256) ldpca_batch_prep_kernel(LdpcaBatch A) {
 __global__ void __launch_bounds__(1024, 1) ldpca_batch_kernel(LdpcaBatch A) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ uint32_t s_ured[32];
-  __shared__ int s_flag[4], s_item[4];
+  __shared__ LdCtl s_ctl[4];
+  __shared__ int s_item[4];
   __shared__ uint4 s_pdesc[XL_PHI_MAX_BINADES];
   xl_phi_stage(A.xt, s_pdesc);
   __syncthreads();
   {
-    const LdGroup<1024, true> g{(int)threadIdx.x, 0};
-    const LdSmem S = ld_carve(smem, A.L_cif.n, A.L_cif.e);
+    const LdGroup<1024, true> g{(int)threadIdx.x, 0, 0};
+    const LdSmem S = ld_carve(smem, A.L_cif);
     for (;;) {
       if (g.t == 0) s_item[0] = A.n_cif ? pop_item(A, 0) : -1;
       g.sync();
       const int item = s_item[0];
       g.sync();
       if (item < 0) break;
-      run_item<LdGroup<1024, true>, 7>(g, A, A.L_cif, item >> 8, item & 0xff, S, s_ured, &s_flag[0], s_pdesc);
+      run_item<LdGroup<1024, true>, 7>(g, A, A.L_cif, item >> 8, item & 0xff, S, s_ured, &s_ctl[0], s_pdesc);
     }
   }
   {
     const int gi = threadIdx.x >> 8;
-    const LdGroup<256, false> g{(int)threadIdx.x & 255, 1 + gi};
-    const size_t quarter = ldpca_smem_bytes(A.L_qcif.n, A.L_qcif.e);
-    const LdSmem S = ld_carve(smem + gi * quarter, A.L_qcif.n, A.L_qcif.e);
+    const LdGroup<256, false> g{(int)threadIdx.x & 255, 1 + gi, 0};
+    const size_t quarter = ldpca_smem_bytes(A.L_qcif.n, A.L_qcif.pos_max);
+    const LdSmem S = ld_carve(smem + gi * quarter, A.L_qcif);
     for (;;) {
       if (g.t == 0) s_item[gi] = A.n_qcif ? pop_item(A, 1) : -1;
       g.sync();
       const int item = s_item[gi];
       g.sync();
       if (item < 0) break;
-      run_item<LdGroup<256, false>, 7>(g, A, A.L_qcif, item >> 8, item & 0xff, S, s_ured + 8 * gi, &s_flag[gi], s_pdesc);
+      run_item<LdGroup<256, false>, 7>(g, A, A.L_qcif, item >> 8, item & 0xff, S, s_ured + 8 * gi, &s_ctl[gi], s_pdesc);
     }
   }
 }
@@ -273,14 +276,15 @@ size_t ldpca_batch_state_bytes(int count) {
 }
 
 // dynamic shared memory of a batch block: one CIF codeword, or four QCIF ones
-static size_t batch_smem_bytes() {
-  const size_t cif = ldpca_smem_bytes(6336, 3 * 6336), qcif4 = 4 * ldpca_smem_bytes(1584, 3 * 1584);
+static size_t batch_smem_bytes(const LdpcaBatch &A) {
+  const size_t cif = ldpca_smem_bytes(A.L_cif.n, A.L_cif.pos_max);
+  const size_t qcif4 = 4 * ldpca_smem_bytes(A.L_qcif.n, A.L_qcif.pos_max);
   return cif > qcif4 ? cif : qcif4;
 }
 
 cudaError_t launch_ldpca_batch(LdpcaBatch A, int count, int grid, cudaStream_t s) {
   if (A.L_cif.n != 6336 || A.L_qcif.n != 1584) return cudaErrorInvalidValue;
-  const size_t smem = batch_smem_bytes();
+  const size_t smem = batch_smem_bytes(A);
   static std::atomic<uint64_t> attr_set{0};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);

@@ -8,7 +8,6 @@
 
 namespace dvc {
 
-size_t ldpca_smem_size(int n, int e);
 // direct form: one block per codeword, no scratch
 cudaError_t launch_ldpca(const LadderDev &L, const LdpcaJob *jobs_dev, int num_jobs, const XlmDev &xt,
                          int max_iter, cudaStream_t stream);

@@ -74,61 +74,65 @@ bool load_ladders(const std::string &path, std::vector<LadderHost> &out, std::st
       }
       for (int k = 0; k < b; k++) L.idx[(size_t)c * L.period + k] = tmp[k];
     }
-    // expand the per-code rows: row of edge e in code c is the first kept
-    // accumulated-syndrome position >= its full-rate row
-    L.synd_len.resize(L.num_codes);
-    L.code_rate.resize(L.num_codes);
-    L.ir.resize((size_t)L.num_codes * L.e);
-    L.row_ptr.assign((size_t)L.num_codes * (L.n + 1), 0);
-    L.row_edge.resize((size_t)L.num_codes * L.e);
-    for (int c = 0; c < L.num_codes; c++) {
-      const int b = L.bpp[c];
-      const int m = (L.n / L.period) * b;
-      L.synd_len[c] = m;
-      L.code_rate[c] = (float)m / (float)L.n;  // ReadLdpcaLadderFile_LdpcaDecoder.cpp:182-183
-      std::vector<int> bounds(m);
-      for (int k = 0; k < m; k++) bounds[k] = L.idx[(size_t)c * L.period + k % b] + (k / b) * L.period;
-      int *rp = &L.row_ptr[(size_t)c * (L.n + 1)];
-      for (int e = 0; e < L.e; e++) {
-        int r = (int)(std::lower_bound(bounds.begin(), bounds.end(), L.ir_full[e]) - bounds.begin());
-        if (r >= m) {
-          fclose(f);
-          err = "ladder expansion out of range";
-          return false;
-        }
-        L.ir[(size_t)c * L.e + e] = (uint16_t)r;
-        rp[r + 1]++;
-      }
-      for (int r = 0; r < m; r++) rp[r + 1] += rp[r];
-      for (int r = m; r < L.n; r++) rp[r + 1] = rp[r];
-      std::vector<int> fill(rp, rp + m);
-      for (int e = 0; e < L.e; e++) {
-        const int r = L.ir[(size_t)c * L.e + e];
-        L.row_edge[(size_t)c * L.e + fill[r]++] = (uint16_t)e;
-      }
-    }
-    // the decoder kernel takes every column to have degree 3 (edge e = 3k + i)
-    // and stages the per-code index arrays with 16-byte copies
+    // the decoder kernels take every column to have degree 3 (edge e = 3k + i)
     for (int k = 0; k <= L.n; k++)
       if (L.jc[k] != 3 * k) {
         fclose(f);
         err = "ladder with a column degree other than 3";
         return false;
       }
-    if (L.e % 8 != 0 || L.e > 65535) {
-      fclose(f);
-      err = "ladder edge count not a multiple of 8 or above 65535";
-      return false;
-    }
-    // row-order positions: pos[e] and the row of each position
-    L.pos.resize((size_t)L.num_codes * L.e);
-    L.rid.resize((size_t)L.num_codes * L.e);
-    for (int c = 0; c < L.num_codes; c++)
-      for (int p = 0; p < L.e; p++) {
-        const int e = L.row_edge[(size_t)c * L.e + p];
-        L.pos[(size_t)c * L.e + e] = (uint16_t)p;
-        L.rid[(size_t)c * L.e + p] = L.ir[(size_t)c * L.e + e];
+    // expand the per-code rows: row of edge e in code c is the first kept
+    // accumulated-syndrome position >= its full-rate row; then the BP layout
+    const int gmax = (L.n + 31) / 32;
+    L.synd_len.resize(L.num_codes);
+    L.code_rate.resize(L.num_codes);
+    L.edge.assign((size_t)L.num_codes * L.e, 0u);
+    L.grp.assign((size_t)L.num_codes * gmax, 0u);
+    L.slot_row.assign((size_t)L.num_codes * L.n, 0);
+    for (int c = 0; c < L.num_codes; c++) {
+      const int b = L.bpp[c];
+      const int m = (L.n / L.period) * b;
+      L.synd_len[c] = m;
+      L.code_rate[c] = (float)m / (float)L.n;  // ReadLdpcaLadderFile_LdpcaDecoder.cpp:182-183
+      std::vector<int> bounds(m), row(L.e), deg(m, 0);
+      for (int k = 0; k < m; k++) bounds[k] = L.idx[(size_t)c * L.period + k % b] + (k / b) * L.period;
+      for (int e = 0; e < L.e; e++) {
+        const int r = (int)(std::lower_bound(bounds.begin(), bounds.end(), L.ir_full[e]) - bounds.begin());
+        if (r >= m) {
+          fclose(f);
+          err = "ladder expansion out of range";
+          return false;
+        }
+        row[e] = r;
+        deg[r]++;
       }
+      std::vector<int> order(m), slot(m), fill(m, 0);
+      for (int r = 0; r < m; r++) order[r] = r;
+      std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return deg[x] > deg[y]; });
+      for (int s = 0; s < m; s++) {
+        slot[order[s]] = s;
+        L.slot_row[(size_t)c * L.n + s] = (uint16_t)order[s];
+      }
+      std::vector<int> base((m + 31) / 32);
+      int pos = 0;
+      for (int g = 0; g * 32 < m; g++) {
+        const int width = std::min(32, m - 32 * g), d = deg[order[32 * g]];
+        base[g] = pos;
+        L.grp[(size_t)c * gmax + g] = (uint32_t)pos | ((uint32_t)d << 16);
+        pos += width * d;
+      }
+      if (pos > 65536 || m > 65536) {
+        fclose(f);
+        err = "ladder code too large for 16-bit positions";
+        return false;
+      }
+      L.pos_max = std::max(L.pos_max, (pos + 3) & ~3);
+      for (int e = 0; e < L.e; e++) {
+        const int r = row[e], s = slot[r], g = s >> 5, width = std::min(32, m - 32 * g);
+        const uint32_t p = (uint32_t)(base[g] + fill[r]++ * width + (s & 31));
+        L.edge[((size_t)c * 3 + e % 3) * L.n + e / 3] = p | ((uint32_t)s << 16);
+      }
+    }
     // CRC-8 is linear over GF(2) for a fixed message length (zero initial
     // value, no final xor), so the CRC of a bitplane is the xor of the CRCs
     // of its single set bits.
@@ -243,10 +247,11 @@ bool LadderGpu::upload(const LadderHost &L, std::string &err) {
   dev.period = L.period;
   dev.num_codes = L.num_codes;
   dev.invh_words = L.invh_words;
+  dev.pos_max = L.pos_max;
   return put(allocs, L.jc, &dev.jc, err) && put(allocs, L.bpp, &dev.bpp, err) && put(allocs, L.idx, &dev.idx, err) &&
          put(allocs, L.synd_len, &dev.synd_len, err) && put(allocs, L.code_rate, &dev.code_rate, err) &&
-         put(allocs, L.row_ptr, &dev.row_ptr, err) && put(allocs, L.pos, &dev.pos, err) &&
-         put(allocs, L.rid, &dev.rid, err) && put(allocs, L.ir_full16, &dev.ir_full, err) &&
+         put(allocs, L.edge, &dev.edge, err) && put(allocs, L.grp, &dev.grp, err) &&
+         put(allocs, L.slot_row, &dev.slot_row, err) && put(allocs, L.ir_full16, &dev.ir_full, err) &&
          put(allocs, L.crc_tab, &dev.crc_tab, err) && put(allocs, L.invh, &dev.invh, err);
 }
 

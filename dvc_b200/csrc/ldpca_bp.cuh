@@ -16,23 +16,38 @@
 // same shared memory.  Each thread keeps the log-LRs of its columns
 // (k = t, t + NT, ...) in registers: MAXC = ceil(n / NT) of them.
 //
-// Edge messages are kept in row order (each row's edges contiguous, in
-// increasing edge index), so a row sum is a sequential pass over contiguous
-// shared memory in the reference's summation order; columns (every column has
-// degree 3) reach their edges through the per-code position array.  The
-// parity check of an iteration's hard decision is folded into the next row
-// pass.  The magnitude phi(y) = -logf(tanhf(y)) is one record read of the
-// packed table (dvc_common.cuh), and the reads of a pass are issued in batches
-// so that several are in flight per thread.
+// A codeword may also be shared by a cluster of C thread blocks (C > 1), each
+// taking every C-th group of rows and a contiguous share of the columns; the
+// edge messages live in the shared memory of the block that owns their row and
+// are written there through distributed shared memory.
 //
-// Shared memory per codeword (n bits, e edges; CIF n=6336, e=19008: 125 KB;
-// QCIF a quarter of it):
-//   msg[e]  f32  edge messages by row-order position, in place:
-//                phi(|v->c|) -> c->v -> next phi(|v->c|)
-//   rowt[n] f32  row sums (after decoding: the decoded bits, one byte each)
-//   sgd[e]  u8   bit 0: sign of the v->c message, bit 1: hard decision of its column
-//   rpar[n] u8   bit 0: syndrome bit of the row, bit 1: sign parity of the row
-//   accs[n/8]    the packed accumulated syndrome, staged once per codeword
+// One BP iteration is two passes with a barrier after each:
+//   rows:  the sum of a row's magnitudes in edge order, its sign parity with
+//          the syndrome bit (the sum's sign bit carries it), and whether the
+//          row's check holds for the last hard decision;
+//   edges: a column's thread forms its three incoming messages
+//          phi(row sum - own magnitude), their total, the hard decision and
+//          the three outgoing magnitudes phi(|total - incoming|), with nothing
+//          stored in between.
+// The message of an edge is one float: its magnitude (phi >= 0) with the sign
+// of the message in the sign bit.  A check is tracked by a bit per row that
+// starts as the syndrome bit and is flipped when a column's decision changes
+// (few do after the first iterations), so no decision is stored per edge.
+// What bounds it: each magnitude phi(y) = -logf(tanhf(y)) is one 16-byte record
+// gathered from the packed table (dvc_common.cuh), two per edge and iteration,
+// and an SM takes one random 32-byte sector per cycle from L2 (measured: 1.0
+// cycle per gather for tables up to 64 MB): 38,016 cycles for a CIF codeword.
+// Rows are stored transposed in groups of 32 of similar degree (LadderDev), so
+// the row pass reads without bank conflicts and spends its time on the sums.
+//
+// Shared memory per codeword (n bits, P = pos_max positions; CIF P = 19,072:
+// 102 KB; QCIF 27 KB):
+//   msg[P]    f32  edge messages
+//   rowt[n]   f32  row sums with the parity sign (after decoding: the decoded
+//                  bits, one byte each)
+//   hdr       uint4 per row group: its place, the syndrome bits of its rows,
+//                  the rows whose check fails
+//   accs[n/8]      the packed accumulated syndrome, staged once per codeword
 #pragma once
 #include <cuda_runtime.h>
 
@@ -45,38 +60,103 @@ namespace dvc {
 #define LDPCA_NONE 0x7f7f7f7f      // "no success yet" (memset pattern 0x7f)
 #define LDPCA_MAX_N 6336           // largest codeword length
 
-// columns per thread of a group of nt threads on codewords of n bits
+// rounds (columns per thread) of a group of nt threads on codewords of n bits
 #define LDPCA_COLS(n, nt) (((n) + (nt) - 1) / (nt))
 
-// stage: the ladder code's index tables (rid, pos: 2 x e uint16) live in
-// shared memory too (see ld_try_code)
-__host__ __device__ inline size_t ldpca_smem_bytes(int n, int e, bool stage = false) {
-  size_t b = (size_t)e * 4;       // msg
-  if (stage) b += (size_t)e * 4;  // rid and pos of the code tried
-  b += (size_t)n * 4;             // rowt
-  b += (size_t)e;            // sgd
-  b += (size_t)n;            // rpar
-  b += (size_t)n / 8;        // accs
+__host__ __device__ inline int ldpca_groups(int n) { return (n + 31) / 32; }
+
+__host__ __device__ inline size_t ldpca_smem_bytes(int n, int pos_max) {
+  size_t b = (size_t)pos_max * 4;          // msg
+  b += (size_t)ldpca_groups(n) * 16;       // hdr
+  b += (size_t)n * 4;                      // rowt
+  b += (size_t)n / 8;                      // accs
   return (b + 15) & ~(size_t)15;
 }
 
-// NT threads decoding one codeword; `t` is the thread's index in the group.
-// BLOCK: the group is the whole thread block and synchronises with the block's
-// barrier (__syncthreads); otherwise on the hardware barrier `bar` (1-15),
-// which only its NT threads use.
-template <int NT_, bool BLOCK>
+// shared words a group coordinates through (one set per group)
+struct LdCtl {
+  uint32_t any[2];  // cluster form: a check failed (by iteration parity)
+  uint32_t stop;    // a lower code of the codeword has succeeded
+  uint32_t crc[8];  // cluster form: each block's part of the CRC
+  int flag;         // free for the caller, and the CRC's verdict
+};
+
+// distributed shared memory: the address of this block's shared word in block
+// `rank` of the cluster, and a store and an xor there
+__device__ __forceinline__ uint32_t ld_mapa(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void ld_st_cluster(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ void ld_xor_cluster(uint32_t addr, uint32_t v) {
+  asm volatile("red.relaxed.cluster.shared::cluster.xor.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ void ld_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// an edge word of the edge pass; volatile, so that it is not loaded before the
+// row pass and waited for there
+__device__ __forceinline__ uint32_t ld_edge(const uint32_t *p) {
+  uint32_t v;
+  asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+
+// NT threads decoding one codeword (or, in a cluster of C blocks, NT threads of
+// each block); `t` is the thread's index in its block's part.  BLOCK: the group
+// is the whole thread block and synchronises with the block's barrier
+// (__syncthreads); otherwise on the hardware barrier `bar` (1-15), which only
+// its NT threads use.
+template <int NT_, bool BLOCK, int C_ = 1>
 struct LdGroup {
-  static constexpr int NT = NT_;
-  int t, bar;
+  static constexpr int NT = NT_, C = C_, STRIDE = NT_ * C_;
+  static_assert(C_ == 1 || BLOCK, "a cluster group takes whole blocks");
+  int t, bar, rank;
+  // Columns of a thread, one per round.  When n is not a multiple of STRIDE
+  // the first round is a partial one: its columns (the last of the codeword)
+  // are spread over all warps, a few lanes of each, and the full rounds
+  // follow.  A partial last round on a few whole warps would leave the memory
+  // system idle while those finish.
+  __device__ __forceinline__ int col0(int n) const {
+    constexpr int nw = STRIDE / 32;
+    const int rest = n % STRIDE, share = (rest + nw - 1) / nw;
+    const int w = (C_ == 1 ? 0 : rank * (NT_ / 32)) + (t >> 5), l = t & 31;
+    if (rest == 0) return colf();
+    const int r = w * share + l;
+    return l < share && r < rest ? n - rest + r : n;  // n: none in this round
+  }
+  __device__ __forceinline__ int colf() const { return C_ == 1 ? t : rank * NT_ + t; }
+  // column of round c > 0
+  __device__ __forceinline__ int col(int n, int c) const {
+    return c == 0 ? col0(n) : colf() + (c - (n % STRIDE != 0)) * STRIDE;
+  }
+  // barrier over the block's part
   __device__ __forceinline__ void sync() const {
     if constexpr (BLOCK)
       __syncthreads();
     else
       asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(NT_) : "memory");
   }
-  // barrier that also returns whether any thread of the group passed p != 0
-  __device__ __forceinline__ int sync_or(int p) const {
-    if constexpr (BLOCK) {
+  // barrier over everything that decodes the codeword
+  __device__ __forceinline__ void sync_all() const {
+    if constexpr (C_ > 1)
+      ld_cluster_sync();
+    else
+      sync();
+  }
+  // sync_all that also returns whether any thread passed p != 0; `ph`
+  // alternates between calls
+  __device__ __forceinline__ int sync_or(int p, LdCtl *ctl, int ph) const {
+    if constexpr (C_ > 1) {
+      if (__any_sync(0xffffffffu, p) && (t & 31) < C_)
+        ld_st_cluster(ld_mapa((uint32_t)__cvta_generic_to_shared(&ctl->any[ph]), (uint32_t)(t & 31)), 1u);
+      ld_cluster_sync();
+      return (int)*(volatile uint32_t *)&ctl->any[ph];
+    } else if constexpr (BLOCK) {
       return __syncthreads_or(p);
     } else {
       int r;
@@ -92,20 +172,17 @@ struct LdGroup {
 
 struct LdSmem {
   float *msg, *rowt;
-  uint16_t *rid, *pos;  // staged index tables of the code tried (null: read from global memory)
-  uint8_t *sgd, *rpar, *dec, *accs;
+  uint4 *hdr;
+  uint8_t *dec, *accs;
 };
 
-__device__ __forceinline__ LdSmem ld_carve(uint8_t *base, int n, int e, bool stage = false) {
+__device__ __forceinline__ LdSmem ld_carve(uint8_t *base, const LadderDev &L) {
   LdSmem S;
   S.msg = reinterpret_cast<float *>(base);
-  S.rid = stage ? reinterpret_cast<uint16_t *>(S.msg + e) : nullptr;  // e is a multiple of 8: 16-byte aligned
-  S.pos = stage ? S.rid + e : nullptr;
-  S.rowt = stage ? reinterpret_cast<float *>(S.pos + e) : S.msg + e;
-  S.sgd = reinterpret_cast<uint8_t *>(S.rowt + n);
-  S.rpar = S.sgd + e;
-  S.accs = S.rpar + n;                          // the codeword's packed accumulated syndrome
-  S.dec = reinterpret_cast<uint8_t *>(S.rowt);  // decoded bits, once BP is over
+  S.hdr = reinterpret_cast<uint4 *>(S.msg + L.pos_max);  // pos_max is a multiple of 4
+  S.rowt = reinterpret_cast<float *>(S.hdr + ldpca_groups(L.n));
+  S.accs = reinterpret_cast<uint8_t *>(S.rowt + L.n);  // the codeword's packed accumulated syndrome
+  S.dec = reinterpret_cast<uint8_t *>(S.rowt);       // decoded bits, once BP is over
   return S;
 }
 
@@ -134,23 +211,26 @@ __device__ __forceinline__ void ld_put_bitplane(const G &g, const LdpcaJob &J, c
 }
 
 // decoded = inv(H) * syndrome of the full-rate code (LdpcaDecoder.cpp:695-716);
-// syndrome words are built in `sw` (n/32 words of shared memory)
+// syndrome words are built in `sw` (n/32 words of shared memory).  A warp
+// takes a row of the inverse at a time, its lanes consecutive words, so the
+// reads (5 MB at CIF) are coalesced.
 template <class G>
 __device__ __forceinline__ void ld_invh_decode(const G &g, const LadderDev &L, const uint8_t *synd, uint8_t *dec,
                                uint32_t *sw) {
   constexpr int NT = G::NT;
-  const int n = L.n, lane = g.t & 31, warp = g.t >> 5;
+  const int n = L.n, nw = L.invh_words, lane = g.t & 31, warp = g.t >> 5;
   for (int base = warp * 32; base < n; base += NT) {
     const int k = base + lane;
     const uint32_t b = __ballot_sync(0xffffffffu, k < n && (synd[k] & 1));
     if (lane == 0) sw[base >> 5] = b;
   }
   g.sync();
-  for (int j = g.t; j < n; j += NT) {
-    const uint32_t *row = L.invh + (size_t)j * L.invh_words;
+  for (int j = warp; j < n; j += NT / 32) {
+    const uint32_t *row = L.invh + (size_t)j * nw;
     uint32_t x = 0;
-    for (int w = 0; w < L.invh_words; w++) x ^= __ldg(row + w) & sw[w];
-    dec[j] = (uint8_t)(__popc(x) & 1);
+    for (int w = lane; w < nw; w += 32) x ^= __ldg(row + w) & sw[w];
+    const uint32_t odd = __ballot_sync(0xffffffffu, __popc(x) & 1);
+    if (lane == 0) dec[j] = (uint8_t)(__popc(odd) & 1);
   }
   g.sync();
 }
@@ -161,10 +241,19 @@ __device__ __forceinline__ uint8_t ld_acc_bit(const uint8_t *packed, int i) {
   return (uint8_t)((packed[i >> 3] >> (7 - (i & 7))) & 1);
 }
 
-// syndrome of ladder code `code` from the accumulated syndrome (LdpcaDecoder.cpp:684-693):
-// bit k of the code is accumulated bit idx[k % nb] + (k / nb) * period xor the
-// same of k - 1.  Thread t takes k = t, t + NT, ...; the quotient and
-// remainder of k by nb advance by those of NT, with no division per bit.
+// bit r of the syndrome of ladder code `code` (LdpcaDecoder.cpp:684-693):
+// accumulated bit idx[r % nb] + (r / nb) * period xor the same of r - 1
+__device__ __forceinline__ uint32_t ld_synd_bit(const LadderDev &L, const int *idx, int nb, const uint8_t *packed,
+                                                int r) {
+  const int P = L.period, q = r / nb, i = r - q * nb;
+  uint32_t s = ld_acc_bit(packed, __ldg(idx + i) + q * P);
+  if (r > 0) s ^= ld_acc_bit(packed, i > 0 ? __ldg(idx + i - 1) + q * P : __ldg(idx + nb - 1) + (q - 1) * P);
+  return s;
+}
+
+// the whole syndrome of a code in row order, one byte per row.  Thread t takes
+// rows t, t + NT, ...; the quotient and remainder of a row by nb advance by
+// those of NT, with no division per bit.
 template <class G>
 __device__ __forceinline__ void ld_build_syndrome(const G &g, const LadderDev &L, int code,
                                                   const uint8_t *packed, uint8_t *synd) {
@@ -186,16 +275,25 @@ __device__ __forceinline__ void ld_build_syndrome(const G &g, const LadderDev &L
   }
 }
 
+// the full-rate code: S.dec = inv(H) * syndrome, over the staged accumulated syndrome
+template <class G>
+__device__ __forceinline__ void ld_full_rate(const G &g, const LadderDev &L, const LdSmem &S) {
+  uint8_t *synd = reinterpret_cast<uint8_t *>(S.msg);                          // n bytes
+  uint32_t *sw = reinterpret_cast<uint32_t *>(synd + ((L.n + 15) & ~15));     // then n/32 words
+  ld_build_syndrome(g, L, L.num_codes - 1, S.accs, synd);
+  g.sync();
+  ld_invh_decode(g, L, synd, S.dec, sw);
+}
+
 // log LR of the group's columns into registers (LdpcaDecoder.cpp:665-666) and,
 // when want_entropy, the entropy terms H_k = (P(-log P + log(1-P)) - log(1-P))
 // / LOG2 with P = LR/(1+LR) (ComputeCE) into `terms` (n floats of shared memory).
 template <class G, int MAXC>
 __device__ __forceinline__ void ld_llr(const G &g, int n, const float *lr, const XlmDev &xt,
                                        const XlSmall &xs, float (&llr)[MAXC], float *terms, float *llr_out) {
-  constexpr int NT = G::NT;
 #pragma unroll
   for (int c = 0; c < MAXC; c++) {
-    const int k = g.t + c * NT;
+    const int k = g.col(n, c);
     llr[c] = 0.0f;
     if (k < n) {
       const float v = lr[k];
@@ -243,203 +341,244 @@ __device__ __forceinline__ int ld_start_code(const LadderDev &L, float h) {
 // parity check holds (success) or max_iter iterations ran or, when `bestp` is
 // given, a lower code of the same codeword has succeeded (*bestp < code), then
 // the CRC-8 of the hard decision (LdpcaDecoder.cpp:684-693, 718-758).
-// Returns 1 when the code decodes with a matching CRC; the decoded bits are
-// then in S.dec.  `iters` receives the BP iterations run.  s_ured holds NT/32
-// words of shared memory, s_flag one int, both the group's own.
-// an index table entry: a shared-memory read when staged, a read-only global one otherwise
-template <bool STAGE>
-__device__ __forceinline__ int ld_idx(const uint16_t *p) {
-  if constexpr (STAGE) return *p;
-  else return __ldg(p);
-}
-
-template <class G, int MAXC, bool STAGE = false>
+// Returns 1 when the code decodes with a matching CRC; `dm` then holds the
+// decoded bits of the thread's columns (bit c: round c), and
+// S.dec all of them (not in a cluster).  `iters` receives the BP iterations
+// run.  s_ured holds NT/32 words of shared memory.
+template <class G, int MAXC>
 __device__ __forceinline__ int ld_try_code(const G &g, const LadderDev &L, int code, const float (&llr)[MAXC],
                            int crc, const XlmDev &xt, const uint4 *pdesc, int max_iter,
-                           const volatile int *bestp, const LdSmem &S, uint32_t *s_ured, int *s_flag, int &iters) {
-  constexpr int NT = G::NT;
-  constexpr int UNR = 8;                  // edge-pass table reads in flight per thread
-  constexpr int CB = 1;  // column-pass columns per batch (3 reads each; more spill at 64 registers)
-  const int n = L.n, E = L.e, t = g.t, lane = t & 31, warp = t >> 5;
+                           const volatile int *bestp, const LdSmem &S, uint32_t *s_ured, LdCtl *ctl, int &iters,
+                           uint32_t &dm) {
+  constexpr int NT = G::NT, C = G::C, NW = NT / 32;
+  // a cluster keeps its columns' magnitudes in registers (they are stored in
+  // other blocks); alone they are read back from shared memory
+  constexpr bool KEEP = C > 1;
+  const int n = L.n, t = g.t, lane = t & 31, warp = t >> 5;
+  const int rank = C > 1 ? g.rank : 0;
+  const bool lead = t == 0 && rank == 0;
   float *msg = S.msg, *rowt = S.rowt;
-  uint8_t *sgd = S.sgd, *rpar = S.rpar, *dec = S.dec;
-  const int m = L.synd_len[code];
-  // STAGE: the code's index tables are copied to shared memory for the whole
-  // try (e is a multiple of 8: 16-byte copies), which keeps a global round
-  // trip off the chain leading to every table gather.  Only where the block
-  // owns its SM and the copy leaves the shared-memory carveout (so the L1
-  // that the in-flight table gathers allocate in) unchanged: QCIF codewords
-  // on 1024 threads.  At CIF the 76 KB of tables would cut L1 to a fifth.
-  const uint16_t *__restrict__ pos = L.pos + (size_t)code * E;
-  const uint16_t *__restrict__ rid = L.rid + (size_t)code * E;
-  if constexpr (STAGE) {
-    const uint4 *gr = reinterpret_cast<const uint4 *>(rid), *gp = reinterpret_cast<const uint4 *>(pos);
-    uint4 *sr = reinterpret_cast<uint4 *>(S.rid), *sp = reinterpret_cast<uint4 *>(S.pos);
-    for (int i = t; i < E / 8; i += NT) {
-      sr[i] = __ldg(gr + i);
-      sp[i] = __ldg(gp + i);
-    }
-    pos = S.pos;
-    rid = S.rid;
-  }
-  ld_build_syndrome(g, L, code, S.accs, rpar);
-  g.sync();
-  const int *rp = L.row_ptr + (size_t)code * (n + 1);
-  // first magnitudes: phi(|LLR|) on the three edges of each column
+  const int m = L.synd_len[code], ng = (m + 31) >> 5;
+  const uint32_t *__restrict__ edge = L.edge + (size_t)code * 3 * n;
+  const uint32_t msg_a = (uint32_t)__cvta_generic_to_shared(msg);
+  const uint32_t hdr_a = (uint32_t)__cvta_generic_to_shared(S.hdr);
+  const uint32_t rowt_a = (uint32_t)__cvta_generic_to_shared(rowt);
+  // an edge word: position in the low half, row slot in the high half; the
+  // row's group (slot / 32) belongs to block group % C
+  auto put = [&](uint32_t ed, uint32_t bits) {
+    if constexpr (C > 1)
+      ld_st_cluster(ld_mapa(msg_a + 4 * (ed & 0xffffu), (ed >> 21) & (C - 1)), bits);
+    else
+      msg[ed & 0xffffu] = __uint_as_float(bits);
+  };
+  auto flip = [&](uint32_t ed) {
+    const uint32_t bit = 1u << ((ed >> 16) & 31u);
+    if constexpr (C > 1)
+      ld_xor_cluster(ld_mapa(hdr_a + 16 * (ed >> 21) + 8, (ed >> 21) & (C - 1)), bit);
+    else
+      atomicXor(&S.hdr[ed >> 21].z, bit);
+  };
+  // padding positions add +0 to their row's sum, which leaves it unchanged
+  for (int p = t; p < L.pos_max / 4; p += NT) reinterpret_cast<float4 *>(msg)[p] = make_float4(0.f, 0.f, 0.f, 0.f);
   {
-    float ph[MAXC];
+    const uint32_t *grp = L.grp + (size_t)code * ldpca_groups(n);
+    const uint16_t *srow = L.slot_row + (size_t)code * n;
+    const int nb = L.bpp[code];
+    const int *idx = L.idx + (size_t)code * L.period;
+    for (int gr = rank + C * warp; gr < ng; gr += C * NW) {
+      const int s = 32 * gr + lane;
+      const uint32_t b = __ballot_sync(0xffffffffu, s < m && ld_synd_bit(L, idx, nb, S.accs, __ldg(srow + min(s, m - 1))));
+      if (lane == 0) S.hdr[gr] = make_uint4(__ldg(grp + gr), b, b, 0u);
+    }
+  }
+  if (t == 0) {
+    ctl->any[0] = ctl->any[1] = 0;
+    ctl->stop = 0;
+  }
+  uint32_t mg[KEEP ? MAXC : 1][3];
+  g.sync_all();
+  // first magnitudes: phi(|LLR|) on the three edges of each column
+#pragma unroll(KEEP ? MAXC : 2)
+  for (int c = 0; c < MAXC; c++) {
+    const int k = g.col(n, c);
+    if (k < n) {
+      const float l = llr[c];
+      const uint32_t bits = (__float_as_uint(xl_phi(xt, pdesc, (fabsf(l) + 1e-9f) / 2.0f)) & 0x7fffffffu) |
+                            (__float_as_uint(l) & 0x80000000u);
 #pragma unroll
-    for (int c = 0; c < MAXC; c++)
-      ph[c] = t + c * NT < n ? xl_phi(xt, pdesc, (fabsf(llr[c]) + 1e-9f) / 2.0f) : 0.0f;
-#pragma unroll
-    for (int c = 0; c < MAXC; c++) {
-      const int k = t + c * NT;
-      if (k < n) {
-        const uint8_t ng = (uint8_t)(__float_as_uint(llr[c]) >> 31);
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-          const int p = ld_idx<STAGE>(pos + 3 * k + i);
-          msg[p] = ph[c];
-          sgd[p] = ng;
-        }
+      for (int i = 0; i < 3; i++) {
+        put(__ldg(edge + i * n + k), bits);
+        if constexpr (KEEP) mg[c][i] = bits;
       }
     }
   }
-  g.sync();
+  // the edge words and the LLR of the next column are read one round ahead
+  // (round 0's during the row pass)
+  uint32_t nx[3];
+  float nl = llr[0];
+  const int kfirst = g.col0(n);
+#pragma unroll
+  for (int i = 0; i < 3; i++) nx[i] = ld_edge(edge + i * n + min(kfirst, n - 1));
+  dm = 0;
+  int best = bestp && lead ? *bestp : LDPCA_NONE;
+  g.sync_all();
   bool converged = false;
   int it = 0;
   for (;;) {
-    // (R) rows: sum of the magnitudes in edge order and the sign parity with
-    //     the syndrome bit, for the next edge pass; from the second pass on
-    //     also the parity check of the previous hard decision
+    // rows: lane l of a warp sums the row in slot 32 g + l of its groups.  The
+    // loads of four edges are issued before their adds, which stay in edge
+    // order; with groups of 3 to 7 edges at the higher codes the pass is bound
+    // by its instructions, so full groups take constant strides
     int wrong = 0;
-    for (int r = t; r < m; r += NT) {
-      const int p0 = rp[r], p1 = rp[r + 1];
+    for (int gr = rank + C * warp; gr < ng; gr += C * NW) {
+      const uint4 hd = S.hdr[gr];
+      const float *p = msg + (hd.x & 0xffffu) + lane;
+      const int deg = (int)(hd.x >> 16);
       float s = 0.0f;
-      uint32_t x = 0;  // bit 0: xor of signs, bit 1: xor of decisions
-      // low codes have few, long rows (up to ~200 edges): the loads of eight
-      // edges are issued before their adds, which stay in edge order
-      int p = p0;
-      for (; p + 8 <= p1; p += 8) {
-        float v[8];
-        uint32_t b[8];
-#pragma unroll
-        for (int q = 0; q < 8; q++) {
-          v[q] = msg[p + q];
-          b[q] = sgd[p + q];
+      uint32_t x = (hd.y >> lane) << 31;  // xor of the signs and the syndrome bit, in the top bit
+      auto add = [&](float v) {
+        s += fabsf(v);
+        x ^= __float_as_uint(v);
+      };
+      auto row = [&](int width) {
+        int left = deg;
+        for (; left >= 4; left -= 4, p += 4 * width) {
+          const float v0 = p[0], v1 = p[width], v2 = p[2 * width], v3 = p[3 * width];
+          add(v0);
+          add(v1);
+          add(v2);
+          add(v3);
         }
+        if (left >= 2) {
+          const float v0 = p[0], v1 = p[width];
+          add(v0);
+          add(v1);
+          p += 2 * width;
+        }
+        if (left & 1) add(p[0]);
+      };
+      const int width = m - 32 * gr;
+      if (width >= 32)
+        row(32);
+      else if (lane < width)
+        row(width);
+      const uint32_t r = __float_as_uint(s) | (x & 0x80000000u);
+      if (lane < width) {
+        if constexpr (C > 1) {
 #pragma unroll
-        for (int q = 0; q < 8; q++) {
-          s += v[q];
-          x ^= b[q];
+          for (int b = 0; b < C; b++) ld_st_cluster(ld_mapa(rowt_a + 4 * (32 * gr + lane), b), r);
+        } else {
+          rowt[32 * gr + lane] = __uint_as_float(r);
         }
       }
-      for (; p < p1; p++) {
-        s += msg[p];
-        x ^= sgd[p];
-      }
-      const uint32_t syn = rpar[r] & 1u;
-      rowt[r] = s;
-      rpar[r] = (uint8_t)(syn | (((x & 1u) ^ syn) << 1));
-      wrong |= (int)(((x >> 1) ^ syn) & 1u);
+      wrong |= (int)(hd.z != 0);
     }
-    if (t == 0) *s_flag = bestp ? (int)(*bestp < code) : 0;
-    const int any_wrong = g.sync_or(wrong);
+    if (lead && best < code) {
+      if constexpr (C > 1) {
+#pragma unroll
+        for (int b = 0; b < C; b++) ld_st_cluster(ld_mapa((uint32_t)__cvta_generic_to_shared(&ctl->stop), b), 1u);
+      } else {
+        ctl->stop = 1;
+      }
+    }
+    const int any_wrong = g.sync_or(wrong, ctl, it & 1);
     if (it > 0 && !any_wrong) {
       converged = true;
       break;
     }
     // abandon a code above a known success
-    if (it == max_iter || *s_flag) break;
+    if (it == max_iter || *(volatile uint32_t *)&ctl->stop) break;
+    if (C > 1 && t == 0) ctl->any[(it & 1) ^ 1] = 0;  // last read before the previous edge pass
     it++;
-    // (E) edges: c->v = phi(row sum - own magnitude) with the product of
-    //     the other signs
-    for (int p0 = t; p0 < E; p0 += UNR * NT) {
-      float c[UNR];
-      int rr[UNR];
+    if (bestp && lead) best = *bestp;  // arrives during the edge pass, used after it
+    // edges, column by column (a rolled loop: seven copies of it would not
+    // stay in the instruction cache)
+    int k = kfirst;
+#pragma unroll(KEEP ? MAXC : 1)
+    for (int c = 0; c < MAXC; c++) {
+      const int kn = c + 1 < MAXC ? g.col(n, c + 1) : kfirst;
+      uint32_t ed[3], mv[3];
+      const float l = nl;
 #pragma unroll
-      for (int q = 0; q < UNR; q++) {
-        // lanes past the last edge repeat it (no branch, so that the UNR
-        // table reads are in flight together) and store nothing
-        const int p = min(p0 + q * NT, E - 1);
-        rr[q] = ld_idx<STAGE>(rid + p);
-        c[q] = xl_phi(xt, pdesc, (rowt[rr[q]] - msg[p] + 1e-9f) / 2.0f);
-      }
+      for (int i = 0; i < 3; i++) ed[i] = nx[i];
 #pragma unroll
-      for (int q = 0; q < UNR; q++) {
-        const int p = p0 + q * NT;
-        if (p < E) msg[p] = c[q] * ((((uint32_t)rpar[rr[q]] >> 1) ^ (sgd[p] & 1u)) ? -1.0f : 1.0f);
-      }
-    }
-    g.sync();
-    // (C) columns: total in edge order, hard decision, extrinsic messages
-    //     and their magnitudes for the next iteration
+      for (int i = 0; i < 3; i++) nx[i] = ld_edge(edge + i * n + min(kn, n - 1));
+      nl = llr[c + 1 < MAXC ? c + 1 : 0];
+      if (k < n) {
 #pragma unroll
-    for (int c0 = 0; c0 < MAXC; c0 += CB) {
-      float ph[CB][3];
-      uint32_t sb[CB][3];
-      int pp[CB][3];
+        for (int i = 0; i < 3; i++) {
+          const uint32_t r = __float_as_uint(rowt[ed[i] >> 16]);
+          const uint32_t a = KEEP ? mg[KEEP ? c : 0][i] : __float_as_uint(msg[ed[i] & 0xffffu]);
+          // c->v: phi(row sum - own magnitude) with the product of the other signs
+          const float y = (fabsf(__uint_as_float(r)) - fabsf(__uint_as_float(a)) + 1e-9f) / 2.0f;
+          mv[i] = __float_as_uint(xl_phi(xt, pdesc, y)) ^ ((r ^ a) & 0x80000000u);
+        }
+        // total in edge order, hard decision, extrinsic messages and their
+        // magnitudes for the next iteration
+        float tot = l;
 #pragma unroll
-      for (int b = 0; b < CB; b++) {
-        const int c = c0 + b, k = t + c * NT;
-        if (c < MAXC && k < n) {
-          float mv[3];
+        for (int i = 0; i < 3; i++) tot += __uint_as_float(mv[i]);
+        if ((__float_as_uint(tot) >> 31) != ((dm >> c) & 1u)) {
+          dm ^= 1u << c;
 #pragma unroll
-          for (int i = 0; i < 3; i++) {
-            pp[b][i] = ld_idx<STAGE>(pos + 3 * k + i);
-            mv[i] = msg[pp[b][i]];
-          }
-          float tmp = llr[c];
-          tmp += mv[0];
-          tmp += mv[1];
-          tmp += mv[2];
-          const uint32_t d = __float_as_uint(tmp) >> 31;
+          for (int i = 0; i < 3; i++) flip(ed[i]);
+        }
 #pragma unroll
-          for (int i = 0; i < 3; i++) {
-            const float v = tmp - mv[i];
-            sb[b][i] = (__float_as_uint(v) >> 31) | (d << 1);
-            ph[b][i] = xl_phi(xt, pdesc, (fabsf(v) + 1e-9f) / 2.0f);
-          }
+        for (int i = 0; i < 3; i++) {
+          const float v = tot - __uint_as_float(mv[i]);
+          mv[i] = (__float_as_uint(xl_phi(xt, pdesc, (fabsf(v) + 1e-9f) / 2.0f)) & 0x7fffffffu) |
+                  (__float_as_uint(v) & 0x80000000u);
+        }
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+          put(ed[i], mv[i]);
+          if constexpr (KEEP) mg[c][i] = mv[i];
         }
       }
-#pragma unroll
-      for (int b = 0; b < CB; b++) {
-        const int c = c0 + b, k = t + c * NT;
-        if (c < MAXC && k < n)
-#pragma unroll
-          for (int i = 0; i < 3; i++) {
-            msg[pp[b][i]] = ph[b][i];
-            sgd[pp[b][i]] = (uint8_t)sb[b][i];
-          }
-      }
+      k = kn;
     }
-    g.sync();
+    g.sync_all();
   }
   iters = it;
   if (!converged) {
-    g.sync();  // every thread has read *s_flag: the caller may reuse it
+    g.sync_all();  // every thread has read ctl: the caller may reuse it
     return 0;
   }
-  // hard decision of each column (bit 1 of its edges' sgd) into dec, and the
-  // CRC-8 of the decoded bitplane as the xor of single-bit CRCs (the CRC is
-  // linear for a fixed length with zero initial value and no final xor)
+  // the hard decisions into dec, and the CRC-8 of the decoded bitplane as the
+  // xor of single-bit CRCs (the CRC is linear for a fixed length with zero
+  // initial value and no final xor)
   uint32_t cr = 0;
-  for (int k = t; k < n; k += NT) {
-    const uint8_t d = (uint8_t)((sgd[ld_idx<STAGE>(pos + 3 * k)] >> 1) & 1u);
-    dec[k] = d;
-    if (d) cr ^= __ldg(L.crc_tab + k);
+  for (int c = 0; c < MAXC; c++) {
+    const int k = g.col(n, c);
+    if (k < n) {
+      const uint32_t d = (dm >> c) & 1u;
+      if constexpr (C == 1) S.dec[k] = (uint8_t)d;
+      if (d) cr ^= __ldg(L.crc_tab + k);
+    }
   }
   for (int o = 16; o > 0; o >>= 1) cr ^= __shfl_xor_sync(0xffffffffu, cr, o);
   if (lane == 0) s_ured[warp] = cr;
   g.sync();
   if (t == 0) {
     uint32_t x = 0;
-    for (int w = 0; w < NT / 32; w++) x ^= s_ured[w];
-    *s_flag = (int)(x & 0xffu) == crc;
+    for (int w = 0; w < NW; w++) x ^= s_ured[w];
+    if constexpr (C > 1) {
+      for (int b = 0; b < C; b++) ld_st_cluster(ld_mapa((uint32_t)__cvta_generic_to_shared(&ctl->crc[rank]), b), x);
+    } else {
+      ctl->flag = (int)(x & 0xffu) == crc;
+    }
   }
-  g.sync();
-  const int ok = *s_flag;
-  g.sync();
+  g.sync_all();
+  int ok;
+  if constexpr (C > 1) {
+    uint32_t x = 0;
+#pragma unroll
+    for (int b = 0; b < C; b++) x ^= *(volatile uint32_t *)&ctl->crc[b];
+    ok = (int)(x & 0xffu) == crc;
+  } else {
+    ok = ctl->flag;
+  }
+  g.sync_all();
   return ok;
 }
 
