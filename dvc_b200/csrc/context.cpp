@@ -119,7 +119,7 @@ bool Context::init(const char *data, const char *tables, int dev) {
       char perr[256];
       if (!dvc_phi_pack(phi.data(), xlm.tanh_ylo, xlm.tanh_y1, 0, pk, perr, sizeof perr)) return fail(perr);
     }
-    if (pk.desc.size() / 4 > XL_PHI_MAX_BINADES) return fail("phi table has too many binades");
+    if (pk.desc.size() / 4 > XL_PHI_MAX_SEGS) return fail("phi table has too many segments");
     auto put = [&](const void *src, size_t bytes, const void **dst) {
       void *p = nullptr;
       if (cudaMalloc(&p, bytes) != cudaSuccess) return false;
@@ -131,7 +131,7 @@ bool Context::init(const char *data, const char *tables, int dev) {
     if (!put(pk.desc.data(), pk.desc.size() * 4, (const void **)&xlm.phi_desc) ||
         !put(pk.rec.data(), pk.rec.size() * 4, (const void **)&xlm.phi_rec))
       return fail("uploading the phi table failed");
-    xlm.phi_nbin = (int)(pk.desc.size() / 4);
+    xlm.phi_nseg = (int)(pk.desc.size() / 4);
     {
       int max_linear = 0;
       cudaDeviceGetAttribute(&max_linear, cudaDevAttrMaxTexture1DLinearWidth, device);
@@ -148,16 +148,17 @@ bool Context::init(const char *data, const char *tables, int dev) {
       xlm.phi_tex = tex;
     }
     phi_bytes = (pk.desc.size() + pk.rec.size()) * 4;
-    // optional L2 persisting window over the records of the binades most BP
-    // reads land in (y in [2^-6, 8), exponents 121..129: about 99% of the reads,
-    // 60 MB), so that other kernels' streaming data does not evict them;
+    // optional L2 persisting window over the records of the segments most BP
+    // reads land in (y in [2^-6, 8), exponents 121..129: about 99% of the
+    // reads), so that other kernels' streaming data does not evict them;
     // DVC_PHI_L2_MB = the set-aside in MB (0 or unset: off)
     set_phi_window(nullptr, 0, 0.0f);
     if (const char *mb = getenv("DVC_PHI_L2_MB")) {
       const size_t want = (size_t)atoi(mb) << 20;
-      const int b_lo = 121 - (int)(xlm.tanh_ylo >> 23), b_hi = 129 - (int)(xlm.tanh_ylo >> 23);
-      if (want > 0 && b_lo >= 0 && b_hi < xlm.phi_nbin) {
-        const size_t r0 = pk.desc[4 * b_lo], r1 = b_hi + 1 < xlm.phi_nbin ? pk.desc[4 * (b_hi + 1)] : pk.rec.size() / 4;
+      const int b_lo = (int)(((121u << 23) - xlm.tanh_ylo) >> XL_PHI_SEG_BITS);
+      const int b_hi = (int)(((130u << 23) - xlm.tanh_ylo) >> XL_PHI_SEG_BITS) - 1;
+      if (want > 0 && b_lo >= 0 && b_hi < xlm.phi_nseg) {
+        const size_t r0 = pk.desc[4 * b_lo], r1 = b_hi + 1 < xlm.phi_nseg ? pk.desc[4 * (b_hi + 1)] : pk.rec.size() / 4;
         int max_persist = 0, max_window = 0;
         cudaDeviceGetAttribute(&max_persist, cudaDevAttrMaxPersistingL2CacheSize, device);
         cudaDeviceGetAttribute(&max_window, cudaDevAttrMaxAccessPolicyWindowSize, device);

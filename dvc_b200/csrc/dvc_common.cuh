@@ -79,18 +79,18 @@ __device__ __forceinline__ float xl_expf(const XlmDev &t, const XlSmall &s, floa
 }
 
 // copy the phi descriptors into shared memory (every thread of the block
-// calls this; follow with __syncthreads); `buf` holds XL_PHI_MAX_BINADES entries
+// calls this; follow with __syncthreads); `buf` holds XL_PHI_MAX_SEGS entries
 __device__ __forceinline__ void xl_phi_stage(const XlmDev &t, uint4 *buf) {
-  for (int i = threadIdx.x; i < t.phi_nbin; i += blockDim.x) buf[i] = t.phi_desc[i];
+  for (int i = threadIdx.x; i < t.phi_nseg; i += blockDim.x) buf[i] = t.phi_desc[i];
 }
 
 // -logf(tanhf(y)), the reference's two library calls (LdpcaDecoder.cpp:513,519),
 // from the packed table over [tanh_ylo, tanh_y1); -0 where tanhf(y) is 1.
 // Every argument the decoder forms is (x + 1e-9f)/2 with x >= 0, so it is at
 // least 5e-10 > 2^-31 = tanh_ylo; a smaller one (never formed) clamps to the
-// first entry rather than reading outside the table.  `desc` is the binade
+// first entry rather than reading outside the table.  `desc` is the segment
 // descriptor array (staged in shared memory by xl_phi_stage); one 16-byte
-// record read per call, the same instructions in every binade, so that the
+// record read per call, the same instructions in every segment, so that the
 // reads of several calls can be in flight together.  Records are cached in
 // L1: messages that stay put from one iteration to the next read the same
 // records again.
@@ -98,11 +98,11 @@ __device__ __forceinline__ float xl_phi(const XlmDev &t, const uint4 *desc, floa
   const uint32_t u = __float_as_uint(y);
   const bool one = u >= t.tanh_y1;  // tanhf(y) == 1 (also NaN/negative patterns, never formed)
   const uint32_t i = (!one && u > t.tanh_ylo) ? u - t.tanh_ylo : 0u;
-  const uint4 d = desc[i >> XL_PHI_BINADE_BITS];
-  const uint32_t j = i & ((1u << XL_PHI_BINADE_BITS) - 1u);
+  const uint4 d = desc[i >> XL_PHI_SEG_BITS];
+  const uint32_t j = i & ((1u << XL_PHI_SEG_BITS) - 1u);
   const uint32_t g = xl_phi_group(j, d.z);
   const uint4 r = tex1Dfetch<uint4>((cudaTextureObject_t)t.phi_tex, (int)(d.x + g));
-  const uint32_t v = xl_phi_decode_bits(j - g * (d.y & 0xffu), d.y, r.x, r.y, r.z, r.w);
+  const uint32_t v = xl_phi_decode_bits(j - g * (d.y & 0xffu), d.y, d.w, r.x, r.y, r.z, r.w);
   return one ? -0.0f : __uint_as_float(v);
 }
 

@@ -35,7 +35,7 @@
 // at all: its argument is a float in [2^-31, y1) (y1 = the first float with
 // tanhf(y) == 1, above which phi is -0), so the library's value of the whole
 // expression is swept once per context for every one of those 2.9e8 floats
-// and stored packed (xl_phi_field below, about 170 MB instead of 1.1 GB), so
+// and stored packed (below, about a tenth of the 1.1 GB of a direct table), so
 // that the part the decoder reads stays in the L2 cache.
 #pragma once
 #include <math.h>
@@ -159,29 +159,31 @@ XL_HD uint32_t xl_tie_dist(double d) {
 
 // ---- packed table of phi(y) = -logf(tanhf(y)) ----
 // Entry i is the library's phi of the float with bits XL_TANH_YLO + i.  The
-// entries are split into binades (2^23 consecutive patterns, one exponent of
-// y); each binade has a descriptor {first record, format, reciprocal} and is
-// cut into groups of G consecutive entries, one 16-byte record per group, in
-// one of two formats:
-//  * delta format (4 <= G <= 32): word 0 = bits of the group's first value,
-//    words 1..3 (96 bits, word 1 lowest) G fields of W = 96 / G bits, field k
-//    at bit k*W, field k = bits(v_0) - bits(v_k) (phi falls as y grows; field
-//    0 is 0), v_k = word 0 - field k;
+// entries are split into segments (2^19 consecutive patterns, a sixteenth of a
+// binade of y); each segment has a descriptor {first record, format,
+// reciprocal, slope} and is cut into groups of G consecutive entries, one
+// 16-byte record per group, in one of two formats:
+//  * line format (6 <= G <= 96): word 0 = the bits at which the group's line
+//    starts, words 1..3 (96 bits, word 1 lowest) G fields of W = 96 / G bits,
+//    field k at bit k*W; v_k = word 0 - ((k * slope) >> 12) - field k.  Over a
+//    segment phi falls at a nearly constant rate (the slope, in 2^-12 ulps per
+//    entry), so a field only holds the library's rounding noise about the line.
 //  * split format (format bit 16, 2 <= G <= 255): the group holds at most
 //    three distinct values, words 0..2; word 3 holds s1 (bits 0..7) and s2
 //    (bits 8..15): v_k = word 0 for k < s1, word 1 for s1 <= k < s2, word 2
-//    from s2 on.  Used where y >= 2: there tanhf takes few values and phi
+//    from s2 on.  Used where y is large: there tanhf takes few values and phi
 //    jumps by more than a field holds.
 // Either way one 16-byte record read gives the value, and the decode is the
 // same instructions for both formats (both candidates are formed and one is
-// selected), so that lanes reading different binades do not diverge.  The
-// group of binade offset j is j / G = umulhi(j, ceil(2^32 / G)) (exact for
-// j < 2^23, G < 512).  The builder (libm_tables.cpp) picks the smallest
-// feasible layout per binade and checks every entry of the packed table
+// selected), so that lanes reading different segments do not diverge.  The
+// group of segment offset j is j / G = umulhi(j, ceil(2^32 / G)) (exact for
+// j < 2^19, G < 512).  The builder (libm_tables.cpp) picks the smallest
+// feasible layout per segment and checks every entry of the packed table
 // against the swept one.
-#define XL_PHI_BINADE_BITS 23
+#define XL_PHI_SEG_BITS 19
 #define XL_PHI_SPLIT 0x10000u
-#define XL_PHI_MAX_BINADES 64
+#define XL_PHI_MAX_SEGS 576
+#define XL_PHI_SLOPE_BITS 12
 
 XL_HD uint32_t xl_umulhi(uint32_t a, uint32_t b) {
 #if defined(__CUDA_ARCH__)
@@ -191,7 +193,7 @@ XL_HD uint32_t xl_umulhi(uint32_t a, uint32_t b) {
 #endif
 }
 
-// group of binade offset j, recip = ceil(2^32 / G)
+// group of segment offset j, recip = ceil(2^32 / G)
 XL_HD uint32_t xl_phi_group(uint32_t j, uint32_t recip) { return xl_umulhi(j, recip); }
 
 // field k of a record's words r1..r3; fmt = G | W << 8 (W = 0 in the split format: field 0)
@@ -208,9 +210,13 @@ XL_HD uint32_t xl_phi_field(uint32_t k, uint32_t fmt, uint32_t r1, uint32_t r2, 
 #endif
 }
 
+// fall of the line at entry k of a group
+XL_HD uint32_t xl_phi_fall(uint32_t k, uint32_t slope) { return (k * slope) >> XL_PHI_SLOPE_BITS; }
+
 // bits of entry k of a group from its record r0..r3 (both formats; xl_phi reads the record)
-XL_HD uint32_t xl_phi_decode_bits(uint32_t k, uint32_t fmt, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
-  const uint32_t delta = r0 - xl_phi_field(k, fmt, r1, r2, r3);
+XL_HD uint32_t xl_phi_decode_bits(uint32_t k, uint32_t fmt, uint32_t slope, uint32_t r0, uint32_t r1, uint32_t r2,
+                                  uint32_t r3) {
+  const uint32_t delta = r0 - xl_phi_fall(k, slope) - xl_phi_field(k, fmt, r1, r2, r3);
   const uint32_t split = k < (r3 & 0xffu) ? r0 : (k < ((r3 >> 8) & 0xffu) ? r1 : r2);
   return (fmt & XL_PHI_SPLIT) ? split : delta;
 }

@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(NT, MINB)
   __shared__ uint32_t s_ured[NT / 32];
   __shared__ LdCtl s_ctl;
   __shared__ int s_start, s_accepted, s_stop;
-  __shared__ uint4 s_pdesc[XL_PHI_MAX_BINADES];
+  __shared__ uint4 s_pdesc[XL_PHI_MAX_SEGS];
   const XlSmall xs = xl_small_global(xt);
   xl_phi_stage(xt, s_pdesc);
 

@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(1024, 1) ldpca_batch_kernel(LdpcaBatch A) {
   __shared__ uint32_t s_ured[32];
   __shared__ LdCtl s_ctl[4];
   __shared__ int s_item[4];
-  __shared__ uint4 s_pdesc[XL_PHI_MAX_BINADES];
+  __shared__ uint4 s_pdesc[XL_PHI_MAX_SEGS];
   xl_phi_stage(A.xt, s_pdesc);
   __syncthreads();
   {

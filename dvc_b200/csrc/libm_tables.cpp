@@ -226,9 +226,9 @@ void dvc_phi_build(float *out, uint32_t ylo, uint32_t y1, int threads) {
 
 bool dvc_phi_pack(const float *phi, uint32_t ylo, uint32_t y1, int threads, PhiPacked &out, char *err, int errlen) {
   if (threads <= 0) threads = hw_threads();
-  const uint32_t B = 1u << XL_PHI_BINADE_BITS;
+  const uint32_t B = 1u << XL_PHI_SEG_BITS;
   if ((ylo & (B - 1)) != 0 || y1 <= ylo) {
-    snprintf(err, errlen, "phi table range [%08x, %08x) does not start a binade", ylo, y1);
+    snprintf(err, errlen, "phi table range [%08x, %08x) does not start a segment", ylo, y1);
     return false;
   }
   const uint64_t n = (uint64_t)y1 - ylo;
@@ -244,43 +244,48 @@ bool dvc_phi_pack(const float *phi, uint32_t ylo, uint32_t y1, int threads, PhiP
       });
     for (auto &th : ts) th.join();
   };
-  // per binade: the smallest feasible layout.  Delta: G entries per record
-  // hold fields of W = 96 / G bits, so a group's span (bits(v_0) - bits of its
-  // last value, which needs the binade to be non-increasing) must stay below
-  // 2^W.  Split: every group may change value at most twice; G = 2 always fits.
-  std::vector<uint32_t> fmt(nb);
+  // per segment: the smallest feasible layout.  Line: the distance of every
+  // value below the line, shifted up so that none lies above it, must stay
+  // below 2^W.  Split: every group may change value at most twice; G = 2
+  // always fits.
+  std::vector<uint32_t> fmt(nb), slope(nb);
   std::vector<uint64_t> nrec(nb);
   pool([&](int b) {
     const uint64_t a = (uint64_t)b * B, e = std::min<uint64_t>(n, a + B), len = e - a;
-    std::vector<uint32_t> pre(len);  // changes in (a, a + t]
-    bool mono = true;
-    uint32_t c = 0;
-    pre[0] = 0;
-    for (uint64_t t = 1; t < len; t++) {
-      const uint32_t u0 = bits(a + t - 1), u1 = bits(a + t);
-      c += u1 != u0;
-      if (u1 > u0) mono = false;
-      pre[t] = c;
-    }
-    uint64_t best = ~0ull;
-    for (uint32_t G = 2; G <= 255; G++) {
-      const uint32_t W = 96 / G;
-      const uint64_t recs = (len + G - 1) / G;
-      uint64_t dmax = 0, rmax = 0;
-      for (uint64_t g0 = 0; g0 < len; g0 += G) {
-        const uint64_t g1 = std::min<uint64_t>(len, g0 + G) - 1;
-        dmax = std::max<uint64_t>(dmax, (uint64_t)bits(a + g0) - bits(a + g1));
-        rmax = std::max<uint64_t>(rmax, pre[g1] - pre[g0]);
+    const int64_t drop = (int64_t)bits(a) - (int64_t)bits(e - 1);
+    slope[b] = drop > 0 && len > 1 ? (uint32_t)std::min<int64_t>((drop << XL_PHI_SLOPE_BITS) / (int64_t)(len - 1), 1 << 23) : 0u;
+    for (uint32_t W = 1; W <= 16; W++) {
+      const uint32_t G = 96 / W;
+      if (W > 1 && 96 / (W - 1) == G) continue;
+      bool fits = true;
+      for (uint64_t g0 = a; g0 < e && fits; g0 += G) {
+        int64_t mn = INT64_MAX, mx = INT64_MIN;
+        for (uint32_t k = 0; k < G && g0 + k < e; k++) {
+          const int64_t r = (int64_t)bits(g0 + k) + xl_phi_fall(k, slope[b]);
+          mn = std::min(mn, r);
+          mx = std::max(mx, r);
+        }
+        fits = mx - mn < (1ll << W);
       }
-      if (G >= 4 && G <= 32 && mono && dmax <= ((1ull << W) - 1) && recs * 16 < best) {
-        best = recs * 16;
+      if (fits) {
         fmt[b] = G | (W << 8);
-        nrec[b] = recs;
+        nrec[b] = (len + G - 1) / G;
+        break;
       }
-      if (rmax <= 2 && recs * 16 < best) {
-        best = recs * 16;
+    }
+    for (uint32_t G = 255; G >= 2; G--) {
+      const uint64_t recs = (len + G - 1) / G;
+      if (fmt[b] && recs >= nrec[b]) break;
+      bool fits = true;
+      for (uint64_t g0 = a; g0 < e && fits; g0 += G) {
+        int changes = 0;
+        for (uint32_t k = 1; k < G && g0 + k < e; k++) changes += bits(g0 + k) != bits(g0 + k - 1);
+        fits = changes <= 2;
+      }
+      if (fits) {
         fmt[b] = G | XL_PHI_SPLIT;
         nrec[b] = recs;
+        break;
       }
     }
   });
@@ -296,6 +301,7 @@ bool dvc_phi_pack(const float *phi, uint32_t ylo, uint32_t y1, int threads, PhiP
     out.desc[4 * b] = (uint32_t)rec0[b];
     out.desc[4 * b + 1] = fmt[b];
     out.desc[4 * b + 2] = (uint32_t)(((1ull << 32) + G - 1) / G);
+    out.desc[4 * b + 3] = slope[b];
   }
   out.rec.assign((size_t)rec0[nb] * 4, 0);
   pool([&](int b) {
@@ -304,11 +310,10 @@ bool dvc_phi_pack(const float *phi, uint32_t ylo, uint32_t y1, int threads, PhiP
     const bool split = (fmt[b] & XL_PHI_SPLIT) != 0;
     uint32_t *rec = out.rec.data() + rec0[b] * 4;
     for (uint64_t g0 = a; g0 < e; g0 += G, rec += 4) {
-      rec[0] = bits(g0);
       if (split) {
         // up to three values; s1, s2 = the entries where the second and third start (G: never)
         uint32_t s1 = G, s2 = G, nv = 1;
-        rec[1] = rec[2] = rec[0];
+        rec[0] = rec[1] = rec[2] = bits(g0);
         for (uint32_t k = 1; k < G && g0 + k < e; k++) {
           if (bits(g0 + k) == bits(g0 + k - 1)) continue;
           if (nv == 1) {
@@ -323,8 +328,11 @@ bool dvc_phi_pack(const float *phi, uint32_t ylo, uint32_t y1, int threads, PhiP
         rec[3] = s1 | (s2 << 8);
         continue;
       }
-      for (uint32_t k = 1; k < G && g0 + k < e; k++) {
-        const uint32_t f = bits(g0) - bits(g0 + k);
+      uint32_t top = 0;
+      for (uint32_t k = 0; k < G && g0 + k < e; k++) top = std::max(top, bits(g0 + k) + xl_phi_fall(k, slope[b]));
+      rec[0] = top;
+      for (uint32_t k = 0; k < G && g0 + k < e; k++) {
+        const uint32_t f = top - xl_phi_fall(k, slope[b]) - bits(g0 + k);
         const uint32_t pos = k * W, wi = pos >> 5, sh = pos & 31u;
         rec[1 + wi] |= f << sh;
         if (sh + W > 32) rec[2 + wi] |= f >> (32 - sh);
@@ -335,10 +343,10 @@ bool dvc_phi_pack(const float *phi, uint32_t ylo, uint32_t y1, int threads, PhiP
   std::atomic<uint64_t> bad{0}, first_bad{~0ull};
   parallel_ranges(0, n - 1, threads, [&](int, uint64_t a, uint64_t e) {
     for (uint64_t i = a; i <= e; i++) {
-      const uint32_t *d = out.desc.data() + 4 * (i >> XL_PHI_BINADE_BITS);
+      const uint32_t *d = out.desc.data() + 4 * (i >> XL_PHI_SEG_BITS);
       const uint32_t j = (uint32_t)(i & (B - 1)), g = xl_phi_group(j, d[2]);
       const uint32_t *r = out.rec.data() + 4 * ((uint64_t)d[0] + g);
-      const uint32_t f = xl_phi_decode_bits(j - g * (d[1] & 0xffu), d[1], r[0], r[1], r[2], r[3]);
+      const uint32_t f = xl_phi_decode_bits(j - g * (d[1] & 0xffu), d[1], d[3], r[0], r[1], r[2], r[3]);
       if (f != bits(i)) {
         if (bad.fetch_add(1) == 0) first_bad = i;
       }
@@ -373,7 +381,7 @@ extern "C" int dvc_phi_table_check(size_t *packed_bytes, char *msg, int msglen) 
   size_t nsplit = 0;
   for (size_t b = 0; b < pk.desc.size() / 4; b++) nsplit += (pk.desc[4 * b + 1] & XL_PHI_SPLIT) != 0;
   if (msg && msglen > 0)
-    snprintf(msg, (size_t)msglen, "%zu entries in %zu binades, %zu records, %zu split binades", phi.size(),
+    snprintf(msg, (size_t)msglen, "%zu entries in %zu segments, %zu records, %zu split segments", phi.size(),
              pk.desc.size() / 4, pk.rec.size() / 4, nsplit);
   return 0;
 }

@@ -32,9 +32,9 @@ typedef struct {
   const uint32_t *log_tab;
   const uint32_t *exp_tab;
   // -logf(tanhf(y)) for y bits in [tanh_ylo, tanh_y1), packed (exact_libm.h):
-  const uint4 *phi_desc;  // per binade: first record, format, ceil(2^32 / G), 0
+  const uint4 *phi_desc;  // per segment: first record, format, ceil(2^32 / G), slope
   const uint4 *phi_rec;   // 16-byte records
-  int phi_nbin;           // binades (descriptors), at most XL_PHI_MAX_BINADES
+  int phi_nseg;           // segments (descriptors), at most XL_PHI_MAX_SEGS
   uint32_t log_mask, exp_mask;  // cap - 1
   int log_shift, exp_shift;     // 32 - log2(cap)
   uint32_t tanh_ylo, tanh_y1;
@@ -61,12 +61,12 @@ int dvc_libm_load(const char *path, XlmHost *out, char *err, int errlen);
 // out[i] = -logf(tanhf(y)) with the C library, y the float with bits ylo + i, i < y1 - ylo
 void dvc_phi_build(float *out, uint32_t ylo, uint32_t y1, int threads);
 
-// packed form of that table (exact_libm.h): desc holds 4 words per binade,
+// packed form of that table (exact_libm.h): desc holds 4 words per segment,
 // rec 4 words per record
 struct PhiPacked {
   std::vector<uint32_t> desc, rec;
 };
-// Packs phi[0 .. y1 - ylo) (ylo must start a binade) and checks every entry
+// Packs phi[0 .. y1 - ylo) (ylo must start a segment) and checks every entry
 // of the packed table against phi; returns false with a message on failure.
 bool dvc_phi_pack(const float *phi, uint32_t ylo, uint32_t y1, int threads, PhiPacked &out, char *err, int errlen);
 #endif
