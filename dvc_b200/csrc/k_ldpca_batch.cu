@@ -209,6 +209,9 @@ __global__ void __launch_bounds__(256) ldpca_batch_prep_kernel(LdpcaBatch A) {
     st.fin = 0;
     st.nsucc = 0;
     st.mask = 0ull;
+    // a slot that has been taken but not filled yet must not match the code
+    // an earlier batch left there
+    for (int s = 0; s < kSlots; s++) st.succ_code[s] = -1;
   }
   // a start at full rate has no BP item: finalise it here with the inverse
   __syncthreads();
