@@ -77,7 +77,8 @@ static int ldpca_run(Context &c, int n, int count, const float *lr, const uint8_
   const size_t nb = (size_t)n / 8;
   if (!c.ld_lr.ensure((size_t)count * n * 4) || !c.ld_acc.ensure((size_t)count * nb) ||
       !c.ld_dec.ensure((size_t)count * n) || !c.ld_res.ensure((size_t)count * 16) ||
-      !c.ld_ent.ensure((size_t)count * 4) || !c.ld_jobs.ensure((size_t)count * sizeof(dvc::LdpcaJob))) {
+      !c.ld_ent.ensure((size_t)count * 4) || !c.ld_jobs.ensure((size_t)count * sizeof(dvc::LdpcaJob)) ||
+      (llr_back && !c.ld_llr.ensure((size_t)count * n * 4))) {
     c.err = "device allocation failed";
     return DVC_E_NOMEM;
   }
@@ -96,10 +97,34 @@ static int ldpca_run(Context &c, int n, int count, const float *lr, const uint8_
       j.use_given_entropy = 1;
       j.given_entropy = given_entropy[i];
     }
-    if (llr_back) j.llr_out = c.ld_lr.as<float>() + (size_t)i * n;
+    if (llr_back) j.llr_out = c.ld_llr.as<float>() + (size_t)i * n;  // apart from lr, which other slots read
   }
   cudaStream_t s = c.stream;
   int st;
+  // Codewords that leave SMs idle are decoded with speculative slots (and
+  // clusters); beyond four per SM a block walks each ladder alone, without
+  // scratch.  One codeword alone, sequential -> so: QCIF 2.2
+  // -> 0.26 ms, CIF 7.9 -> 0.43 ms; 33 QCIF codewords 4.5 -> 0.89 ms, 203 CIF
+  // ones 19.8 -> 13.2 ms.
+  int sms = 148, K = 1, C = 1;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
+  dvc::LdpcaSpec sp;
+  if (count <= 4 * sms) {
+    dvc::ldpca_spec_shape(n, count, sms, K, C);
+    // once for every count (at most 4 * sms slots of either length by default)
+    const size_t had = c.ld_spec.bytes;
+    if (!c.ld_spec.ensure(std::max(dvc::ldpca_spec_scratch_bytes(6336, 4 * sms, 4),
+                                   dvc::ldpca_spec_scratch_bytes(n, count, K)))) {
+      c.err = "device allocation failed";
+      return DVC_E_NOMEM;
+    }
+    if (c.ld_spec.bytes != had) c.ld_spec_jobs = 0;
+    sp = dvc::ldpca_spec_carve(c.ld_spec.p, count, K, true);
+    if (c.ld_spec_jobs != count || c.ld_spec_k != K) {
+      c.ld_spec_jobs = 0;
+      if ((st = cuda_status(c, dvc::ldpca_spec_reset(sp, count, K, s), "LDPCA scratch"))) return st;
+    }
+  }
   if ((st = cuda_status(c, cudaMemcpyAsync(c.ld_lr.p, lr, (size_t)count * n * 4, cudaMemcpyHostToDevice, s), "H2D lr")))
     return st;
   if ((st = cuda_status(c, cudaMemcpyAsync(c.ld_acc.p, acc, (size_t)count * nb, cudaMemcpyHostToDevice, s), "H2D acc")))
@@ -108,7 +133,11 @@ static int ldpca_run(Context &c, int n, int count, const float *lr, const uint8_
                                            cudaMemcpyHostToDevice, s),
                         "H2D jobs")))
     return st;
-  if ((st = cuda_status(c, dvc::launch_ldpca(*L, c.ld_jobs.as<dvc::LdpcaJob>(), count, c.xlm, max_iter, s), "ldpca launch")))
+  c.ld_spec_jobs = 0;  // until the launch has run
+  if ((st = cuda_status(c,
+                        sp.best ? dvc::launch_ldpca_spec(*L, c.ld_jobs.as<dvc::LdpcaJob>(), count, c.xlm, max_iter, K, C, sp, s)
+                                : dvc::launch_ldpca(*L, c.ld_jobs.as<dvc::LdpcaJob>(), count, c.xlm, max_iter, s),
+                        "ldpca launch")))
     return st;
   if (decoded &&
       (st = cuda_status(c, cudaMemcpyAsync(decoded, c.ld_dec.p, (size_t)count * n, cudaMemcpyDeviceToHost, s), "D2H dec")))
@@ -119,10 +148,14 @@ static int ldpca_run(Context &c, int n, int count, const float *lr, const uint8_
       (st = cuda_status(c, cudaMemcpyAsync(entropy, c.ld_ent.p, (size_t)count * 4, cudaMemcpyDeviceToHost, s), "D2H ent")))
     return st;
   if (llr_back &&
-      (st = cuda_status(c, cudaMemcpyAsync(llr_back, c.ld_lr.p, (size_t)count * n * 4, cudaMemcpyDeviceToHost, s),
+      (st = cuda_status(c, cudaMemcpyAsync(llr_back, c.ld_llr.p, (size_t)count * n * 4, cudaMemcpyDeviceToHost, s),
                         "D2H llr")))
     return st;
   if ((st = cuda_status(c, cudaStreamSynchronize(s), "ldpca sync"))) return st;
+  if (sp.best) {
+    c.ld_spec_jobs = count;
+    c.ld_spec_k = K;
+  }
   return DVC_OK;
 }
 
@@ -613,7 +646,8 @@ extern "C" int dvc_session_create(dvc_ctx *ctx, int count, const dvc_wz_frame *f
   // batches: level by level, frames of a level in the caller's order, at most
   // max_batch per batch, streams assigned round-robin
   const int nlev = *std::max_element(level.begin(), level.end()) + 1;
-  std::vector<int> batch_of(count, -1);
+  std::vector<int> batch_of(count, -1), level_frames(nlev, 0);
+  for (int i = 0; i < count; i++) level_frames[level[i]]++;
   for (int lv = 0; lv < nlev; lv++) {
     std::vector<int> fl;
     for (int i = 0; i < count; i++)
@@ -679,8 +713,8 @@ extern "C" int dvc_session_create(dvc_ctx *ctx, int count, const dvc_wz_frame *f
       specs.push_back(sp);
     }
     cudaStream_t sb = S->streams[S->batch_stream[b]];
-    // frames decoding at once: one batch per stream
-    const int concurrent = std::min(count, nstreams * max_batch);
+    // frames decoding at once: those of the batch's level, one batch per stream
+    const int concurrent = std::min(level_frames[level[S->batch_frames[b][0]]], nstreams * max_batch);
     if (!S->batches[b].prepare(c, specs, sb, concurrent)) return bail(DVC_E_CUDA);
     if ((st = cuda_status(c, cudaStreamSynchronize(sb), "session prepare"))) return bail(st);
   }

@@ -202,6 +202,9 @@ void Context::release() {
   ld_res.release();
   ld_ent.release();
   ld_jobs.release();
+  ld_llr.release();
+  ld_spec.release();
+  ld_spec_jobs = ld_spec_k = 0;
   near_ties.release();
   for (DevBuf *b : {&bt_lr, &bt_acc, &bt_dec, &bt_res, &bt_ent, &bt_cw, &bt_state}) b->release();
   if (stream) cudaStreamDestroy(stream);

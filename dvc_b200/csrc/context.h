@@ -37,7 +37,8 @@ struct Context {
   std::vector<LadderGpu> ladders_gpu;
   cudaStream_t stream = nullptr;
   // scratch for the batched LDPCA entry point
-  DevBuf ld_lr, ld_acc, ld_dec, ld_res, ld_ent, ld_jobs;
+  DevBuf ld_lr, ld_acc, ld_dec, ld_res, ld_ent, ld_jobs, ld_llr, ld_spec;
+  int ld_spec_jobs = 0, ld_spec_k = 0;  // layout of ld_spec, which every launch leaves in its initial state
   // buffers of the batched LDPCA entry point (dvc_ldpca_decode_batch)
   DevBuf bt_lr, bt_acc, bt_dec, bt_res, bt_ent, bt_cw, bt_state;
   // count of reconstruction steps near a rounding tie (recon_kernel), one

@@ -39,6 +39,8 @@ struct LadderDev {
 struct LdpcaJob {
   int active;            // 0: the block returns at once (frame not in this step)
   const float *lr;       // [n] p0/p1 per 4x4 block (condBitProb output)
+  const float *llr_in;   // [n] log(p0/p1) and [n] entropy terms (ld_bit_terms) of lr,
+  const float *term_in;  //     when the caller has them; null: computed from lr
   const uint8_t *acc;    // [n/8] accumulated syndrome bytes, MSB first
   int crc;               // CRC-8 of the source bitplane
   uint8_t *decoded;      // [n] decoded bits (may be null)
@@ -54,10 +56,12 @@ struct LdpcaJob {
 };
 
 // Scratch of the speculative ladder form (k_ldpca.cu): per codeword the lowest
-// successful code, summed BP iterations and first code; per (codeword, block)
-// the code it succeeded with and its decoded bits.
+// successful code, summed BP iterations and first code; per (codeword, slot)
+// the code it succeeded with and its decoded bits; when wanted, the BP
+// iterations of every code tried ([64] per codeword, from the first code).
 struct LdpcaSpec {
   int *best = nullptr, *iters = nullptr, *start = nullptr, *done = nullptr, *slot_code = nullptr;
+  int *code_iters = nullptr;
   uint8_t *slot_dec = nullptr;
 };
 

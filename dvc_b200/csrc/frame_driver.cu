@@ -55,7 +55,7 @@ cudaError_t launch_side_info(FrameDev *fr, int nf, int w, int h, cudaStream_t s)
 cudaError_t launch_frame_prep(FrameDev *fr, int nf, int w, int h, cudaStream_t s);
 cudaError_t launch_noise_dist(FrameDev *fr, int nf, int max_nsir, const XlmDev &xt, int band, int max_range,
                               cudaStream_t s);
-cudaError_t launch_cond_bit(FrameDev *fr, int nf, int w, int h, int band, int bit, cudaStream_t s);
+cudaError_t launch_cond_bit(FrameDev *fr, int nf, int w, int h, const XlmDev &xt, int band, int bit, cudaStream_t s);
 cudaError_t launch_band_end(FrameDev *fr, int nf, int w, int h, int max_nsir, int band, const XlmDev &xt,
                             cudaStream_t s);
 cudaError_t launch_final_inverse(FrameDev *fr, int nf, int max_nsir, cudaStream_t s);
@@ -82,7 +82,7 @@ bool Slot::ensure(int w_, int h_, size_t pdf_floats, size_t in_bytes, size_t out
   const size_t fs = (size_t)w_ * h_, n = fs / 16;
   const size_t b16n = fs / 256, b8n = fs / 64, octn = (size_t)(w_ - 3) * (h_ - 3) * 16;
   bool ok = si.ensure(fs, a) && dbf.ensure(fs, a) && residue.ensure(fs * 4, a) && side_trans.ensure(fs * 4, a) &&
-            recons_trans.ensure(fs * 4, a) && alpha.ensure(fs * 4, a) && lr.ensure(n * 4, a) &&
+            recons_trans.ensure(fs * 4, a) && alpha.ensure(fs * 4, a) && lr.ensure(3 * n * 4, a) &&
             oct.ensure(octn * 2, a) && smf.ensure(n * 81 * 4, a) && pdf.ensure(pdf_floats * 4, a) &&
             mb_mv.ensure(b16n * sizeof(MVd), a) && fmv.ensure(b16n * sizeof(MVd), a) &&
             blk_mv.ensure(b8n * sizeof(MVd), a) && blk_mv2.ensure(b8n * sizeof(MVd), a) && holes.ensure(b16n * 16, a) &&
@@ -190,7 +190,12 @@ bool FrameBatcher::prepare(Context &ctx, const std::vector<FrameSpec> &frames, c
       if (coded) maxbits = std::max(maxbits, kQBits[frames[f].qindex][kZigzag[band]]);
     }
     if (maxbits == 0) break;
-    for (int bit = maxbits; bit >= 1; bit--) steps.push_back({band, bit});
+    for (int bit = maxbits; bit >= 1; bit--) {
+      Step st;
+      st.band = band;
+      st.bit = bit;
+      steps.push_back(st);
+    }
   }
   const size_t jobs_off = pinned_need;
   pinned_need += align16(sizeof(LdpcaJob) * steps.size() * nf);
@@ -298,6 +303,8 @@ bool FrameBatcher::prepare(Context &ctx, const std::vector<FrameSpec> &frames, c
     D.si_mv = S.si_mv.as<int>();
     D.pdf = S.pdf.as<float>();
     D.lr = S.lr.as<float>();
+    D.llr = D.lr + n;
+    D.term = D.llr + n;
     D.oct = S.oct.as<int16_t>();
     D.mb_mv = S.mb_mv.as<MVd>();
     D.fmv = S.fmv.as<MVd>();
@@ -350,6 +357,8 @@ bool FrameBatcher::prepare(Context &ctx, const std::vector<FrameSpec> &frames, c
       Slot &S = slots_[f];
       J.active = 1;
       J.lr = fd[f].lr;
+      J.llr_in = fd[f].llr;
+      J.term_in = fd[f].term;
       J.acc = S.in.as<uint8_t>() + pk[f].acc + (size_t)plane * nb;
       J.crc = frames[f].crc[plane];
       J.result = S.out.as<int>() + plane * 4;
@@ -367,21 +376,17 @@ bool FrameBatcher::prepare(Context &ctx, const std::vector<FrameSpec> &frames, c
                    "H2D jobs"))
     return false;
 
-  // speculative ladder width: spread each codeword over idle SMs when the batch is small
+  // speculative slots and blocks per slot of every step
   {
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device);
-    // speculation pays even on a full GPU (it shortens the slowest codeword of
-    // every lockstep bitplane step); on the bench's 640 CIF frames the
-    // autotuner measured 4 blocks per codeword fastest (911 ms a step, against
-    // 956 at 8, 966 at 2 and 1168 at 1); at least 4 blocks per codeword, more
-    // when SMs are idle.  DVC_LDPCA_SPEC_FLOOR replaces the floor of 4 (the
-    // autotuner's setting), DVC_LDPCA_SPEC fixes the width outright
-    int floor_k = 4;
-    if (const char *e = getenv("DVC_LDPCA_SPEC_FLOOR")) floor_k = std::max(1, std::min(32, atoi(e)));
-    int k = std::max(floor_k, sms / std::max(1, std::max(nf, concurrent)));
-    if (const char *e = getenv("DVC_LDPCA_SPEC")) k = atoi(e);
-    spec_k_ = std::max(1, std::min(32, k));
+    spec_k_ = 1;
+    for (size_t si = 0; si < steps.size(); si++) {
+      int active = 0;
+      for (int f = 0; f < nf; f++) active += plane_of_[si * nf + f] >= 0;
+      ldpca_spec_shape(n, (int)((long long)active * std::max(nf, concurrent) / nf), sms, steps[si].spec_k, steps[si].spec_c);
+      spec_k_ = std::max(spec_k_, steps[si].spec_k);
+    }
     if (!spec_.ensure(ldpca_spec_scratch_bytes(n, nf, spec_k_), alloc_stream_))
       return ctx.fail("device allocation failed");
     if (!ctx.cuda_ok(ldpca_spec_reset(ldpca_spec_carve(spec_.p, nf, spec_k_), nf, spec_k_, s), "LDPCA scratch"))
@@ -453,7 +458,7 @@ bool FrameBatcher::execute(Context &ctx, cudaStream_t s, int max_iter, ProfileSt
     if (!ctx.cuda_ok(launch_noise_dist(fdev, nf, max_nsir, ctx.xlm, band, max_range, s), "noise distribution"))
       return false;
     for (; si < steps.size() && steps[si].band == band; si++) {
-      if (!ctx.cuda_ok(launch_cond_bit(fdev, nf, w, h, band, steps[si].bit, s), "conditional bit probability"))
+      if (!ctx.cuda_ok(launch_cond_bit(fdev, nf, w, h, ctx.xlm, band, steps[si].bit, s), "conditional bit probability"))
         return false;
       for (int f = 0; f < nf; f++)
         if (frames[f].dbg_lr && plane_of_[si * nf + f] >= 0) {
@@ -464,7 +469,7 @@ bool FrameBatcher::execute(Context &ctx, cudaStream_t s, int max_iter, ProfileSt
             return false;
         }
       if (prof) cudaEventRecord(ev_[ev_used_], s);
-      if (!ctx.cuda_ok(launch_ldpca_spec(*L, jobs_dev_.as<LdpcaJob>() + si * nf, nf, ctx.xlm, max_iter, spec_k_,
+      if (!ctx.cuda_ok(launch_ldpca_spec(*L, jobs_dev_.as<LdpcaJob>() + si * nf, nf, ctx.xlm, max_iter, steps[si].spec_k, steps[si].spec_c,
                                          ldpca_spec_carve(spec_.p, nf, spec_k_), s),
                        "LDPCA"))
         return false;

@@ -97,7 +97,7 @@ class FrameBatcher {
   std::vector<Slot> slots_;
   DevBuf frames_dev_, jobs_dev_, spec_;
   cudaStream_t alloc_stream_ = nullptr;
-  int spec_k_ = 1;
+  int spec_k_ = 1;  // most speculative slots per codeword of any step (the scratch's layout)
   void *pinned_ = nullptr;
   size_t pinned_bytes_ = 0;
   std::vector<void *> retired_pinned_;  // outgrown pinned buffers, freed by release()
@@ -105,6 +105,7 @@ class FrameBatcher {
   // prepared state
   struct Step {
     int band, bit;
+    int spec_k = 1, spec_c = 1;  // speculative slots per codeword, blocks per slot
   };
   std::vector<Step> steps_;
   std::vector<FrameDev> fd_;

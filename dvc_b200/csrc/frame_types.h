@@ -22,7 +22,8 @@ struct FrameDev {
   // state and outputs
   uint8_t *recon, *si, *dbf;
   int *residue, *side_trans, *recons_trans;
-  float *alpha, *smf, *pdf, *lr;
+  float *alpha, *smf, *pdf;
+  float *lr, *llr, *term;     // [w*h/16] likelihood ratios of the current bitplane, their logs, their entropy terms
   int *si_mv;                 // [2*nsir] last refinement's best candidate index, past then future (-1: none)
   int16_t *oct;               // [(h-3)*(w-3)*16] over-complete transform of the side information
   MVd *mb_mv, *fmv, *blk_mv, *blk_mv2;

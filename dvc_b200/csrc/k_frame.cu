@@ -15,6 +15,7 @@
 #include "dvc_common.cuh"
 #include "frame_types.h"
 #include "kernels.h"
+#include "ldpca_bp.cuh"
 
 namespace dvc {
 
@@ -909,15 +910,21 @@ __device__ __forceinline__ void interval_sums(const float *p, int lo0, int hi0, 
 // condBitProb, noiseModel.cpp:191-310: LR = p0/p1 from sequential interval
 // sums of the pdf, one thread per 4x4 block.  Non-WZ blocks get the
 // reference's certain-zero ratio when the frame has skip or intra blocks.
-__global__ void cond_bit_kernel(FrameDev *frames, int band, int bit) {
+// Beside each ratio go its logarithm and its term of the entropy bound, which
+// every speculative block of the ladder would otherwise compute again.
+__global__ void cond_bit_kernel(FrameDev *frames, XlmDev xt, int band, int bit) {
   FrameDev &F = frames[blockIdx.y];
   if (!F.active || !in_step(F, band, bit)) return;
   const int w = F.w, b4w = w / 4, b4n = b4w * (F.h / 4);
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= b4n) return;
+  const XlSmall xs = xl_small_global(xt);
   const int s_idx = F.sir_of_blk[k];
   if (s_idx < 0) {
     if (F.skip_mode == 1 || F.intra_mode == 1) F.lr[k] = 0.9999f / 0.0001f;
+    const float lr = F.lr[k];
+    F.llr[k] = xl_logf(xt, xs, lr);
+    F.term[k] = ld_entropy_term(lr, xt, xs);
     return;
   }
   const int index = c_zigzag[band], step = F.step[index], range = F.crange[index];
@@ -956,6 +963,8 @@ __global__ void cond_bit_kernel(FrameDev *frames, int band, int bit) {
   else
     lr = p0 / p1;
   F.lr[k] = lr;
+  F.llr[k] = xl_logf(xt, xs, lr);
+  F.term[k] = ld_entropy_term(lr, xt, xs);
 }
 
 // ------------------------------------------------------- reconstruction
@@ -1647,8 +1656,8 @@ cudaError_t launch_noise_dist(FrameDev *fr, int nf, int max_nsir, const XlmDev &
   return cudaGetLastError();
 }
 
-cudaError_t launch_cond_bit(FrameDev *fr, int nf, int w, int h, int band, int bit, cudaStream_t s) {
-  cond_bit_kernel<<<g2((w / 4) * (h / 4), 128, nf), 128, 0, s>>>(fr, band, bit);
+cudaError_t launch_cond_bit(FrameDev *fr, int nf, int w, int h, const XlmDev &xt, int band, int bit, cudaStream_t s) {
+  cond_bit_kernel<<<g2((w / 4) * (h / 4), 128, nf), 128, 0, s>>>(fr, xt, band, bit);
   return cudaGetLastError();
 }
 

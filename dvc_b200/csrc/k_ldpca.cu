@@ -29,6 +29,9 @@
 // in ldpca_bp.cuh.
 #include <cuda_runtime.h>
 
+#include <stdlib.h>
+
+#include <algorithm>
 #include <atomic>
 
 #include "dvc_common.cuh"
@@ -38,71 +41,97 @@
 
 namespace dvc {
 
-// One thread block of NT threads per (codeword, speculative slot), each thread
-// holding MAXC = ceil(n / NT) columns, MINB blocks per SM.  By default NT = 1024 for both lengths
-// (CIF: one block per SM, 102 KB of shared memory; QCIF: 27 KB, 5 edges per
-// thread); QCIF codewords can also run with 256 or 512 threads, four or two
-// blocks per SM (the autotuner measures which is faster).
-template <int NT, int MAXC, int MINB>
+// One thread block of NT threads per (codeword, speculative slot), or a cluster
+// of C of them, each thread holding MAXC = ceil(n / (C * NT)) columns, MINB
+// blocks per SM.  Alone NT = 1024 for both lengths (CIF: one block per SM, 105
+// KB of shared memory; QCIF: 27 KB); QCIF codewords can also run with 256 or
+// 512 threads, four or two blocks per SM (the autotuner measures which is faster).
+template <int NT, int MAXC, int MINB, int C>
 __global__ void __launch_bounds__(NT, MINB)
     ldpca_ladder_kernel(LadderDev L, const LdpcaJob *__restrict__ jobs, XlmDev xt, int max_iter, int K,
                         LdpcaSpec sp) {
   extern __shared__ __align__(16) uint8_t smem[];
-  const int j = blockIdx.x / K, kk = blockIdx.x - j * K;
+  // codeword j and its speculative slot kk: the first slots of all codewords
+  // come first, so that blocks waiting for an SM are those of later codes
+  const int unit = blockIdx.x / C, nj = gridDim.x / (C * K);
+  const int kk = unit / nj, j = unit - kk * nj, slot = j * K + kk;
   const LdpcaJob J = jobs[j];
   if (!J.active) return;
   const bool spec = sp.best != nullptr;
-  const LdGroup<NT, true> g{(int)threadIdx.x, 0, 0};
+  using G = LdGroup<NT, true, C>;
+  const G g{(int)threadIdx.x, 0, C > 1 ? (int)blockIdx.x - unit * C : 0};
   const int n = L.n, tid = threadIdx.x;
+  const bool lead = tid == 0 && g.rank == 0;
   const LdSmem S = ld_carve(smem, L);
   __shared__ uint32_t s_ured[NT / 32];
   __shared__ LdCtl s_ctl;
-  __shared__ int s_start, s_accepted, s_stop;
+  __shared__ int s_word[4];  // broadcast words: late, start code, then stop flags in turn
   __shared__ uint4 s_pdesc[XL_PHI_MAX_SEGS];
   const XlSmall xs = xl_small_global(xt);
   xl_phi_stage(xt, s_pdesc);
+  if constexpr (C > 1) g.sync_all();  // every block of the cluster has started
+  const int last = L.num_codes - 1;
+  int total_iters = 0, accepted = last, start = 0;
+  // a slot that starts after its codeword has been decoded by a lower code
+  // than its own has nothing to do
+  bool late = false;
+  if (spec && kk > 0 && kk < K - 1) {  // the last slot reports the bound
+    int l = 0;
+    if (lead) {
+      const int best = *(volatile int *)(sp.best + j);
+      __threadfence();
+      l = best != LDPCA_NONE && *(volatile int *)(sp.start + j) + kk > best;
+    }
+    late = g.bcast(l, &s_word[0]) != 0;
+    if (late) start = *(volatile int *)(sp.start + j);
+  }
+  if (!late) {
 
   // accumulated syndrome bits (ByteToBit, LdpcaDecoder.cpp:81-107), log LR and
   // the entropy terms (ComputeCE), the bound as a sequential sum in block order
-  float llr[MAXC];
-  ld_llr(g, n, J.lr, xt, xs, llr, S.msg, (J.llr_out && kk == 0) ? J.llr_out : nullptr);
+  float llr[MAXC], part = 0.0f;
+  ld_llr(g, n, J.lr, xt, xs, llr, S.msg, (J.llr_out && kk == 0) ? J.llr_out : nullptr, J.llr_in, J.term_in, &part);
   ld_stage_acc(g, J.acc, n, S.accs);
-  g.sync();
-  if (tid == 0) {
-    float h = ld_entropy_sum(S.msg, n);
-    if (J.use_given_entropy) h = J.given_entropy;
-    const int start = ld_start_code(L, h);
-    s_start = start;
-    s_accepted = L.num_codes - 1;
-    if (kk == 0) {
-      if (J.entropy) *J.entropy = h;
-      if (spec) sp.start[j] = start;
+  // The bound itself is only needed where it is reported (by the slot with the
+  // least likely code, whose delay matters least) and when the parallel sum
+  // leaves the start code open.
+  start = J.use_given_entropy ? ld_start_code(L, J.given_entropy) : ld_start_near(g, L, part, s_ured, &s_ctl);
+  if (start < 0 || kk == K - 1) {
+    g.sync_all();
+    int exact = start;
+    if (lead) {
+      const float h = ld_entropy_sum(S.msg, n);
+      if (exact < 0) exact = ld_start_code(L, h);
+      if (J.entropy && kk == K - 1) *J.entropy = J.use_given_entropy ? J.given_entropy : h;
     }
+    start = g.bcast(exact, &s_word[1]);
   }
-  g.sync();
-  const int start = s_start;
-  const int last = L.num_codes - 1;
-  int total_iters = 0;
+  if (spec && lead) *(volatile int *)(sp.start + j) = start;  // the same in every slot
   volatile int *bestp = spec ? sp.best + j : nullptr;
 
+  int turn = 0;
   for (int code = start + kk; code < last; code += K) {
     if (spec) {
-      if (tid == 0) s_stop = *bestp < code;
-      g.sync();
-      if (s_stop) break;
+      if (g.bcast(lead && *bestp < code, &s_word[2 + turn])) break;
+      turn ^= 1;
     }
     int it = 0;
     uint32_t dm = 0;
     const int ok = ld_try_code(g, L, code, llr, J.crc, xt, s_pdesc, max_iter, bestp, S, s_ured, &s_ctl, it, dm);
     total_iters += it;
+    if (spec && sp.code_iters && lead) sp.code_iters[j * 64 + code - start] = it;
     if (ok) {
-      if (tid == 0) s_accepted = code;
+      accepted = code;
       if (spec) {
-        uint8_t *slot = sp.slot_dec + (size_t)blockIdx.x * n;
-        for (int k = tid; k < n; k += NT) slot[k] = S.dec[k];
-        g.sync();
-        if (tid == 0) {
-          sp.slot_code[blockIdx.x] = code;
+        uint8_t *dec = sp.slot_dec + (size_t)slot * n;
+        for (int c = 0; c < MAXC; c++) {
+          const int k = g.col(n, c);
+          if (k < n) dec[k] = (uint8_t)((dm >> c) & 1u);
+        }
+        __threadfence();
+        g.sync_all();
+        if (lead) {
+          sp.slot_code[slot] = code;
           __threadfence();
           atomicMin(sp.best + j, code);
         }
@@ -110,35 +139,46 @@ __global__ void __launch_bounds__(NT, MINB)
       break;
     }
   }
+  }
   if (spec) {
-    // the last of the codeword's K blocks to finish writes its result: the
-    // lowest successful code (or the full-rate inverse when no code below it
-    // succeeded), then puts the codeword's scratch back to its initial state
+    // the last of the codeword's K slots to finish writes its result (in a
+    // cluster its first block does): the lowest successful code (or the
+    // full-rate code when no code below it succeeded), then puts the
+    // codeword's scratch back to its initial state
     // for the next launch (no memset between the steps of a batch)
-    __shared__ int s_slot, s_iters;
-    g.sync();
+    __shared__ int s_last, s_slot, s_iters, s_acc;
+    g.sync_all();  // nothing in a block's shared memory is read by another one after this
+    if (C > 1 && g.rank != 0) return;
     if (tid == 0) {
       atomicAdd(sp.iters + j, total_iters);
       __threadfence();
-      s_stop = atomicAdd(sp.done + j, 1) == K - 1;
+      s_last = atomicAdd(sp.done + j, 1) == K - 1;
     }
-    g.sync();
-    if (!s_stop) return;
+    __syncthreads();
+    if (!s_last) return;
     __threadfence();
     if (tid == 0) {
       const int best = __ldcg(sp.best + j);
-      int acc = last, slot = -1;
+      int acc = last, from = -1;
       if (best != LDPCA_NONE && best < last)
         for (int k = 0; k < K; k++)
           if (__ldcg(sp.slot_code + j * K + k) == best) {
-            slot = k;
+            from = k;
             acc = best;
           }
-      s_accepted = acc;
-      s_slot = slot;
-      s_iters = __ldcg(sp.iters + j);
+      s_acc = acc;
+      s_slot = from;
+      // the BP iterations of the sequential ladder (every code up to the
+      // accepted one ran to its end), or those of every code tried
+      int iters = 0;
+      if (sp.code_iters)
+        for (int c = start; c <= min(acc, last - 1); c++) iters += __ldcg(sp.code_iters + j * 64 + c - start);
+      else
+        iters = __ldcg(sp.iters + j);
+      s_iters = iters;
     }
-    g.sync();
+    __syncthreads();
+    accepted = s_acc;
     if (s_slot >= 0) {
       const uint8_t *src = sp.slot_dec + (size_t)(j * K + s_slot) * n;
       for (int k = tid; k < n; k += NT) S.dec[k] = __ldcg(src + k);
@@ -151,11 +191,9 @@ __global__ void __launch_bounds__(NT, MINB)
       sp.done[j] = 0;
     }
   }
-  g.sync();
-  const int accepted = s_accepted;
-  if (accepted == last) {
-    ld_full_rate(g, L, S);
-  }
+  __syncthreads();
+  const LdGroup<NT, true> b{tid, 0, 0};
+  if (accepted == last) ld_full_rate(b, L, S);
   if (tid == 0) {
     J.result[0] = L.synd_len[accepted] + 8;
     J.result[1] = start;
@@ -164,7 +202,7 @@ __global__ void __launch_bounds__(NT, MINB)
   }
   if (J.decoded)
     for (int k = tid; k < n; k += NT) J.decoded[k] = S.dec[k];
-  if (J.recons_trans) ld_put_bitplane(g, J, S.dec, n);
+  if (J.recons_trans) ld_put_bitplane(b, J, S.dec, n);
 }
 
 // the L2 persisting window of the table reads (set when a context is created;
@@ -189,10 +227,11 @@ unsigned phi_window_attr(cudaLaunchAttribute &a) {
   return 1;
 }
 
-template <int NT, int MAXC, int MINB>
+template <int NT, int MAXC, int MINB, int C = 1>
 static cudaError_t launch_nt(const LadderDev &L, const LdpcaJob *jobs, int num_jobs, const XlmDev &xt, int max_iter,
                              int K, const LdpcaSpec &sp, cudaStream_t stream) {
-  if (L.n > LDPCA_MAX_N || LDPCA_COLS(L.n, NT) > MAXC) return cudaErrorInvalidValue;
+  if (L.n > LDPCA_MAX_N || LDPCA_COLS(L.n, NT * C) > MAXC) return cudaErrorInvalidValue;
+  auto kernel = ldpca_ladder_kernel<NT, MAXC, MINB, C>;
   const size_t smem = ldpca_smem_bytes(L.n, L.pos_max);
   // the attributes are per device: set them once for each device
   static std::atomic<uint64_t> attr_set{0};
@@ -201,28 +240,33 @@ static cudaError_t launch_nt(const LadderDev &L, const LdpcaJob *jobs, int num_j
   if (e != cudaSuccess) return e;
   const uint64_t bit = 1ull << (dev & 63);
   if (!(attr_set.load() & bit)) {
-    e = cudaFuncSetAttribute(ldpca_ladder_kernel<NT, MAXC, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     // the smallest shared-memory split that holds the blocks an SM runs (MINB
     // of them), so that the rest of the SM's 256 KB is L1 for the
     // phi records, which BP iterations re-read (percent of the 228 KB maximum;
     // the driver rounds up to a supported split)
-    const size_t need = (size_t)MINB * (smem + 4096);
+    const size_t need = (size_t)MINB * (smem + 12 * 1024);  // with the descriptors and the block's own
     const int pct = (int)((need * 100 + 228 * 1024 - 1) / (228 * 1024));
-    e = cudaFuncSetAttribute(ldpca_ladder_kernel<NT, MAXC, MINB>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             pct > 100 ? 100 : pct);
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct > 100 ? 100 : pct);
     if (e != cudaSuccess) return e;
     attr_set.fetch_or(bit);
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(num_jobs * K);
+  cfg.gridDim = dim3(num_jobs * K * C);
   cfg.blockDim = dim3(NT);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   cfg.attrs = attr;
   cfg.numAttrs = phi_window_attr(attr[0]);
-  return cudaLaunchKernelEx(&cfg, ldpca_ladder_kernel<NT, MAXC, MINB>, L, jobs, xt, max_iter, K, sp);
+  if (C > 1) {
+    cudaLaunchAttribute &a = attr[cfg.numAttrs++];
+    a.id = cudaLaunchAttributeClusterDimension;
+    a.val.clusterDim.x = C;
+    a.val.clusterDim.y = a.val.clusterDim.z = 1;
+  }
+  return cudaLaunchKernelEx(&cfg, kernel, L, jobs, xt, max_iter, K, sp);
 }
 
 // threads per codeword block: CIF 1024 (or 512), QCIF 1024 (or 256, 512)
@@ -251,11 +295,40 @@ cudaError_t launch_ldpca(const LadderDev &L, const LdpcaJob *jobs_dev, int num_j
   return launch_shape(L, jobs_dev, num_jobs, xt, max_iter, 1, none, stream);
 }
 
-size_t ldpca_spec_scratch_bytes(int n, int num_jobs, int K) {
-  return (size_t)num_jobs * 16 + (size_t)num_jobs * K * 4 + (size_t)num_jobs * K * n + 64;
+// Slots beyond those the SMs hold at once cost little (they start in code order
+// and find their codeword decoded), and hard codewords need many: four times
+// the SMs, at least 4 and at most 32 slots a codeword.  Measured with once,
+// twice and four times the SMs: three GOP-8 QCIF streams 147, 114, 106 ms, four
+// GOP-4 CIF streams 246, 196, 183 ms, 54 mixed requests 57, 48, 48 ms; 64 slots
+// instead of 32 slow a lone frame by 0.1-0.3 ms.  When fewer codewords are
+// active than the SMs could serve, a slot is a cluster of C blocks: a BP
+// iteration on 1, 2, 4 and 8 blocks takes 46, 35, 21 and 13 K cycles at CIF and
+// 13, 11, 8.3 and 7.8 K at QCIF (a remote store per edge, and the latency of two
+// table gathers, do not shrink with C).  So CIF keeps four slots per codeword
+// resident (a lone CIF frame 11.5 -> 6.5 ms at C = 8, four frames 24 -> 12 ms,
+// eleven at QIndex 8 80 -> 73 ms at C = 2; six or three slots instead of four:
+// four frames 14.6 or 12.3 ms), and QCIF, which gains less, sixteen (a lone
+// frame 3.45 -> 3.04 ms at C = 4; with eight, the three QCIF streams lose 5%).
+// DVC_LDPCA_SPEC_FLOOR replaces the least number of slots (the autotuner's
+// setting), DVC_LDPCA_SPEC fixes it outright.
+void ldpca_spec_shape(int n, int active, int sms, int &K, int &C) {
+  const int N = std::max(1, active);
+  const bool small = n < LDPCA_MAX_N;
+  const int resident = small ? 16 : 4;
+  C = small ? 4 : 8;
+  while (C > 1 && N * C * resident > sms) C /= 2;
+  int least = 4;
+  if (const char *e = getenv("DVC_LDPCA_SPEC_FLOOR")) least = std::max(1, std::min(32, atoi(e)));
+  K = std::max(least, 4 * sms / (N * C));
+  if (const char *e = getenv("DVC_LDPCA_SPEC")) K = atoi(e);
+  K = std::max(1, std::min(32, K));
 }
 
-LdpcaSpec ldpca_spec_carve(void *base, int num_jobs, int K) {
+size_t ldpca_spec_scratch_bytes(int n, int num_jobs, int K) {
+  return (size_t)num_jobs * 16 + (size_t)num_jobs * K * 4 + (size_t)num_jobs * K * n + (size_t)num_jobs * 256 + 64;
+}
+
+LdpcaSpec ldpca_spec_carve(void *base, int num_jobs, int K, bool code_iters) {
   LdpcaSpec sp;
   uint8_t *p = (uint8_t *)base;
   sp.best = (int *)p;
@@ -268,6 +341,8 @@ LdpcaSpec ldpca_spec_carve(void *base, int num_jobs, int K) {
   p += (size_t)num_jobs * 4;
   sp.slot_code = (int *)p;
   p += (size_t)num_jobs * K * 4;
+  if (code_iters) sp.code_iters = (int *)p;
+  p += (size_t)num_jobs * 256;
   sp.slot_dec = p;
   return sp;
 }
@@ -281,8 +356,15 @@ cudaError_t ldpca_spec_reset(const LdpcaSpec &sp, int num_jobs, int K, cudaStrea
 }
 
 cudaError_t launch_ldpca_spec(const LadderDev &L, const LdpcaJob *jobs_dev, int num_jobs, const XlmDev &xt,
-                              int max_iter, int K, const LdpcaSpec &sp, cudaStream_t stream) {
+                              int max_iter, int K, int C, const LdpcaSpec &sp, cudaStream_t stream) {
   if (num_jobs <= 0) return cudaSuccess;
+  // threads per block: the columns of a block in whole rounds
+  if (L.n == 1584 && C == 4) return launch_nt<416, 1, 1, 4>(L, jobs_dev, num_jobs, xt, max_iter, K, sp, stream);
+  if (L.n == 1584 && C == 2) return launch_nt<800, 1, 1, 2>(L, jobs_dev, num_jobs, xt, max_iter, K, sp, stream);
+  if (L.n == 6336 && C == 8) return launch_nt<800, 1, 1, 8>(L, jobs_dev, num_jobs, xt, max_iter, K, sp, stream);
+  if (L.n == 6336 && C == 4) return launch_nt<800, 2, 1, 4>(L, jobs_dev, num_jobs, xt, max_iter, K, sp, stream);
+  if (L.n == 6336 && C == 2) return launch_nt<800, 4, 1, 2>(L, jobs_dev, num_jobs, xt, max_iter, K, sp, stream);
+  if (C != 1) return cudaErrorInvalidValue;
   return launch_shape(L, jobs_dev, num_jobs, xt, max_iter, K, sp, stream);
 }
 

@@ -194,10 +194,7 @@ __global__ void __launch_bounds__(256) ldpca_batch_prep_kernel(LdpcaBatch A) {
   const XlSmall xs = xl_small_global(A.xt);
   const float *lr = A.lr + C.lr_off;
   for (int k = threadIdx.x; k < n; k += blockDim.x) {
-    const float v = lr[k];
-    const float pco = v / (1.0f + v);
-    const float tmp = xl_logf(A.xt, xs, 1.0f - pco);
-    terms[k] = (pco * (-xl_logf(A.xt, xs, pco) + tmp) - tmp) / LDPCA_LOG2;
+    terms[k] = ld_entropy_term(lr[k], A.xt, xs);
   }
   __syncthreads();
   LdpcaBatchState &st = A.state[j];
@@ -296,7 +293,7 @@ cudaError_t launch_ldpca_batch(LdpcaBatch A, int count, int grid, cudaStream_t s
   if (!(attr_set.load() & bit)) {
     e = cudaFuncSetAttribute(ldpca_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    const int pct = (int)(((smem + 4096) * 100 + 228 * 1024 - 1) / (228 * 1024));
+    const int pct = (int)(((smem + 12 * 1024) * 100 + 228 * 1024 - 1) / (228 * 1024));
     e = cudaFuncSetAttribute(ldpca_batch_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
     if (e != cudaSuccess) return e;
     attr_set.fetch_or(bit);

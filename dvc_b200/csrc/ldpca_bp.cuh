@@ -148,6 +148,21 @@ struct LdGroup {
     else
       sync();
   }
+  // the value v of the leading thread (t = 0 of rank 0) in every thread,
+  // through the word *w of each block; ends in no barrier, so a word is reused
+  // only after a later one
+  __device__ __forceinline__ int bcast(int v, int *w) const {
+    if (t == 0 && rank == 0) {
+      if constexpr (C_ > 1) {
+#pragma unroll
+        for (int b = 0; b < C_; b++) ld_st_cluster(ld_mapa((uint32_t)__cvta_generic_to_shared(w), b), (uint32_t)v);
+      } else {
+        *w = v;
+      }
+    }
+    sync_all();
+    return *(volatile int *)w;
+  }
   // sync_all that also returns whether any thread passed p != 0; `ph`
   // alternates between calls
   __device__ __forceinline__ int sync_or(int p, LdCtl *ctl, int ph) const {
@@ -285,24 +300,38 @@ __device__ __forceinline__ void ld_full_rate(const G &g, const LadderDev &L, con
   ld_invh_decode(g, L, synd, S.dec, sw);
 }
 
-// log LR of the group's columns into registers (LdpcaDecoder.cpp:665-666) and,
-// when want_entropy, the entropy terms H_k = (P(-log P + log(1-P)) - log(1-P))
-// / LOG2 with P = LR/(1+LR) (ComputeCE) into `terms` (n floats of shared memory).
+// log LR of a bit (LdpcaDecoder.cpp:665-666) and its term of the entropy bound,
+// (P(-log P + log(1-P)) - log(1-P)) / LOG2 with P = LR/(1+LR) (ComputeCE)
+__device__ __forceinline__ float ld_entropy_term(float lr, const XlmDev &xt, const XlSmall &xs) {
+  const float pco = lr / (1.0f + lr);
+  const float tmp = xl_logf(xt, xs, 1.0f - pco);
+  return (pco * (-xl_logf(xt, xs, pco) + tmp) - tmp) / LDPCA_LOG2;
+}
+
+// log LR of the group's columns into registers and,
+// when wanted, the entropy terms into `terms` (n floats of shared memory, in a
+// cluster those of its first block, whose every block has started) and the sum
+// of the thread's own added to *part.  llr_in and term_in: both, when they are
+// at hand.
 template <class G, int MAXC>
 __device__ __forceinline__ void ld_llr(const G &g, int n, const float *lr, const XlmDev &xt,
-                                       const XlSmall &xs, float (&llr)[MAXC], float *terms, float *llr_out) {
+                                       const XlSmall &xs, float (&llr)[MAXC], float *terms, float *llr_out,
+                                       const float *llr_in = nullptr, const float *term_in = nullptr,
+                                       float *part = nullptr) {
 #pragma unroll
   for (int c = 0; c < MAXC; c++) {
     const int k = g.col(n, c);
     llr[c] = 0.0f;
     if (k < n) {
-      const float v = lr[k];
       if (terms) {
-        const float pco = v / (1.0f + v);
-        const float tmp = xl_logf(xt, xs, 1.0f - pco);
-        terms[k] = (pco * (-xl_logf(xt, xs, pco) + tmp) - tmp) / LDPCA_LOG2;
+        const float term = term_in ? __ldg(term_in + k) : ld_entropy_term(lr[k], xt, xs);
+        if (part) *part += term;
+        if constexpr (G::C > 1)
+          ld_st_cluster(ld_mapa((uint32_t)__cvta_generic_to_shared(terms + k), 0), __float_as_uint(term));
+        else
+          terms[k] = term;
       }
-      llr[c] = xl_logf(xt, xs, v);
+      llr[c] = llr_in ? __ldg(llr_in + k) : xl_logf(xt, xs, lr[k]);
       if (llr_out) llr_out[k] = llr[c];
     }
   }
@@ -334,6 +363,42 @@ __device__ __forceinline__ int ld_start_code(const LadderDev &L, float h) {
   int start = 0;
   while (start < L.num_codes - 1 && L.code_rate[start] < h) start++;
   return start;
+}
+
+// The start code from a parallel sum of the entropy terms: `part` is the sum of
+// the thread's own terms.  The bound itself is a chain of n dependent float
+// additions (25 K cycles at CIF, as long as a BP iteration of a lone block and
+// several of a cluster's), but all a ladder needs from it is the start code.
+// Adding n non-negative terms one by one in float stays within n * 2^-24 of
+// their sum, so when both ends of that range (doubled for the errors of the
+// parallel sum and the division) select one code, it is the code.  Returns -1
+// when they do not, or when a term is not a number; every thread gets the result.
+template <class G>
+__device__ __forceinline__ int ld_start_near(const G &g, const LadderDev &L, float part, uint32_t *s_red, LdCtl *ctl) {
+  constexpr int NW = G::NT / 32;
+  const int lane = g.t & 31, warp = g.t >> 5;
+  for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+  if (lane == 0) s_red[warp] = __float_as_uint(part);
+  g.sync();
+  if (g.t == 0) {
+    float x = 0.0f;
+    for (int w = 0; w < NW; w++) x += __uint_as_float(s_red[w]);
+    if constexpr (G::C > 1) {
+      for (int b = 0; b < G::C; b++)
+        ld_st_cluster(ld_mapa((uint32_t)__cvta_generic_to_shared(&ctl->crc[g.rank]), b), __float_as_uint(x));
+    } else {
+      ctl->crc[0] = __float_as_uint(x);
+    }
+  }
+  g.sync_all();
+  float h = 0.0f;
+#pragma unroll
+  for (int b = 0; b < G::C; b++) h += __uint_as_float(*(volatile uint32_t *)&ctl->crc[b]);
+  h /= (float)L.n;
+  const float err = h * ((float)L.n * 0x1p-23f);
+  if (!(h >= 0.0f) || h > 1e30f) return -1;
+  const int lo = ld_start_code(L, h - err), hi = ld_start_code(L, h + err);
+  return lo == hi ? lo : -1;
 }
 
 // One ladder code below full rate: its syndrome (from the accumulated syndrome
