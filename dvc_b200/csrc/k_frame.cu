@@ -377,68 +377,180 @@ __global__ void forward_me_post_kernel(FrameDev *frames) {
   F.mb_mv[i] = o;
 }
 
+// SAD of the BL x BL block (every second half-pel sample of a 2BL x 2BL area)
+// at f and p, by LP = 32 or 4 lanes, l the lane's number among them: some rows
+// each, or a share of one row.  All lanes of a candidate get the sum.
+template <int BL, int LP>
+__device__ __forceinline__ int bidirect_sad(const uint8_t *f, const uint8_t *p, int w2, int l) {
+  constexpr int SPLIT = LP > BL ? LP / BL : 1;   // lanes per row
+  constexpr int ROWS = LP > BL ? 1 : BL / LP;    // rows per lane
+  constexpr int PX = BL / SPLIT;                 // samples per lane and row
+  const int r0 = LP > BL ? l / SPLIT : l * ROWS, x0 = (l % SPLIT) * PX * 2;
+  int sad = 0;
+#pragma unroll
+  for (int r = 0; r < ROWS; r++) {
+    const int o = 2 * (r0 + r) * w2 + x0;
+    int a[PX], b[PX];
+#pragma unroll
+    for (int i = 0; i < PX; i++) {
+      a[i] = __ldg(f + o + 2 * i);
+      b[i] = __ldg(p + o + 2 * i);
+    }
+#pragma unroll
+    for (int i = 0; i < PX; i++) sad += abs(a[i] - b[i]);
+  }
+  if constexpr (LP == 32) {
+    return __reduce_add_sync(0xffffffffu, sad);
+  } else {
+    sad += __shfl_xor_sync(0xffffffffu, sad, 1);
+    return sad + __shfl_xor_sync(0xffffffffu, sad, 2);
+  }
+}
+
 // bidirectME, sideInfoCreation.cpp:235-310.  The reference visits blocks in
 // raster order and updates the vectors in place; a block's search window uses
 // its top and left neighbours' updated and its bottom and right neighbours'
-// previous vectors.  Blocks on one anti-diagonal are therefore independent:
-// this single-block-per-frame kernel walks the anti-diagonals, one warp per
-// block, which is equivalent to the raster order.
-template <int NT>
-__global__ void __launch_bounds__(NT) bidirect_me_kernel(FrameDev *frames, int bl) {
+// previous vectors.  Blocks on one anti-diagonal are therefore independent, and
+// this kernel (one thread block per frame) walks the anti-diagonals, which is
+// equivalent to the raster order.
+// What bounds it: the chain of 39 (16x16 blocks) or 79 (8x8) dependent
+// diagonals of a CIF frame.  Most windows hold one candidate, which needs no
+// search, and a few hold hundreds, so the candidates of all blocks of a diagonal are dealt out to all
+// warps: small windows a candidate at a time, its samples over 32 lanes, larger
+// ones eight at a time, four lanes each (neighbouring candidates' samples share
+// sectors).  One warp per block, a lane per candidate took 592 us a launch.
+template <int BL>
+__global__ void __launch_bounds__(1024) bidirect_me_kernel(FrameDev *frames) {
   FrameDev &F = frames[blockIdx.x];
   if (!F.active) return;
-  MVd *mv = bl == 16 ? F.mb_mv : F.blk_mv;
-  const int w = F.w, h = F.h, bh = h / bl, bw = w / bl, w2 = w << 1, bl2 = bl << 1;
-  const int srb = (h << 1) - bl2, srr = w2 - bl2;
+  constexpr int BL2 = 2 * BL, NW = 32, SMALL = 4;
+  constexpr int MAXD = 288 / BL, MAXB = MAXD * (352 / BL);
+  MVd *mv = BL == 16 ? F.mb_mv : F.blk_mv;
+  const int w = F.w, h = F.h, bh = h / BL, bw = w / BL, w2 = w << 1;
+  const int srb = (h << 1) - BL2, srr = w2 - BL2;
   const double scale = F.ipc / F.ifc;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint8_t *fut = F.future_ip, *pas = F.past_ip;
-  for (int d = 0; d < bh + bw - 1; d++) {
-    const int i0 = d - (bw - 1) > 0 ? d - (bw - 1) : 0;
-    const int i1 = d < bh - 1 ? d : bh - 1;
-    for (int i = i0 + warp; i <= i1; i += NT / 32) {
-      const int j = d - i;
-      const int bi = i * bw + j;
-      const int y2 = i * bl2, x2 = j * bl2;
-      const int st = (i - 1 >= 0) ? (int)mv[bi - bw].fy + bl2 : (int)mv[bi].fy;
-      const int sb = (i + 1 < bh) ? (int)mv[bi + bw].fy - bl2 : (int)mv[bi].fy;
-      const int sl = (j - 1 >= 0) ? (int)mv[bi - 1].fx + bl2 : (int)mv[bi].fx;
-      const int sr = (j + 1 < bw) ? (int)mv[bi + 1].fx - bl2 : (int)mv[bi].fx;
-      const int cw = sr - sl + 1, chh = sb - st + 1;
-      const int nc = (cw > 0 && chh > 0) ? cw * chh : 0;
-      double best = 1e300;
-      int bc = 0x7fffffff;
-      for (int c = lane; c < nc; c += 32) {
-        const int fy = st + c / cw, fx = sl + c % cw;
-        const int py = end_point(y2, (double)(y2 - fy), scale, 0, srb);
-        const int px = end_point(x2, (double)(x2 - fx), scale, 0, srr);
-        int mad = 0;
-        for (int m = 0; m < bl2; m += 2) {
-          const uint8_t *pr = pas + (py + m) * w2 + px;
-          const uint8_t *fr = fut + (fy + m) * w2 + fx;
-          for (int n = 0; n < bl2; n += 2) mad += abs((int)fr[n] - (int)pr[n]);
+  __shared__ int16_t px_[MAXB], py_[MAXB];       // future end point of every block
+  __shared__ int4 win[MAXD];                     // window of a diagonal's block: top, left, columns, candidates
+  __shared__ int first[MAXD + 1];                // first work item of each
+  __shared__ double scost[MAXD][NW];             // best cost and candidate by warp
+  __shared__ int sidx[MAXD][NW];
+  __shared__ int s_d;
+  auto past_y = [&](int y2, int fy) { return end_point(y2, (double)(y2 - fy), scale, 0, srb); };
+  auto past_x = [&](int x2, int fx) { return end_point(x2, (double)(x2 - fx), scale, 0, srr); };
+  auto update = [&](int i, int j, int fy, int fx) {
+    const int py = past_y(i * BL2, fy), px = past_x(j * BL2, fx), bi = i * bw + j;
+    MVd b;
+    b.fx = (double)fx;
+    b.fy = (double)fy;
+    b.px = (double)px;
+    b.py = (double)py;
+    b.vx = (double)(px - fx);
+    b.vy = (double)(py - fy);
+    mv[bi] = b;
+    px_[bi] = (int16_t)fx;
+    py_[bi] = (int16_t)fy;
+  };
+  for (int b = threadIdx.x; b < bh * bw; b += 1024) {
+    px_[b] = (int16_t)(int)mv[b].fx;
+    py_[b] = (int16_t)(int)mv[b].fy;
+  }
+  __syncthreads();
+  for (int d = 0;; d++) {
+    if (warp == 0) {
+      // the windows of the next diagonal that has a choice to make: a block
+      // with one candidate takes it whatever its SAD (the cost is below the
+      // limit of 10^7 for any: 256 * 255 * (1 + 0.05 * |(704, 576)|))
+      for (; d < bh + bw - 1; d++) {
+        const int i0 = d - (bw - 1) > 0 ? d - (bw - 1) : 0;
+        const int i1 = d < bh - 1 ? d : bh - 1, nb = i1 - i0 + 1;
+        int base = 0;
+        for (int q0 = 0; q0 < nb; q0 += 32) {
+          const int q = q0 + lane, i = i0 + q, j = d - i, bi = i * bw + j;
+          int items = 0;
+          if (q < nb) {
+            const int st = (i - 1 >= 0) ? py_[bi - bw] + BL2 : py_[bi];
+            const int sb = (i + 1 < bh) ? py_[bi + bw] - BL2 : py_[bi];
+            const int sl = (j - 1 >= 0) ? px_[bi - 1] + BL2 : px_[bi];
+            const int sr = (j + 1 < bw) ? px_[bi + 1] - BL2 : px_[bi];
+            const int cw = sr - sl + 1, chh = sb - st + 1;
+            const int nc = (cw > 0 && chh > 0) ? cw * chh : 0;
+            win[q] = make_int4(st, sl, cw, nc);
+            if (nc == 1)
+              update(i, j, st, sl);
+            else
+              items = nc <= SMALL ? nc : (nc + 7) >> 3;
+          }
+          if (__any_sync(0xffffffffu, items)) {
+            int sum = items;
+            for (int o = 1; o < 32; o <<= 1) {
+              const int v = __shfl_up_sync(0xffffffffu, sum, o);
+              if (lane >= o) sum += v;
+            }
+            if (q < nb) first[q] = base + sum - items;
+            base += __shfl_sync(0xffffffffu, sum, 31);
+          } else if (q < nb) {
+            first[q] = base;
+          }
         }
-        const double cost = cost_func((double)mad, (double)(px - fx), (double)(py - fy));
-        if (cost < 10000000.0) better(best, bc, cost, c);
+        if (lane == 0) first[nb] = base;
+        __syncwarp();
+        if (base) break;
       }
-      for (int o = 16; o > 0; o >>= 1) {
-        const double c2 = __shfl_xor_sync(0xffffffffu, best, o);
-        const int i2 = __shfl_xor_sync(0xffffffffu, bc, o);
-        better(best, bc, c2, i2);
+      if (lane == 0) s_d = d;
+    } else {
+      for (int k = threadIdx.x - 32; k < MAXD * NW; k += 1024 - 32) {
+        scost[k >> 5][k & 31] = 1e300;
+        sidx[k >> 5][k & 31] = 0x7fffffff;
       }
-      if (lane == 0 && bc != 0x7fffffff) {
-        const int fy = st + bc / cw, fx = sl + bc % cw;
-        const int py = end_point(y2, (double)(y2 - fy), scale, 0, srb);
-        const int px = end_point(x2, (double)(x2 - fx), scale, 0, srr);
-        MVd b;
-        b.fx = (double)fx;
-        b.fy = (double)fy;
-        b.px = (double)px;
-        b.py = (double)py;
-        b.vx = (double)(px - fx);
-        b.vy = (double)(py - fy);
-        mv[bi] = b;
+    }
+    __syncthreads();
+    d = s_d;
+    if (d >= bh + bw - 1) break;
+    const int i0 = d - (bw - 1) > 0 ? d - (bw - 1) : 0;
+    const int i1 = d < bh - 1 ? d : bh - 1, nb = i1 - i0 + 1;
+    const int total = first[nb], per = (total + NW - 1) / NW;
+    int it = warp * per;
+    const int end = min(total, it + per);
+    if (it < end) {
+      int q = 0;
+      while (first[q + 1] <= it) q++;
+      while (it < end) {
+        const int4 W = win[q];
+        const int stop = min(end, first[q + 1]), i = i0 + q, y2 = i * BL2, x2 = (d - i) * BL2;
+        const bool small = W.w <= SMALL;
+        double best = 1e300;
+        int bc = 0x7fffffff;
+        for (; it < stop; it++) {
+          const int k = it - first[q];
+          const int c = small ? k : min(8 * k + (lane >> 2), W.w - 1);  // past the last: the last again
+          const int cy = c / W.z, fy = W.x + cy, fx = W.y + c - cy * W.z;
+          const int py = past_y(y2, fy), px = past_x(x2, fx);
+          const uint8_t *fr = fut + fy * w2 + fx, *pr = pas + py * w2 + px;
+          const int mad = small ? bidirect_sad<BL, 32>(fr, pr, w2, lane) : bidirect_sad<BL, 4>(fr, pr, w2, lane & 3);
+          // the weight is at least 1: only a SAD not above the best cost can win
+          if ((double)mad <= best) {
+            const double cost = cost_func((double)mad, (double)(px - fx), (double)(py - fy));
+            if (cost < 10000000.0) better(best, bc, cost, c);
+          }
+        }
+        warp_argmin_nonneg(best, bc);
+        if (lane == 0) {
+          scost[q][warp] = best;
+          sidx[q][warp] = bc;
+        }
+        q++;
+        while (q < nb && first[q + 1] <= it) q++;  // blocks with nothing to search
       }
+    }
+    __syncthreads();
+    for (int q = warp; q < nb; q += NW) {
+      if (first[q + 1] == first[q]) continue;
+      double c = scost[q][lane];
+      int bc = sidx[q][lane];
+      warp_argmin_nonneg(c, bc);
+      if (lane == 0 && bc != 0x7fffffff) update(i0 + q, d - i0 - q, win[q].x + bc / win[q].z, win[q].y + bc % win[q].z);
     }
     __syncthreads();
   }
@@ -1618,9 +1730,9 @@ cudaError_t launch_side_info(FrameDev *fr, int nf, int w, int h, cudaStream_t s)
   else
     forward_me_kernel<256><<<dim3(b16n, nf), 256, 0, s>>>(fr);
   forward_me_post_kernel<<<g2(b16n, 128, nf), 128, 0, s>>>(fr);
-  bidirect_me_kernel<1024><<<nf, 1024, 0, s>>>(fr, 16);
+  bidirect_me_kernel<16><<<nf, 1024, 0, s>>>(fr);
   init_blk_mv_kernel<<<g2(b8n, 128, nf), 128, 0, s>>>(fr);
-  bidirect_me_kernel<1024><<<nf, 1024, 0, s>>>(fr, 8);
+  bidirect_me_kernel<8><<<nf, 1024, 0, s>>>(fr);
   mfc_mse_kernel<<<g2(b8n, 128, nf), 128, 0, s>>>(fr);
   mfc_wvmf_kernel<<<g2(b8n, 128, nf), 128, 0, s>>>(fr);
   mfc_comp_kernel<<<dim3((w + 127) / 128, nf, h), 128, 0, s>>>(fr);
