@@ -339,27 +339,32 @@ __global__ void __launch_bounds__(NT) forward_me_kernel(FrameDev *frames) {
 }
 
 // forwardME, sideInfoCreation.cpp:120-142 (nearest projected hole per
-// macroblock) and the half-pel scaling of createSideInfo (:511-521)
+// macroblock) and the half-pel scaling of createSideInfo (:511-521).  A warp
+// per macroblock: its lanes share the holes, the first of the nearest wins (a
+// thread per macroblock reading all holes took 58 us for a CIF frame, 5 us so).
 __global__ void forward_me_post_kernel(FrameDev *frames) {
   FrameDev &F = frames[blockIdx.y];
   if (!F.active) return;
   const int w = F.w, h = F.h, b16w = w / 16, b16n = b16w * (h / 16);
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (i >= b16n) return;
   const int top = (i / b16w) << 4, left = (i % b16w) << 4;
   const double maxd = w * w + h * h;
   double mind = maxd;
-  int bj = -1;
-  for (int j = 0; j < b16n; j++) {
-    const double hx = F.holes[2 * j], hy = F.holes[2 * j + 1];
-    const double d = (left - hx) * (left - hx) + (top - hy) * (top - hy);
+  int bj = 0x7fffffff;
+#pragma unroll 4
+  for (int j = lane; j < b16n; j += 32) {
+    const double2 hole = reinterpret_cast<const double2 *>(F.holes)[j];
+    const double d = (left - hole.x) * (left - hole.x) + (top - hole.y) * (top - hole.y);
     if (d < mind) {
       mind = d;
       bj = j;
     }
   }
+  warp_argmin_nonneg(mind, bj);
+  if (lane != 0) return;
   MVd b{};
-  if (bj >= 0) b = F.fmv[bj];
+  if (bj != 0x7fffffff) b = F.fmv[bj];
   MVd o;
   o.fx = (double)end_point(left, -b.vx, F.ifc, 0, w - 16);
   o.fy = (double)end_point(top, -b.vy, F.ifc, 0, h - 16);
@@ -418,7 +423,8 @@ __device__ __forceinline__ int bidirect_sad(const uint8_t *f, const uint8_t *p, 
 // search, and a few hold hundreds, so the candidates of all blocks of a diagonal are dealt out to all
 // warps: small windows a candidate at a time, its samples over 32 lanes, larger
 // ones eight at a time, four lanes each (neighbouring candidates' samples share
-// sectors).  One warp per block, a lane per candidate took 592 us a launch.
+// sectors).  One warp per block, a lane per candidate took 592 us a launch for
+// either size on a lone CIF frame; now 167 (16x16) and 239 us (cold caches).
 template <int BL>
 __global__ void __launch_bounds__(1024) bidirect_me_kernel(FrameDev *frames) {
   FrameDev &F = frames[blockIdx.x];
@@ -597,53 +603,51 @@ __global__ void mfc_mse_kernel(FrameDev *frames) {
 }
 
 // motionFilterAndComp, sideInfoCreation.cpp:344-405: weighted vector median
-// over the 3x3 neighbourhood, then the new end points
+// over the 3x3 neighbourhood, then the new end points.  A lane per candidate
+// neighbour (16 lanes a block, up to nine of them at work) sums its weighted
+// distances in neighbour order; the choice is then the sequential scan's.
+// (One thread per block did 72 divisions and roots in a row, 31 us; 9 us so.)
 __global__ void mfc_wvmf_kernel(FrameDev *frames) {
   FrameDev &F = frames[blockIdx.y];
   if (!F.active) return;
   const int w = F.w, h = F.h, b8w = w / 8, b8h = h / 8, b8n = b8w * b8h;
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= b8n) return;
+  const int k = min((int)(blockIdx.x * blockDim.x + threadIdx.x) >> 4, b8n - 1), c = threadIdx.x & 15;
   const int i = k / b8w, j = k % b8w;
   const int srb = (h << 1) - 16, srr = (w << 1) - 16;
   const int y2 = i << 4, x2 = j << 4;
-  int nbr[9], cnt = 0;
-  for (int m = i - 1; m <= i + 1; m++) {
-    if (m < 0 || m >= b8h) continue;
-    for (int n = j - 1; n <= j + 1; n++) {
-      if (n < 0 || n >= b8w) continue;
-      nbr[cnt++] = m * b8w + n;
-    }
-  }
+  // neighbours in raster order, those outside the frame left out
+  const int r0 = max(i - 1, 0), r1 = min(i + 1, b8h - 1), c0 = max(j - 1, 0), c1 = min(j + 1, b8w - 1);
+  const int nw = c1 - c0 + 1, cnt = nw * (r1 - r0 + 1);
   const MVd *mv = F.blk_mv;
   const double *mse = F.mse;
-  double minw = 0.0;
-  int bestb = nbr[0];
-  for (int q = 1; q < cnt; q++) {
-    const int o = nbr[q];
-    const double dx = mv[bestb].vx - mv[o].vx, dy = mv[bestb].vy - mv[o].vy;
-    minw += mse[bestb] / mse[o] * sqrt(dx * dx + dy * dy);
+  const int cb = (r0 + min(c, cnt - 1) / nw) * b8w + c0 + min(c, cnt - 1) % nw;
+  const double vx = mv[cb].vx, vy = mv[cb].vy, m = mse[cb];
+  double wv = 0.0;
+  // (both blocks of a warp take all nine turns: the shuffles need every lane)
+  for (int q = 0; q < 9; q++) {
+    // neighbour q's vector and error from its lane
+    const double ox = __shfl_sync(0xffffffffu, vx, q, 16), oy = __shfl_sync(0xffffffffu, vy, q, 16);
+    const double om = __shfl_sync(0xffffffffu, m, q, 16);
+    if (c == q || q >= cnt) continue;
+    const double dx = vx - ox, dy = vy - oy;
+    wv += m / om * sqrt(dx * dx + dy * dy);
   }
-  for (int c = 1; c < cnt; c++) {
-    const int cb = nbr[c];
-    double wv = 0.0;
-    for (int q = 0; q < cnt; q++) {
-      if (c == q) continue;
-      const int o = nbr[q];
-      const double dx = mv[cb].vx - mv[o].vx, dy = mv[cb].vy - mv[o].vy;
-      wv += mse[cb] / mse[o] * sqrt(dx * dx + dy * dy);
-    }
-    if (wv < minw) {
-      minw = wv;
-      bestb = cb;
+  double minw = __shfl_sync(0xffffffffu, wv, 0, 16);
+  int bc = 0;
+  for (int q = 1; q < 9; q++) {
+    const double v = __shfl_sync(0xffffffffu, wv, q, 16);
+    if (q < cnt && v < minw) {
+      minw = v;
+      bc = q;
     }
   }
-  const double vx = mv[bestb].vx, vy = mv[bestb].vy;
+  const double bx = __shfl_sync(0xffffffffu, vx, bc, 16), by = __shfl_sync(0xffffffffu, vy, bc, 16);
+  if (c != 0) return;
   MVd o;
-  o.fx = (double)end_point(x2, -vx, F.ifc, 0, srr);
-  o.fy = (double)end_point(y2, -vy, F.ifc, 0, srb);
-  o.px = (double)end_point(x2, vx, F.ipc, 0, srr);
-  o.py = (double)end_point(y2, vy, F.ipc, 0, srb);
+  o.fx = (double)end_point(x2, -bx, F.ifc, 0, srr);
+  o.fy = (double)end_point(y2, -by, F.ifc, 0, srb);
+  o.px = (double)end_point(x2, bx, F.ipc, 0, srr);
+  o.py = (double)end_point(y2, by, F.ipc, 0, srb);
   o.vx = o.px - o.fx;
   o.vy = o.py - o.fy;
   F.blk_mv2[k] = o;
@@ -699,38 +703,60 @@ __global__ void residue_transform_kernel(FrameDev *frames) {
 
 // noiseParameter, noiseModel.cpp:14-45: band mean and variance of |T| over
 // every 4x4 block.  The variance accumulates squares past 2^24, so each band's
-// sums run sequentially in raster block order, one thread per band.
-// The sums stay sequential in block raster order (one thread per band); the
-// block stages 8 block rows of coefficients at a time in shared memory with
-// coalesced loads, so those threads read shared memory instead of waiting on
-// scattered global loads.
-__global__ void __launch_bounds__(256) noise_band_stats_kernel(FrameDev *frames) {
+// sums run sequentially in raster block order, one lane of warp 0 per band.
+// What bounds it: that chain, two dependent additions per block side by side
+// (6336 blocks at CIF).  The other warps bring the next 4 block rows of
+// coefficients into the second half of a double buffer meanwhile, and the
+// lanes read eight blocks ahead of their additions: 254 -> 49 us a CIF frame.
+// A row is padded by four words so that the 16 lanes (4 x 4 positions of a
+// block) read 16 banks.
+__global__ void __launch_bounds__(512) noise_band_stats_kernel(FrameDev *frames) {
   FrameDev &F = frames[blockIdx.x];
   if (!F.active) return;
-  constexpr int RB = 8;  // block rows per chunk
-  __shared__ int chunk[RB * 4][352];
+  constexpr int RB = 4, ST = 352 + 4;  // block rows per chunk, words per row
+  __shared__ int chunk[2][RB * 4][ST];
   const int band = threadIdx.x;
   const int index = c_zigzag[band & 15];
   // bands are coded while Qbits > 0 in zig-zag order; later ones are unused
   bool active = band < 16;
   for (int b = 0; active && b <= band; b++) active = F.qbits[c_zigzag[b]] > 0;
-  const int w = F.w, b4w = w / 4, b4h = F.h / 4, b4n = b4w * b4h;
-  float mean = 0.0f, var = 0.0f;
-  for (int i0 = 0; i0 < b4h; i0 += RB) {
-    const int rows = (b4h - i0 < RB ? b4h - i0 : RB) * 4;
-    __syncthreads();
-    for (int k = threadIdx.x; k < rows * w; k += blockDim.x) {
-      const int r = k / w, x = k - r * w;
-      chunk[r][x] = F.side_trans[(4 * i0 + r) * w + x];
+  const int w = F.w, b4w = w / 4, b4h = F.h / 4, b4n = b4w * b4h;  // b4w is a multiple of 4
+  auto load = [&](int i0, int t, int nt) {
+    const int rows = min(RB, b4h - i0) * 4, w4 = w >> 2;
+    int4(*dst)[ST / 4] = reinterpret_cast<int4(*)[ST / 4]>(chunk[(i0 / RB) & 1]);
+    const int4 *src = reinterpret_cast<const int4 *>(F.side_trans + (size_t)4 * i0 * w);
+    for (int k = t; k < rows * w4; k += nt) {
+      const int r = k / w4;
+      dst[r][k - r * w4] = src[k];
     }
+  };
+  float mean = 0.0f, var = 0.0f;
+  load(0, threadIdx.x, blockDim.x);
+  for (int i0 = 0; i0 < b4h; i0 += RB) {
     __syncthreads();
-    if (active)
-      for (int i = 0; i < rows / 4; i++)
-        for (int j = 0; j < b4w; j++) {
-          const float c = fabsf((float)chunk[4 * i + (index >> 2)][4 * j + (index & 3)]);
+    if (threadIdx.x >= 32) {
+      if (i0 + RB < b4h) load(i0 + RB, threadIdx.x - 32, blockDim.x - 32);
+    } else if (active) {
+      for (int i = 0; i < RB && i0 + i < b4h; i++) {
+        const int *row = chunk[(i0 / RB) & 1][4 * i + (index >> 2)] + (index & 3);
+        int j = 0;
+        for (; j + 8 <= b4w; j += 8) {
+          float c[8];
+#pragma unroll
+          for (int q = 0; q < 8; q++) c[q] = fabsf((float)row[4 * (j + q)]);
+#pragma unroll
+          for (int q = 0; q < 8; q++) {
+            mean += c[q];
+            var += c[q] * c[q];
+          }
+        }
+        for (; j < b4w; j++) {
+          const float c = fabsf((float)row[4 * j]);
           mean += c;
           var += c * c;
         }
+      }
+    }
   }
   if (!active) return;
   mean /= (float)b4n;
@@ -979,39 +1005,37 @@ __global__ void __launch_bounds__(NT) noise_dist_kernel(FrameDev *frames, XlmDev
 }
 
 // p[lo0..hi0) and p[lo1..hi1), each summed in ascending order (the float sums
-// of condBitProb).  The rows are read 16 bytes at a time once aligned, and
-// the two chains advance together, so two additions are in flight.
+// of condBitProb).  Each lane walks its own row, so the reads wait on memory:
+// once aligned they are 16 bytes each, and up to four of either chain are in
+// flight before their additions (one of either: 20 us for a lone CIF frame).
 __device__ __forceinline__ void interval_sums(const float *p, int lo0, int hi0, int lo1, int hi1, float &s0,
                                               float &s1) {
   float a = 0.0f, b = 0.0f;
   int q0 = lo0, q1 = lo1;
   for (; q0 < hi0 && (reinterpret_cast<uintptr_t>(p + q0) & 15); q0++) a += __ldg(p + q0);
   for (; q1 < hi1 && (reinterpret_cast<uintptr_t>(p + q1) & 15); q1++) b += __ldg(p + q1);
-  for (; q0 + 4 <= hi0 && q1 + 4 <= hi1; q0 += 4, q1 += 4) {
-    const float4 u = __ldg(reinterpret_cast<const float4 *>(p + q0));
-    const float4 v = __ldg(reinterpret_cast<const float4 *>(p + q1));
-    a += u.x;
-    b += v.x;
-    a += u.y;
-    b += v.y;
-    a += u.z;
-    b += v.z;
-    a += u.w;
-    b += v.w;
-  }
-  for (; q0 + 4 <= hi0; q0 += 4) {
-    const float4 u = __ldg(reinterpret_cast<const float4 *>(p + q0));
-    a += u.x;
-    a += u.y;
-    a += u.z;
-    a += u.w;
-  }
-  for (; q1 + 4 <= hi1; q1 += 4) {
-    const float4 v = __ldg(reinterpret_cast<const float4 *>(p + q1));
-    b += v.x;
-    b += v.y;
-    b += v.z;
-    b += v.w;
+  auto add4 = [](float &s, const float4 &v) {
+    s += v.x;
+    s += v.y;
+    s += v.z;
+    s += v.w;
+  };
+  constexpr int U = 4;
+  while (q0 + 4 <= hi0 || q1 + 4 <= hi1) {
+    float4 u[U], v[U];
+#pragma unroll
+    for (int i = 0; i < U; i++) {
+      // a chain past its last whole quad adds +0 to a sum that is not negative
+      u[i] = q0 + 4 * i + 4 <= hi0 ? __ldg(reinterpret_cast<const float4 *>(p + q0) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[i] = q1 + 4 * i + 4 <= hi1 ? __ldg(reinterpret_cast<const float4 *>(p + q1) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int i = 0; i < U; i++) {
+      add4(a, u[i]);
+      add4(b, v[i]);
+    }
+    q0 = max(q0, min(q0 + 4 * U, q0 + ((hi0 - q0) & ~3)));
+    q1 = max(q1, min(q1 + 4 * U, q1 + ((hi1 - q1) & ~3)));
   }
   for (; q0 < hi0; q0++) a += __ldg(p + q0);
   for (; q1 < hi1; q1++) b += __ldg(p + q1);
@@ -1729,12 +1753,12 @@ cudaError_t launch_side_info(FrameDev *fr, int nf, int w, int h, cudaStream_t s)
     forward_me_kernel<512><<<dim3(b16n, nf), 512, 0, s>>>(fr);
   else
     forward_me_kernel<256><<<dim3(b16n, nf), 256, 0, s>>>(fr);
-  forward_me_post_kernel<<<g2(b16n, 128, nf), 128, 0, s>>>(fr);
+  forward_me_post_kernel<<<g2(b16n * 32, 128, nf), 128, 0, s>>>(fr);
   bidirect_me_kernel<16><<<nf, 1024, 0, s>>>(fr);
   init_blk_mv_kernel<<<g2(b8n, 128, nf), 128, 0, s>>>(fr);
   bidirect_me_kernel<8><<<nf, 1024, 0, s>>>(fr);
   mfc_mse_kernel<<<g2(b8n, 128, nf), 128, 0, s>>>(fr);
-  mfc_wvmf_kernel<<<g2(b8n, 128, nf), 128, 0, s>>>(fr);
+  mfc_wvmf_kernel<<<g2(b8n * 16, 128, nf), 128, 0, s>>>(fr);
   mfc_comp_kernel<<<dim3((w + 127) / 128, nf, h), 128, 0, s>>>(fr);
   return cudaGetLastError();
 }
@@ -1742,7 +1766,7 @@ cudaError_t launch_side_info(FrameDev *fr, int nf, int w, int h, cudaStream_t s)
 cudaError_t launch_frame_prep(FrameDev *fr, int nf, int w, int h, cudaStream_t s) {
   const int b4n = (w / 4) * (h / 4);
   residue_transform_kernel<<<g2(b4n, 128, nf), 128, 0, s>>>(fr);
-  noise_band_stats_kernel<<<nf, 256, 0, s>>>(fr);
+  noise_band_stats_kernel<<<nf, 512, 0, s>>>(fr);
   noise_alpha_kernel<<<g2(b4n, 128, nf), 128, 0, s>>>(fr);
   over_complete_kernel<<<dim3((w - 3 + 127) / 128, nf, h - 3), 128, 0, s>>>(fr, -1);
   init_ml_kernel<<<g2(b4n, 128, nf), 128, 0, s>>>(fr);
