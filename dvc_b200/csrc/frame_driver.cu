@@ -119,6 +119,12 @@ bool FrameBatcher::ensure_pinned(size_t b) {
 void FrameBatcher::release() {
   for (cudaEvent_t e : ev_) cudaEventDestroy(e);
   ev_.clear();
+  for (cudaStream_t st : side_) cudaStreamDestroy(st);
+  side_.clear();
+  for (cudaEvent_t e : side_done_) cudaEventDestroy(e);
+  side_done_.clear();
+  if (fork_) cudaEventDestroy(fork_);
+  fork_ = nullptr;
   for (auto &s : slots_) s.release();
   slots_.clear();
   frames_dev_.release();
@@ -133,7 +139,8 @@ void FrameBatcher::release() {
 
 static size_t align16(size_t v) { return (v + 15) & ~(size_t)15; }
 
-bool FrameBatcher::prepare(Context &ctx, const std::vector<FrameSpec> &frames, cudaStream_t s, int concurrent) {
+bool FrameBatcher::prepare(Context &ctx, const std::vector<FrameSpec> &frames, cudaStream_t s, int concurrent,
+                           int max_groups) {
   const int nf = (int)frames.size();
   nf_ = 0;
   if (nf == 0) return true;
@@ -158,7 +165,6 @@ bool FrameBatcher::prepare(Context &ctx, const std::vector<FrameSpec> &frames, c
   // ---- host-side per-frame constants, WZ block lists and upload packing
   std::vector<FrameDev> fd(nf);
   std::vector<std::vector<int>> plane_base(nf);
-  int max_nsir = 0;
   struct Packed {
     size_t mode, sir, sob, crc, acc, pmode, total;
   };
@@ -180,25 +186,47 @@ bool FrameBatcher::prepare(Context &ctx, const std::vector<FrameSpec> &frames, c
   }
   const size_t fd_off = pinned_need;
   pinned_need += align16(sizeof(FrameDev) * nf);
-  // LDPCA steps: (band, bit) while any frame codes the band
-  std::vector<Step> steps;
-  for (int band = 0; band < 16; band++) {
-    int maxbits = 0;
-    for (int f = 0; f < nf; f++) {
-      bool coded = true;
-      for (int b = 0; b <= band; b++) coded = coded && kQBits[frames[f].qindex][kZigzag[b]] > 0;
-      if (coded) maxbits = std::max(maxbits, kQBits[frames[f].qindex][kZigzag[band]]);
+  // Groups, and the LDPCA steps of each: (band, bit) while any of its frames
+  // codes the band.  A lockstep step waits for its slowest codeword, so while
+  // few frames decode at once the frames of a batch go in up to eight groups
+  // on streams of their own.  One group of up to 16 frames against eight:
+  // sessions of 16 + 32 CIF frames in two levels 141 -> 104 ms, 32 and 64 CIF
+  // frames 84 -> 65 and 82 -> 64 ms, 6 + 12 + 24 QCIF frames in three levels
+  // 102 -> 89 ms, eleven CIF frames at QIndex 8 70 -> 56 ms.  Past 64 frames the
+  // device is full: 128 CIF frames 108 -> 102 ms from a graph, but 111 -> 115 ms
+  // launched one by one, 96 QCIF frames 106 -> 106 ms.  A server's cohorts, which
+  // are launched one by one and overlap each other, lose to the launches and to
+  // streams sharing hardware queues (54 mixed requests 56 -> 77 ms), so they
+  // ask for one group.
+  const int together = std::max(nf, concurrent);
+  const int per = together > 64 ? nf : (nf + max_groups - 1) / max_groups;
+  std::vector<Group> groups;
+  size_t njobs = 0;
+  for (int f0 = 0; f0 < nf; f0 += per) {
+    Group G;
+    G.f0 = f0;
+    G.nf = std::min(per, nf - f0);
+    for (int band = 0; band < 16; band++) {
+      int maxbits = 0;
+      for (int f = f0; f < f0 + G.nf; f++) {
+        bool coded = true;
+        for (int b = 0; b <= band; b++) coded = coded && kQBits[frames[f].qindex][kZigzag[b]] > 0;
+        if (coded) maxbits = std::max(maxbits, kQBits[frames[f].qindex][kZigzag[band]]);
+      }
+      if (maxbits == 0) break;
+      for (int bit = maxbits; bit >= 1; bit--) {
+        Step st;
+        st.band = band;
+        st.bit = bit;
+        G.steps.push_back(st);
+      }
     }
-    if (maxbits == 0) break;
-    for (int bit = maxbits; bit >= 1; bit--) {
-      Step st;
-      st.band = band;
-      st.bit = bit;
-      steps.push_back(st);
-    }
+    G.job0 = njobs;
+    njobs += G.steps.size() * G.nf;
+    groups.push_back(std::move(G));
   }
   const size_t jobs_off = pinned_need;
-  pinned_need += align16(sizeof(LdpcaJob) * steps.size() * nf);
+  pinned_need += align16(sizeof(LdpcaJob) * njobs);
   const size_t res_off = pinned_need;
   size_t res_bytes = 0;
   for (int f = 0; f < nf; f++) res_bytes += (size_t)qb[f] * 20;
@@ -272,7 +300,6 @@ bool FrameBatcher::prepare(Context &ctx, const std::vector<FrameSpec> &frames, c
       }
     }
     D.nsir = nsir;
-    max_nsir = std::max(max_nsir, nsir);
     memcpy(P + p.crc, F.crc, qb[f]);
     if (F.past_mode)
       memcpy(P + p.pmode, F.past_mode, b8n);
@@ -340,66 +367,91 @@ bool FrameBatcher::prepare(Context &ctx, const std::vector<FrameSpec> &frames, c
     return false;
   FrameDev *fdev = frames_dev_.as<FrameDev>();
 
-  // LDPCA jobs for every step
+  // LDPCA jobs for every step of every group
   LdpcaJob *jobs = (LdpcaJob *)(pin + jobs_off);
-  plane_of_.assign(steps.size() * nf, -1);
-  for (size_t si = 0; si < steps.size(); si++) {
-    const int band = steps[si].band, bit = steps[si].bit, index = kZigzag[band];
-    for (int f = 0; f < nf; f++) {
-      LdpcaJob &J = jobs[si * nf + f];
-      memset(&J, 0, sizeof J);
-      const int q = frames[f].qindex;
-      bool coded = true;
-      for (int b = 0; b <= band; b++) coded = coded && kQBits[q][kZigzag[b]] > 0;
-      if (!coded || bit > kQBits[q][index]) continue;
-      const int plane = plane_base[f][band] + (kQBits[q][index] - bit);
-      plane_of_[si * nf + f] = plane;
-      Slot &S = slots_[f];
-      J.active = 1;
-      J.lr = fd[f].lr;
-      J.llr_in = fd[f].llr;
-      J.term_in = fd[f].term;
-      J.acc = S.in.as<uint8_t>() + pk[f].acc + (size_t)plane * nb;
-      J.crc = frames[f].crc[plane];
-      J.result = S.out.as<int>() + plane * 4;
-      J.entropy = (float *)(S.out.as<uint8_t>() + (size_t)qb[f] * 16) + plane;
-      J.recons_trans = fd[f].recons_trans;
-      J.mode = fd[f].mode;
-      J.w = w;
-      J.index_in_blk = index;
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device);
+  size_t spec_bytes = 0;
+  for (Group &G : groups) {
+    G.plane_of.assign(G.steps.size() * G.nf, -1);
+    for (int f = G.f0; f < G.f0 + G.nf; f++) {
+      G.max_nsir = std::max(G.max_nsir, fd[f].nsir);
+      G.deblock = G.deblock || fd[f].deblock;
+    }
+    for (size_t si = 0; si < G.steps.size(); si++) {
+      const int band = G.steps[si].band, bit = G.steps[si].bit, index = kZigzag[band];
+      for (int k = 0; k < G.nf; k++) {
+        const int f = G.f0 + k;
+        LdpcaJob &J = jobs[G.job0 + si * G.nf + k];
+        memset(&J, 0, sizeof J);
+        const int q = frames[f].qindex;
+        bool coded = true;
+        for (int b = 0; b <= band; b++) coded = coded && kQBits[q][kZigzag[b]] > 0;
+        if (!coded || bit > kQBits[q][index]) continue;
+        const int plane = plane_base[f][band] + (kQBits[q][index] - bit);
+        G.plane_of[si * G.nf + k] = plane;
+        Slot &S = slots_[f];
+        J.active = 1;
+        J.lr = fd[f].lr;
+        J.llr_in = fd[f].llr;
+        J.term_in = fd[f].term;
+        J.acc = S.in.as<uint8_t>() + pk[f].acc + (size_t)plane * nb;
+        J.crc = frames[f].crc[plane];
+        J.result = S.out.as<int>() + plane * 4;
+        J.entropy = (float *)(S.out.as<uint8_t>() + (size_t)qb[f] * 16) + plane;
+        J.recons_trans = fd[f].recons_trans;
+        J.mode = fd[f].mode;
+        J.w = w;
+        J.index_in_blk = index;
+      }
     }
   }
-  if (!jobs_dev_.ensure(sizeof(LdpcaJob) * std::max<size_t>(1, steps.size() * nf), alloc_stream_))
-    return ctx.fail("device allocation failed");
-  if (!steps.empty() &&
-      !ctx.cuda_ok(cudaMemcpyAsync(jobs_dev_.p, jobs, sizeof(LdpcaJob) * steps.size() * nf, cudaMemcpyHostToDevice, s),
-                   "H2D jobs"))
-    return false;
-
-  // speculative slots and blocks per slot of every step
-  {
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device);
-    spec_k_ = 1;
-    for (size_t si = 0; si < steps.size(); si++) {
+  // speculative slots and blocks per slot of every step, from the codewords
+  // then active in the batch (a group is taken to be at the step its frames
+  // would be at in lockstep) and in the batches beside it
+  for (Group &G : groups) {
+    G.spec_k = 1;
+    for (Step &st : G.steps) {
       int active = 0;
-      for (int f = 0; f < nf; f++) active += plane_of_[si * nf + f] >= 0;
-      ldpca_spec_shape(n, (int)((long long)active * std::max(nf, concurrent) / nf), sms, steps[si].spec_k, steps[si].spec_c);
-      spec_k_ = std::max(spec_k_, steps[si].spec_k);
+      for (int f = 0; f < nf; f++) {
+        const int q = frames[f].qindex;
+        bool coded = true;
+        for (int b = 0; b <= st.band; b++) coded = coded && kQBits[q][kZigzag[b]] > 0;
+        active += coded && st.bit <= kQBits[q][kZigzag[st.band]];
+      }
+      ldpca_spec_shape(n, (int)((long long)active * together / nf), sms, st.spec_k, st.spec_c);
+      G.spec_k = std::max(G.spec_k, st.spec_k);
     }
-    if (!spec_.ensure(ldpca_spec_scratch_bytes(n, nf, spec_k_), alloc_stream_))
-      return ctx.fail("device allocation failed");
-    if (!ctx.cuda_ok(ldpca_spec_reset(ldpca_spec_carve(spec_.p, nf, spec_k_), nf, spec_k_, s), "LDPCA scratch"))
-      return false;
+    G.spec_off = spec_bytes;
+    spec_bytes += (ldpca_spec_scratch_bytes(n, G.nf, G.spec_k) + 255) & ~(size_t)255;
   }
-  steps_ = steps;
+  if (!jobs_dev_.ensure(sizeof(LdpcaJob) * std::max<size_t>(1, njobs), alloc_stream_) ||
+      !spec_.ensure(std::max<size_t>(1, spec_bytes), alloc_stream_))
+    return ctx.fail("device allocation failed");
+  if (njobs && !ctx.cuda_ok(cudaMemcpyAsync(jobs_dev_.p, jobs, sizeof(LdpcaJob) * njobs, cudaMemcpyHostToDevice, s),
+                            "H2D jobs"))
+    return false;
+  for (const Group &G : groups)
+    if (!ctx.cuda_ok(ldpca_spec_reset(ldpca_spec_carve(spec_.as<uint8_t>() + G.spec_off, G.nf, G.spec_k), G.nf, G.spec_k, s),
+                     "LDPCA scratch"))
+      return false;
+  while (side_.size() + 1 < groups.size()) {
+    cudaStream_t st;
+    if (!ctx.cuda_ok(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "stream")) return false;
+    side_.push_back(st);
+    cudaEvent_t e;
+    if (!ctx.cuda_ok(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event")) return false;
+    side_done_.push_back(e);
+  }
+  if (groups.size() > 1 && !fork_ && !ctx.cuda_ok(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming), "event"))
+    return false;
+  groups_ = std::move(groups);
   fd_ = fd;
   qb_ = qb;
   spec_copy_ = frames;
   nf_ = nf;
   w_ = w;
   h_ = h;
-  max_nsir_ = max_nsir;
   res_off_ = res_off;
   L_ = L;
   return true;
@@ -407,40 +459,32 @@ bool FrameBatcher::prepare(Context &ctx, const std::vector<FrameSpec> &frames, c
 
 long long FrameBatcher::launches_per_execute() const {
   if (nf_ == 0) return 0;
-  long long bands = 0;
-  for (size_t i = 0; i < steps_.size(); i++)
-    if (i == 0 || steps_[i].band != steps_[i - 1].band) bands++;
-  bool deblock = false;
-  for (const FrameDev &f : fd_) deblock = deblock || f.deblock;
-  // side info 8, prep 6, per band 1 + 5, per step condBitProb + ladder, final 1, deblocking 5
-  return 8 + 6 + bands * 6 + (long long)steps_.size() * 2 + 1 + (deblock ? 5 : 0);
+  long long total = 0;
+  for (const Group &G : groups_) {
+    long long bands = 0;
+    for (size_t i = 0; i < G.steps.size(); i++)
+      if (i == 0 || G.steps[i].band != G.steps[i - 1].band) bands++;
+    // side info 8, prep 6, per band 1 + 5, per step condBitProb + ladder, final 1, deblocking 5
+    total += 8 + 6 + bands * 6 + (long long)G.steps.size() * 2 + 1 + (G.deblock ? 5 : 0);
+  }
+  return total;
 }
 
-bool FrameBatcher::execute(Context &ctx, cudaStream_t s, int max_iter, ProfileStats *prof) {
-  if (nf_ == 0) return true;
-  const int nf = nf_, w = w_, h = h_, max_nsir = max_nsir_;
+// a group's frames up to the first band
+bool FrameBatcher::launch_start(Context &ctx, const Group &G, cudaStream_t s) {
+  const int w = w_, h = h_;
   const std::vector<FrameDev> &fd = fd_;
   const std::vector<FrameSpec> &frames = spec_copy_;
-  const std::vector<Step> &steps = steps_;
-  const LadderDev *L = L_;
-  FrameDev *fdev = frames_dev_.as<FrameDev>();
-  for (int f = 0; f < nf; f++) {
+  FrameDev *fdev = frames_dev_.as<FrameDev>() + G.f0;
+  for (int f = G.f0; f < G.f0 + G.nf; f++) {
     if (!ctx.cuda_ok(cudaMemsetAsync(fd[f].recons_trans, 0, (size_t)w * h * 4, s), "memset")) return false;
     if (!ctx.cuda_ok(cudaMemsetAsync(fd[f].si_mv, 0xff, (size_t)w * h / 16 * 8, s), "memset")) return false;
     if (!ctx.cuda_ok(cudaMemsetAsync(fd[f].dbf, 0, (size_t)w * h, s), "memset")) return false;
     if (!ctx.cuda_ok(cudaMemsetAsync(fd[f].alpha, 0, (size_t)w * h * 4, s), "memset")) return false;
   }
-  ev_used_ = 0;
-  if (prof)
-    while (ev_.size() < 2 * steps.size()) {
-      cudaEvent_t e;
-      if (!ctx.cuda_ok(cudaEventCreate(&e), "event")) return false;
-      ev_.push_back(e);
-    }
-  // ---- the decode
-  if (!ctx.cuda_ok(launch_side_info(fdev, nf, w, h, s), "side information")) return false;
-  if (!ctx.cuda_ok(launch_frame_prep(fdev, nf, w, h, s), "frame preparation")) return false;
-  for (int f = 0; f < nf; f++) {
+  if (!ctx.cuda_ok(launch_side_info(fdev, G.nf, w, h, s), "side information")) return false;
+  if (!ctx.cuda_ok(launch_frame_prep(fdev, G.nf, w, h, s), "frame preparation")) return false;
+  for (int f = G.f0; f < G.f0 + G.nf; f++) {
     if (frames[f].dbg_si_initial &&
         !ctx.cuda_ok(cudaMemcpyAsync(frames[f].dbg_si_initial, fd[f].si, (size_t)w * h, cudaMemcpyDeviceToDevice, s),
                      "debug copy"))
@@ -450,50 +494,104 @@ bool FrameBatcher::execute(Context &ctx, cudaStream_t s, int max_iter, ProfileSt
                      "debug copy"))
       return false;
   }
-  size_t si = 0;
-  while (si < steps.size()) {
-    const int band = steps[si].band;
-    int max_range = 0;
-    for (int f = 0; f < nf; f++) max_range = std::max(max_range, fd[f].crange[kZigzag[band]]);
-    if (!ctx.cuda_ok(launch_noise_dist(fdev, nf, max_nsir, ctx.xlm, band, max_range, s), "noise distribution"))
+  return true;
+}
+
+// the next band of a group
+bool FrameBatcher::launch_band(Context &ctx, Group &G, cudaStream_t s, int max_iter, ProfileStats *prof) {
+  const int w = w_, h = h_;
+  const std::vector<FrameDev> &fd = fd_;
+  const std::vector<FrameSpec> &frames = spec_copy_;
+  FrameDev *fdev = frames_dev_.as<FrameDev>() + G.f0;
+  const LdpcaSpec sp = ldpca_spec_carve(spec_.as<uint8_t>() + G.spec_off, G.nf, G.spec_k);
+  size_t &si = G.next;
+  const int band = G.steps[si].band;
+  int max_range = 0;
+  for (int f = G.f0; f < G.f0 + G.nf; f++) max_range = std::max(max_range, fd[f].crange[kZigzag[band]]);
+  if (!ctx.cuda_ok(launch_noise_dist(fdev, G.nf, G.max_nsir, ctx.xlm, band, max_range, s), "noise distribution"))
+    return false;
+  for (; si < G.steps.size() && G.steps[si].band == band; si++) {
+    const Step &st = G.steps[si];
+    if (!ctx.cuda_ok(launch_cond_bit(fdev, G.nf, w, h, ctx.xlm, band, st.bit, s), "conditional bit probability"))
       return false;
-    for (; si < steps.size() && steps[si].band == band; si++) {
-      if (!ctx.cuda_ok(launch_cond_bit(fdev, nf, w, h, ctx.xlm, band, steps[si].bit, s), "conditional bit probability"))
+    for (int k = 0; k < G.nf; k++) {
+      const int f = G.f0 + k, plane = G.plane_of[si * G.nf + k];
+      if (!frames[f].dbg_lr || plane < 0) continue;
+      const size_t n = (size_t)w * h / 16;
+      if (!ctx.cuda_ok(cudaMemcpyAsync(frames[f].dbg_lr + (size_t)plane * n, fd[f].lr, n * 4, cudaMemcpyDeviceToDevice, s),
+                       "debug copy"))
         return false;
-      for (int f = 0; f < nf; f++)
-        if (frames[f].dbg_lr && plane_of_[si * nf + f] >= 0) {
-          const size_t n = (size_t)w * h / 16;
-          if (!ctx.cuda_ok(cudaMemcpyAsync(frames[f].dbg_lr + (size_t)plane_of_[si * nf + f] * n, fd[f].lr, n * 4,
-                                           cudaMemcpyDeviceToDevice, s),
-                           "debug copy"))
-            return false;
-        }
-      if (prof) cudaEventRecord(ev_[ev_used_], s);
-      if (!ctx.cuda_ok(launch_ldpca_spec(*L, jobs_dev_.as<LdpcaJob>() + si * nf, nf, ctx.xlm, max_iter, steps[si].spec_k, steps[si].spec_c,
-                                         ldpca_spec_carve(spec_.p, nf, spec_k_), s),
-                       "LDPCA"))
-        return false;
-      if (prof) {
-        cudaEventRecord(ev_[ev_used_ + 1], s);
-        ev_used_ += 2;
-        prof->ldpca_launches++;
-        prof->ldpca_codewords += nf;
-      }
     }
-    if (!ctx.cuda_ok(launch_band_end(fdev, nf, w, h, max_nsir, band, ctx.xlm, s), "band reconstruction")) return false;
+    if (prof) cudaEventRecord(ev_[ev_used_], s);
+    if (!ctx.cuda_ok(launch_ldpca_spec(*L_, jobs_dev_.as<LdpcaJob>() + G.job0 + si * G.nf, G.nf, ctx.xlm, max_iter,
+                                       st.spec_k, st.spec_c, sp, s),
+                     "LDPCA"))
+      return false;
+    if (prof) {
+      cudaEventRecord(ev_[ev_used_ + 1], s);
+      ev_used_ += 2;
+      prof->ldpca_launches++;
+      prof->ldpca_codewords += G.nf;
+    }
   }
-  if (!ctx.cuda_ok(launch_final_inverse(fdev, nf, max_nsir, s), "inverse transform")) return false;
-  bool any_deblock = false;
-  for (int f = 0; f < nf; f++) any_deblock = any_deblock || fd[f].deblock;
-  if (any_deblock && !ctx.cuda_ok(launch_deblock(fdev, nf, w, h, s), "deblocking")) return false;
-  for (int f = 0; f < nf; f++)
-    if (frames[f].dbg_si_final &&
-        !ctx.cuda_ok(cudaMemcpyAsync(frames[f].dbg_si_final, fd[f].si, (size_t)w * h, cudaMemcpyDeviceToDevice, s),
+  return ctx.cuda_ok(launch_band_end(fdev, G.nf, w, h, G.max_nsir, band, ctx.xlm, s), "band reconstruction");
+}
+
+// what follows a group's last band
+bool FrameBatcher::launch_end(Context &ctx, const Group &G, cudaStream_t s) {
+  const int w = w_, h = h_;
+  FrameDev *fdev = frames_dev_.as<FrameDev>() + G.f0;
+  if (!ctx.cuda_ok(launch_final_inverse(fdev, G.nf, G.max_nsir, s), "inverse transform")) return false;
+  if (G.deblock && !ctx.cuda_ok(launch_deblock(fdev, G.nf, w, h, s), "deblocking")) return false;
+  for (int f = G.f0; f < G.f0 + G.nf; f++)
+    if (spec_copy_[f].dbg_si_final &&
+        !ctx.cuda_ok(cudaMemcpyAsync(spec_copy_[f].dbg_si_final, fd_[f].si, (size_t)w * h, cudaMemcpyDeviceToDevice, s),
                      "debug copy"))
       return false;
-
-  if (prof) prof->kernel_launches += launches_per_execute();
   return true;
+}
+
+bool FrameBatcher::execute(Context &ctx, cudaStream_t s, int max_iter, ProfileStats *prof) {
+  if (nf_ == 0) return true;
+  ev_used_ = 0;
+  if (prof) {
+    size_t launches = 0;
+    for (const Group &G : groups_) launches += G.steps.size();
+    while (ev_.size() < 2 * launches) {
+      cudaEvent_t e;
+      if (!ctx.cuda_ok(cudaEventCreate(&e), "event")) return false;
+      ev_.push_back(e);
+    }
+  }
+  const size_t ng = groups_.size();
+  if (ng > 1) {
+    if (!ctx.cuda_ok(cudaEventRecord(fork_, s), "event")) return false;
+    for (size_t g = 1; g < ng; g++)
+      if (!ctx.cuda_ok(cudaStreamWaitEvent(side_[g - 1], fork_, 0), "wait")) return false;
+  }
+  auto stream_of = [&](size_t g) { return g == 0 ? s : side_[g - 1]; };
+  bool ok = true;
+  for (size_t g = 0; g < ng && ok; g++) {
+    groups_[g].next = 0;
+    ok = launch_start(ctx, groups_[g], stream_of(g));
+  }
+  // band by band over the groups, so that none waits for another's launches
+  for (bool more = true; more && ok;) {
+    more = false;
+    for (size_t g = 0; g < ng && ok; g++) {
+      if (groups_[g].next >= groups_[g].steps.size()) continue;
+      ok = launch_band(ctx, groups_[g], stream_of(g), max_iter, prof);
+      more = true;
+    }
+  }
+  for (size_t g = 0; g < ng && ok; g++) ok = launch_end(ctx, groups_[g], stream_of(g));
+  // the batch's stream joins the others even after a failure
+  for (size_t g = 1; g < ng; g++)
+    if (!ctx.cuda_ok(cudaEventRecord(side_done_[g - 1], side_[g - 1]), "event") ||
+        !ctx.cuda_ok(cudaStreamWaitEvent(s, side_done_[g - 1], 0), "wait"))
+      return false;
+  if (ok && prof) prof->kernel_launches += launches_per_execute();
+  return ok;
 }
 
 void FrameBatcher::harvest(ProfileStats *prof) {

@@ -70,8 +70,11 @@ class FrameBatcher {
   // LDPCA jobs, uploaded once; execute: the kernels only (no host transfer, no
   // synchronisation); collect: per-bitplane results to the host.
   // concurrent_frames: frames expected to decode on the device at the same time
-  // (this batch included; 0 = this batch alone), which sets the speculation width
-  bool prepare(Context &ctx, const std::vector<FrameSpec> &frames, cudaStream_t stream, int concurrent_frames = 0);
+  // (this batch included; 0 = this batch alone), which sets the speculation
+  // width; max_groups: into how many groups on streams of their own the batch
+  // may be split
+  bool prepare(Context &ctx, const std::vector<FrameSpec> &frames, cudaStream_t stream, int concurrent_frames = 0,
+               int max_groups = 8);
   bool execute(Context &ctx, cudaStream_t stream, int max_iter = 50, ProfileStats *prof = nullptr);
   bool collect(Context &ctx, std::vector<FrameResult> &results, cudaStream_t stream);
   // asynchronous form of collect: enqueue the result copies on the stream, and
@@ -97,7 +100,6 @@ class FrameBatcher {
   std::vector<Slot> slots_;
   DevBuf frames_dev_, jobs_dev_, spec_;
   cudaStream_t alloc_stream_ = nullptr;
-  int spec_k_ = 1;  // most speculative slots per codeword of any step (the scratch's layout)
   void *pinned_ = nullptr;
   size_t pinned_bytes_ = 0;
   std::vector<void *> retired_pinned_;  // outgrown pinned buffers, freed by release()
@@ -107,13 +109,30 @@ class FrameBatcher {
     int band, bit;
     int spec_k = 1, spec_c = 1;  // speculative slots per codeword, blocks per slot
   };
-  std::vector<Step> steps_;
+  // frames [f0, f0 + nf) of the batch, which decode in lockstep; the first
+  // group on the batch's stream, the others on streams of their own
+  struct Group {
+    int f0 = 0, nf = 0, max_nsir = 0;
+    bool deblock = false;
+    std::vector<Step> steps;
+    std::vector<int> plane_of;  // [step * nf + frame]: the frame's bitplane decoded at that step, or -1
+    size_t job0 = 0;            // first of its steps.size() * nf jobs
+    int spec_k = 1;             // most speculative slots of any step (its scratch's layout)
+    size_t spec_off = 0;        // its part of the scratch
+    size_t next = 0;            // execute(): next step to launch
+  };
+  std::vector<Group> groups_;
+  std::vector<cudaStream_t> side_;      // streams of groups 1, 2, ...
+  std::vector<cudaEvent_t> side_done_;  // their ends, and the batch's start
+  cudaEvent_t fork_ = nullptr;
+  bool launch_start(Context &ctx, const Group &G, cudaStream_t s);
+  bool launch_band(Context &ctx, Group &G, cudaStream_t s, int max_iter, ProfileStats *prof);
+  bool launch_end(Context &ctx, const Group &G, cudaStream_t s);
   std::vector<FrameDev> fd_;
   std::vector<int> qb_, wz_bits0_;
-  std::vector<int> plane_of_;  // [step * frames + frame]: the frame's bitplane decoded at that step, or -1
   std::vector<const FrameSpec *> specs_;
   std::vector<FrameSpec> spec_copy_;
-  int nf_ = 0, w_ = 0, h_ = 0, max_nsir_ = 0;
+  int nf_ = 0, w_ = 0, h_ = 0;
   size_t res_off_ = 0;
   const LadderDev *L_ = nullptr;
   std::vector<cudaEvent_t> ev_;  // start/stop pairs of the LDPCA launches of one execute()

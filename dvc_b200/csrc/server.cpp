@@ -286,7 +286,7 @@ static bool start_cohort(dvc_server *S, int i) {
   int in_flight = 0;
   for (auto &o : S->cohorts) in_flight += (int)o.reqs.size();
   C.batcher.set_alloc_stream(s);
-  if (!C.batcher.prepare(c, specs, s, in_flight) || !C.batcher.execute(c, s, 50, nullptr)) return false;
+  if (!C.batcher.prepare(c, specs, s, in_flight, 1) || !C.batcher.execute(c, s, 50, nullptr)) return false;
   for (int f = 0; f < nf; f++)
     if (!c.cuda_ok(cudaMemcpyAsync(C.pinned_out + f * fs, C.out[f].p, fs, cudaMemcpyDeviceToHost, s), "D2H recon"))
       return false;
