@@ -12,6 +12,8 @@
 // with -fmad=false so no multiply-add is fused.
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include "dvc_common.cuh"
 #include "frame_types.h"
 #include "kernels.h"
@@ -166,38 +168,6 @@ __device__ __forceinline__ void warp_argmin_nonneg(double &c, int &i) {
   const unsigned mi = __reduce_min_sync(0xffffffffu, (hw == mh && lw == ml) ? (unsigned)i : 0xffffffffu);
   c = __longlong_as_double((long long)(((unsigned long long)mh << 32) | ml));
   i = (int)mi;
-}
-
-// block_argmin of two independent (cost, index) pairs with costs >= 0 in one
-// reduction; sc and si hold 2 * NT / 32 entries
-template <int NT>
-__device__ __forceinline__ void block_argmin2(double &c0, int &i0, double &c1, int &i1, double *sc, int *si) {
-  warp_argmin_nonneg(c0, i0);
-  warp_argmin_nonneg(c1, i1);
-  constexpr int NW = NT / 32;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0) {
-    sc[warp] = c0;
-    si[warp] = i0;
-    sc[NW + warp] = c1;
-    si[NW + warp] = i1;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < NW; w++) {
-      better(c0, i0, sc[w], si[w]);
-      better(c1, i1, sc[NW + w], si[NW + w]);
-    }
-    sc[0] = c0;
-    si[0] = i0;
-    sc[NW] = c1;
-    si[NW] = i1;
-  }
-  __syncthreads();
-  c0 = sc[0];
-  i0 = si[0];
-  c1 = sc[NW];
-  i1 = si[NW];
 }
 
 // ---------------------------------------------------------------- filters
@@ -1192,261 +1162,273 @@ __device__ __forceinline__ uint32_t sad4_acc(uint32_t a, uint32_t b, uint32_t c)
 // integer search against the past and future reconstructions (cost = SAD with
 // the motion-vector weight; strict-< row-major argmin), a +-1 half-pel
 // refinement in the interpolated frames, and the bidirectional average.
+//
+// One thread block takes a 16x16 tile of a frame, whose (up to) 16 WZ blocks
+// search nearly the same 80x80 pixels of either reference; a warp takes a
+// block.  What bounds it is instruction issue, so candidates are ruled out
+// eight to a lane and step before their SADs are formed: the tile's window holds,
+// for every position, the floored means of the four 2x2 quadrants of the 4x4
+// block there, one word.  With d the sum of the four mean differences (one
+// packed instruction), SAD >= 4 d - 12; the weight of a candidate is at least
+// 1 + 0.1 max(|dx|, |dy|); so one whose bound exceeds the best cost so far can
+// neither win nor tie.  0.5 to 2% of the candidates are left once the best is
+// near its final value, and it starts from the zero-motion candidate and the
+// previous band's best.  Those left are queued per warp (by groups of eight
+// columns) and weighed 32 at a time; the (cost, index) order makes the result
+// independent of the order in which candidates are weighed.
+// All SADs of a block by packed instructions took 93 us for a band of two CIF
+// frames (40 M warp instructions a frame) and 70 us for a lone one; so 72 and 43
+// us (20 M) with 256 threads, two blocks to a warp and three thread blocks an
+// SM, 74 and 50 us with 512 threads (two an SM: a frame's 396 tiles need a
+// second wave; held to 40 registers for three, 99 and 61 us).
+constexpr int kSiTile = 16;                  // pixels a side
+constexpr int kSiRows = kSiTile + 2 * 32;    // pixel rows of the window
+constexpr int kSiStride = 96;                // bytes of a pixel row: 80, and the word after any 4-byte group
+constexpr int kSiMeanStride = 84;            // bytes of a row of 2x2 means
+constexpr int kSiQuadStride = 80;            // words of a row of quadrant means
+constexpr int kSiQueue = 36;                 // groups waiting in a warp: fewer than 4, and the 32 of a step
+
+struct SiShared {
+  uint32_t quad[2][(kSiRows - 3) * kSiQuadStride];
+  uint8_t px[2][kSiRows * kSiStride];
+  uint8_t mean[(kSiRows - 1) * kSiMeanStride + 4];
+  uint16_t queue[16][kSiQueue];
+  uint16_t most[16][SEARCH_R + 4];  // by max(|dx|, |dy|): largest d that is weighed
+};
+
 template <int NT>
-__global__ void __launch_bounds__(NT) update_si_kernel(FrameDev *frames, int band) {
+__global__ void __launch_bounds__(NT, NT == 512 ? 2 : 3) update_si_kernel(FrameDev *frames, int band) {
   FrameDev &F = frames[blockIdx.y];
   if (!F.active || !in_step(F, band, 0)) return;
-  const int s_idx = blockIdx.x;
-  if (s_idx >= F.nsir) return;
+  constexpr int NW = NT / 32, BPW = 16 / NW;  // warps, WZ blocks per warp
   const int w = F.w, h = F.h, b4w = w / 4, w2 = w << 1, h2 = h << 1;
-  const int blk = F.sir[s_idx];
-  const int top = (blk / b4w) << 2, left = (blk % b4w) << 2;
-  int st = top - SEARCH_R, sb = top + SEARCH_R, sl = left - SEARCH_R, sr = left + SEARCH_R;
-  if (st < 0) st = 0;
-  if (sb > h - 4) sb = h - 4;
-  if (sl < 0) sl = 0;
-  if (sr > w - 4) sr = w - 4;
-  const int ww = sr - sl + 4, wh = sb - st + 4;  // <= 68 x 68
-  // windows with a 96-byte row stride: the bytes of [sl & ~15, sl + ww)
-  // (at most 6 16-byte chunks), so that the word after any 4-byte group of a
-  // row is still inside the row
-  constexpr int WS = 96;
-  __shared__ __align__(16) uint8_t wp[68 * WS], wf[68 * WS];
-  __shared__ uint32_t cur4[4];  // the block's rows, 4 pixels packed per word (first pixel lowest)
-  __shared__ int cur[16];
-  __shared__ double sca[2 * (NT / 32)];
-  __shared__ int sia[2 * (NT / 32)];
-  // window rows copied in 16-byte chunks straight to shared memory: lanes are
-  // (row of a pair, reference, chunk); w and the planes' bases are multiples
-  // of 16, so the chunks of [sl & ~15, sl + ww) are aligned and stay inside
-  // the frame row; the window starts at byte `wo` of each shared row
-  const int s16 = sl & ~15, wo = sl - s16, nch = (wo + ww + 15) >> 4;
+  const int tpr = w / kSiTile, ty = (int)blockIdx.x / tpr * kSiTile, tx = (int)blockIdx.x % tpr * kSiTile;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // WZ list positions of the tile's blocks, in the lanes of every warp
+  const int mine = lane < 16 ? F.sir_of_blk[((ty >> 2) + (lane >> 2)) * b4w + (tx >> 2) + (lane & 3)] : -1;
+  if (__ballot_sync(0xffffffffu, mine >= 0) == 0) return;
+  extern __shared__ __align__(16) uint8_t si_smem[];
+  SiShared &S = *reinterpret_cast<SiShared *>(si_smem);
+  // the window: rows and columns [r0, r1) x [c0, c1) of both references, in
+  // 16-byte chunks (the tile, the frame and the planes' bases are multiples of 16)
+  const int r0 = max(0, ty - SEARCH_R), r1 = min(h, ty + kSiTile + SEARCH_R);
+  const int c0 = max(0, tx - SEARCH_R), c1 = min(w, tx + kSiTile + SEARCH_R);
+  const int rows = r1 - r0;
   {
-    const int lane = threadIdx.x & 31, ch = lane & 7, ref = (lane >> 3) & 1;
-    if (ch < nch) {
-      const uint8_t *src = (ref ? F.future : F.past) + (size_t)st * w + s16 + ch * 16;
-      const uint32_t dst = (uint32_t)__cvta_generic_to_shared((ref ? wf : wp) + ch * 16);
-      for (int y = 2 * (threadIdx.x >> 5) + (lane >> 4); y < wh; y += 2 * (NT / 32))
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + y * WS), "l"(src + (size_t)y * w)
-                     : "memory");
+    const int ch = (int)threadIdx.x % 5;
+    for (int y = (int)threadIdx.x / 5; y < rows; y += NT / 5) {
+      if (16 * ch >= c1 - c0 || (int)threadIdx.x >= NT / 5 * 5) continue;
+#pragma unroll
+      for (int ref = 0; ref < 2; ref++) {
+        const uint8_t *src = (ref ? F.future : F.past) + (size_t)(r0 + y) * w + c0 + 16 * ch;
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(S.px[ref] + y * kSiStride + 16 * ch);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+      }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
   }
-  if (threadIdx.x < 16) cur[threadIdx.x] = F.recon[(top + (threadIdx.x >> 2)) * w + left + (threadIdx.x & 3)];
-  __syncthreads();
-  if (threadIdx.x < 4) {
-    const int m = threadIdx.x;
-    cur4[m] = (uint32_t)cur[4 * m] | ((uint32_t)cur[4 * m + 1] << 8) | ((uint32_t)cur[4 * m + 2] << 16) |
-              ((uint32_t)cur[4 * m + 3] << 24);
-  }
-  __syncthreads();
-  // each thread walks candidate columns of one reference: the SAD of candidate row yo
-  // is the sum over m of the 4-pixel SAD of window row yo + m against block
-  // row m, accumulated while walking the window rows once.  The weight is at
-  // least 1, so cost = sad * weight >= sad (rounding is monotone): a candidate
-  // can only match or beat the item's best if sad <= floor(best), and only
-  // those are weighed; the rest could neither win nor tie.
-  const int cw = sr - sl + 1;
-  const uint32_t c0 = cur4[0], c1 = cur4[1], c2 = cur4[2], c3 = cur4[3];
-  // 4x4 SAD of the candidate at window offset (yo, xo) of window wb
-  auto sad_at = [&](const uint8_t *wb, int yo, int xo) {
-    const uint32_t *rw = reinterpret_cast<const uint32_t *>(wb) + ((xo + wo) >> 2) + yo * (WS / 4);
-    const int sh = ((xo + wo) & 3) * 8;
-    uint32_t sad = sad4_acc(__funnelshift_r(rw[0], rw[1], sh), c0, 0u);
-    sad = sad4_acc(__funnelshift_r(rw[WS / 4], rw[WS / 4 + 1], sh), c1, sad);
-    sad = sad4_acc(__funnelshift_r(rw[WS / 2], rw[WS / 2 + 1], sh), c2, sad);
-    return (int)sad4_acc(__funnelshift_r(rw[3 * WS / 4], rw[3 * WS / 4 + 1], sh), c3, sad);
-  };
-  // every thread starts from the zero-motion candidate of each reference and
-  // from the best candidate of the block's previous refinement (the window is
-  // the same in every band); they are candidates like any other, so the lowest
-  // (cost, index) is unchanged.  Their cost bounds the item's best from the
-  // first row on, so a lane weighs only candidates near the optimum and a
-  // warp seldom takes the weighing branch
-  // (lanes 0-3 of each warp weigh the four starts; the warp shares them)
-  const int y0 = top - st, x0 = left - sl;
-  int *last = F.si_mv + 2 * s_idx;
-  double bp, bf;
-  int ip, jf;
-  {
-    const int lane = threadIdx.x & 31;
-    // lane 0: zero motion in the past window, 1: in the future one, 2 and 3:
-    // the previous band's best in each (-1 before the first band)
-    const int idx = lane < 2 ? y0 * cw + x0 : (lane < 4 ? last[lane - 2] : -1);
-    double c = 1e300;
-    if (idx >= 0) {
-      const int yo = idx / cw, xo = idx - yo * cw;
-      c = (double)sad_at((lane & 1) ? wf : wp, yo, xo) * d_si_weight[(st - top + 32 + yo) * 65 + (sl + xo - left + 32)];
-    }
-    bp = __shfl_sync(0xffffffffu, c, 0);
-    bf = __shfl_sync(0xffffffffu, c, 1);
-    ip = jf = y0 * cw + x0;
-    const double c2 = __shfl_sync(0xffffffffu, c, 2), c3 = __shfl_sync(0xffffffffu, c, 3);
-    const int i2 = __shfl_sync(0xffffffffu, idx, 2), i3 = __shfl_sync(0xffffffffu, idx, 3);
-    if (i2 >= 0) better(bp, ip, c2, i2);
-    if (i3 >= 0) better(bf, jf, c3, i3);
-  }
-  // two adjacent candidate columns (xo, xo + 1) of one reference per thread:
-  // one row read (two words) serves both, and one vote per four rows covers
-  // the eight candidates they complete.  With an odd number of columns the
-  // last column of each reference goes candidate by candidate below.
-  const int np = cw >> 1;
-  for (int pi = threadIdx.x; pi < 2 * np; pi += NT) {
-    const bool fut = pi >= np;
-    const int xo = 2 * (fut ? pi - np : pi);
-    const uint8_t *wb = fut ? wf : wp;
-    const uint32_t *row = reinterpret_cast<const uint32_t *>(wb) + ((xo + wo) >> 2);
-    const int sh = ((xo + wo) & 3) * 8;
-    const double *wt = d_si_weight + (st - top + 32) * 65 + (sl + xo - left + 32);
-    // running SADs of candidate rows y-3 .. y (indexed by row & 3) of both columns
-    int pa[4] = {0, 0, 0, 0}, pb[4] = {0, 0, 0, 0};
-    double best = fut ? bf : bp;
-    int bi = fut ? jf : ip, thr = (int)best;
-    // window row y is row m of candidate y - m; candidate y - 3 is complete at row y
-    auto add_row = [&](int y, int slot) {
-      const uint32_t *rw = row + y * (WS / 4);
-      const uint32_t lo = rw[0], hi = rw[1];
-      const uint32_t va = __funnelshift_r(lo, hi, sh), vb = __funnelshift_rc(lo, hi, sh + 8);
-      pa[slot & 3] = (int)sad4_acc(va, c0, 0u);
-      pb[slot & 3] = (int)sad4_acc(vb, c0, 0u);
-      pa[(slot - 1) & 3] = (int)sad4_acc(va, c1, (uint32_t)pa[(slot - 1) & 3]);
-      pb[(slot - 1) & 3] = (int)sad4_acc(vb, c1, (uint32_t)pb[(slot - 1) & 3]);
-      pa[(slot - 2) & 3] = (int)sad4_acc(va, c2, (uint32_t)pa[(slot - 2) & 3]);
-      pb[(slot - 2) & 3] = (int)sad4_acc(vb, c2, (uint32_t)pb[(slot - 2) & 3]);
-      pa[(slot - 3) & 3] = (int)sad4_acc(va, c3, (uint32_t)pa[(slot - 3) & 3]);
-      pb[(slot - 3) & 3] = (int)sad4_acc(vb, c3, (uint32_t)pb[(slot - 3) & 3]);
-    };
-    // column xo + xc, candidate row yo
-    auto weigh = [&](int yo, int xc, int sad) {
-      if (sad <= thr) {
-        const double cst = (double)sad * __ldg(wt + yo * 65 + xc);
-        const int idx = yo * cw + xo + xc;
-        if (cst < 10000000.0 && (cst < best || (cst == best && idx < bi))) {
-          best = cst;
-          bi = idx;
-          thr = (int)best;
-        }
-      }
-    };
-    // rows 0..2 only start candidates (wh >= 4 always: the window holds the block)
-    add_row(0, 0);
-    add_row(1, 1);
-    add_row(2, 2);
-    int y = 3;
-    // slots of rows y .. y+3 are 3, 0, 1, 2 (y = 3 mod 4); the candidates
-    // completed by a group are weighed after it, and only when one lane of the
-    // warp has one that can match its best (the lanes run the same rows, so
-    // the vote is taken by the whole active warp): a warp branches once per
-    // four rows, and rarely.  The (cost, index) order makes the result
-    // independent of the order in which candidates are weighed.
-    for (; y + 3 < wh; y += 4) {
-      int sa[4], sb[4];
+  // the thread's column (four pixels) and run of rows when the means are made
+  constexpr int RUN = (kSiRows + NT / 20 - 1) / (NT / 20);
+  const int by_ = (int)threadIdx.x / 20 * RUN, bx_ = by_ < kSiRows ? (int)threadIdx.x % 20 : 20, mcols = (c1 - c0) >> 2;
+  const float inv_w = 1.0001f / (1.0f + 0.1f * (float)lane);  // over the weight of a candidate lane away, rounded up
 #pragma unroll
-      for (int r = 0; r < 4; r++) {
-        add_row(y + r, 3 + r);
-        sa[r] = pa[r & 3];
-        sb[r] = pb[r & 3];
-      }
-      const int mn = min(min(min(sa[0], sa[1]), min(sa[2], sa[3])), min(min(sb[0], sb[1]), min(sb[2], sb[3])));
-      if (__any_sync(__activemask(), mn <= thr)) {
+  for (int ref = 0; ref < 2; ref++) {
+    __syncthreads();
+    // means of 2x2 pixels at every position, four to a word, a run of rows per
+    // thread: the pair sums of a row serve the means above and below it
+    if (bx_ < mcols) {
+      constexpr uint32_t M = 0x00ff00ffu;
+      const uint32_t *p = reinterpret_cast<const uint32_t *>(S.px[ref]) + by_ * (kSiStride / 4) + bx_;
+      uint32_t *o = reinterpret_cast<uint32_t *>(S.mean) + by_ * (kSiMeanStride / 4) + bx_;
+      uint32_t even = 0, odd = 0;
 #pragma unroll
-        for (int r = 0; r < 4; r++) {
-          weigh(y + r - 3, 0, sa[r]);
-          weigh(y + r - 3, 1, sb[r]);
+      for (int i = 0; i <= RUN; i++) {
+        if (by_ + i < rows) {
+          const uint32_t v = p[i * (kSiStride / 4)], u = __funnelshift_r(v, p[i * (kSiStride / 4) + 1], 8);
+          const uint32_t e = (v & M) + (u & M), d = ((v >> 8) & M) + ((u >> 8) & M);
+          if (i > 0) o[(i - 1) * (kSiMeanStride / 4)] = (((even + e) >> 2) & M) | ((((odd + d) >> 2) & M) << 8);
+          even = e;
+          odd = d;
         }
       }
     }
-    for (; y < wh; y++) {  // the last rows; y - 3 mod 4 as above
-      const uint32_t *rw = row + y * (WS / 4);
-      const uint32_t lo = rw[0], hi = rw[1];
-      const int q = y & 3;
-      const int done = (q + 1) & 3;  // slot of candidate y - 3
-      // the same updates with the slot of row y known only at run time:
-      // slot q gets the new candidate, q-1 += row 1, q-2 += row 2, q-3 (= q+1) += row 3
+    __syncthreads();
+    // the four quadrants' means of the block at every position, one word each
+    if (bx_ < mcols) {
+      const uint32_t *m = reinterpret_cast<const uint32_t *>(S.mean) + by_ * (kSiMeanStride / 4) + bx_;
+      uint4 *o = reinterpret_cast<uint4 *>(S.quad[ref] + by_ * kSiQuadStride) + bx_;
+      uint32_t h0[RUN + 2], h1[RUN + 2];  // left and right means of a row's positions, side by side
 #pragma unroll
-      for (int xc = 0; xc < 2; xc++) {
-        const uint32_t v = xc ? __funnelshift_rc(lo, hi, sh + 8) : __funnelshift_r(lo, hi, sh);
-        int *part = xc ? pb : pa;
-        const int s0 = (int)__vsadu4(v, c0), s1 = (int)__vsadu4(v, c1), s2 = (int)__vsadu4(v, c2),
-                  s3 = (int)__vsadu4(v, c3);
-        int n[4] = {part[0], part[1], part[2], part[3]};
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          const int d = (q - k) & 3;  // 0: new candidate, 1..3: candidates started 1..3 rows ago
-          n[k] = d == 0 ? s0 : d == 1 ? n[k] + s1 : d == 2 ? n[k] + s2 : n[k] + s3;
+      for (int i = 0; i < RUN + 2; i++) {
+        if (by_ + i < rows - 1) {
+          const uint32_t l = m[i * (kSiMeanStride / 4)], r = __funnelshift_r(l, m[i * (kSiMeanStride / 4) + 1], 16);
+          h0[i] = __byte_perm(l, r, 0x5140);
+          h1[i] = __byte_perm(l, r, 0x7362);
+          if (i >= 2)
+            o[(i - 2) * (kSiQuadStride / 4)] =
+                make_uint4(__byte_perm(h0[i - 2], h0[i], 0x5410), __byte_perm(h0[i - 2], h0[i], 0x7632),
+                           __byte_perm(h1[i - 2], h1[i], 0x5410), __byte_perm(h1[i - 2], h1[i], 0x7632));
         }
-        part[0] = n[0];
-        part[1] = n[1];
-        part[2] = n[2];
-        part[3] = n[3];
-        weigh(y - 3, xc, done == 0 ? n[0] : done == 1 ? n[1] : done == 2 ? n[2] : n[3]);
       }
     }
-    if (fut) better(bf, jf, best, bi);
-    else better(bp, ip, best, bi);
-  }
-  if (cw & 1) {
-    // the last column (cw - 1) of each reference: candidate k of the past
-    // window's column for k < nrow, of the future window's above
-    const int nrow = wh - 3, xo = cw - 1;
-    for (int k = threadIdx.x; k < 2 * nrow; k += NT) {
-      const bool fut = k >= nrow;
-      const int yo = k - (fut ? nrow : 0);
-      const int sad = sad_at(fut ? wf : wp, yo, xo);
-      const double cst = (double)sad * __ldg(d_si_weight + (st - top + 32 + yo) * 65 + (sl + xo - left + 32));
-      if (cst < 10000000.0) {
-        if (fut) better(bf, jf, cst, yo * cw + xo);
-        else better(bp, ip, cst, yo * cw + xo);
-      }
-    }
-  }
-  block_argmin2<NT>(bp, ip, bf, jf, sca, sia);
-  if (threadIdx.x == 0) {
-    last[0] = ip;
-    last[1] = jf;
-  }
-  // subPelRefine in the half-pel planes, no vector weight
-  // (sideInfoCreation.cpp:598-640): one thread per (reference, offset) SAD,
-  // then the strict-< scan over the offsets in the reference's (di, dj) order
-  __shared__ int ssad[18];
-  __shared__ int sbest[2][2];
-  const int t = threadIdx.x;
-  if (t < 18) {
-    const int which = t >= 9, k = t - 9 * which;
-    const int id = which ? jf : ip;
-    const int tt = ((st + id / cw) << 1) + k / 3 - 1, ll = ((sl + id % cw) << 1) + k % 3 - 1;
-    int sad = -1;  // offset outside the half-pel plane: not a candidate
-    if (tt >= 0 && tt <= h2 - 8 && ll >= 0 && ll <= w2 - 8) {
-      const uint8_t *ref = which ? F.future_ip : F.past_ip;
-      sad = 0;
-      for (int m = 0; m < 4; m++)
-        for (int n = 0; n < 4; n++) sad += abs(cur[4 * m + n] - (int)ref[(tt + 2 * m) * w2 + ll + 2 * n]);
-    }
-    ssad[t] = sad;
   }
   __syncthreads();
-  if (t < 2) {
-    const int id = t ? jf : ip;
-    const int by = st + id / cw, bx = sl + id % cw;
-    double minc = 10000000.0;
-    int nbx = bx, nby = by;
-    for (int k = 0; k < 9; k++) {
-      const int sad = ssad[9 * t + k];
-      if (sad >= 0 && (double)sad < minc) {
-        minc = (double)sad;
-        nbx = (bx << 1) + k % 3 - 1;
-        nby = (by << 1) + k / 3 - 1;
+#pragma unroll
+  for (int bw = 0; bw < BPW; bw++) {
+    const int blk = warp + bw * NW, s_idx = __shfl_sync(0xffffffffu, mine, blk);
+    if (s_idx < 0) continue;
+    const int top = ty + (blk >> 2) * 4, left = tx + (blk & 3) * 4;
+    const int st = max(0, top - SEARCH_R), sb = min(h - 4, top + SEARCH_R);
+    const int sl = max(0, left - SEARCH_R), sr = min(w - 4, left + SEARCH_R);
+    const int cw = sr - sl + 1, nrow = sb - st + 1;  // cw is one more than a multiple of 4
+    const int y0 = top - st, x0 = left - sl;         // zero motion; x0 is a multiple of 4
+    const double *wt = d_si_weight + (SEARCH_R - y0) * 65 + SEARCH_R - x0;
+    uint16_t *most = S.most[warp], *queue = S.queue[warp];
+    uint32_t cur[4], cq = 0;
+#pragma unroll
+    for (int m = 0; m < 4; m++) cur[m] = *reinterpret_cast<const uint32_t *>(F.recon + (size_t)(top + m) * w + left);
+#pragma unroll
+    for (int m = 0; m < 2; m++) {
+      constexpr uint32_t M = 0x00ff00ffu;
+      const uint32_t v = (cur[2 * m] & M) + ((cur[2 * m] >> 8) & M) + (cur[2 * m + 1] & M) + ((cur[2 * m + 1] >> 8) & M);
+      cq |= ((v & 0xffffu) >> 2 | (v >> 18) << 8) << (16 * m);
+    }
+    // a candidate is row << 8 | column of the block's window, in the scan's order
+    const int zero = y0 << 8 | x0, last = lane < 2 ? F.si_mv[2 * s_idx + lane] : -1;
+    int found[2];
+#pragma unroll
+    for (int ref = 0; ref < 2; ref++) {
+      const uint32_t *px = reinterpret_cast<const uint32_t *>(S.px[ref]) + (st - r0) * (kSiStride / 4) + ((sl - c0) >> 2);
+      const uint32_t *quad = S.quad[ref] + (st - r0) * kSiQuadStride + (sl - c0);
+      // SAD of the candidate in row r, column x
+      auto sad_at = [&](int r, int x) {
+        const uint32_t *p = px + r * (kSiStride / 4) + (x >> 2);
+        const int sh = (x & 3) * 8;
+        uint32_t sad = 0;
+#pragma unroll
+        for (int m = 0; m < 4; m++, p += kSiStride / 4) sad = sad4_acc(__funnelshift_r(p[0], p[1], sh), cur[m], sad);
+        return sad;
+      };
+      // zero motion (lane 0) and the previous band's best (lane 1; -1 before the first band)
+      double best;
+      int bi = zero;
+      {
+        const int prev = __shfl_sync(0xffffffffu, last, ref), at = lane == 1 && prev >= 0 ? prev : zero;
+        const int r = at >> 8, x = at & 255;
+        const double c = (double)(int)sad_at(r, x) * __ldg(wt + r * 65 + x);
+        best = __shfl_sync(0xffffffffu, c, 0);
+        const double c1 = __shfl_sync(0xffffffffu, c, 1);
+        if (prev >= 0) better(best, bi, c1, prev);
+      }
+      auto set_most = [&]() {
+        __syncwarp();
+        const float b = (float)best;
+        most[lane] = (uint16_t)(((int)(b * inv_w) + 1 + 12) >> 2);
+        if (lane < 2) most[SEARCH_R + lane] = (uint16_t)(((int)(b * (1.0001f / 4.2f)) + 1 + 12) >> 2);
+        __syncwarp();
+      };
+      set_most();
+      int cnt = 0;
+      // weigh the last n (at most 4) groups of the queue, a lane per candidate
+      auto weigh = [&](int n) {
+        __syncwarp();
+        cnt -= n;
+        const int e = queue[cnt + min(lane >> 3, n - 1)], r = e >> 4, x = min(8 * (e & 15) + (lane & 7), cw - 1);
+        // d <= most means SAD <= 4 most - 9 for the same distance: most groups end here
+        const uint32_t sad = sad_at(r, x);
+        const bool near = (int)sad <= 4 * (int)most[max(abs(x - x0), abs(r - y0))] - 9;
+        if (__any_sync(0xffffffffu, near)) {
+          int i = r << 8 | x;
+          double c = near ? (double)(int)sad * __ldg(wt + r * 65 + x) : 1e300;
+          const bool win = c < best || (c == best && i < bi);
+          if (__any_sync(0xffffffffu, win)) {
+            if (!win) {
+              c = 1e300;
+              i = 0x7fffffff;
+            }
+            warp_argmin_nonneg(c, i);
+            best = c;
+            bi = i;
+            set_most();
+          }
+        }
+        __syncwarp();
+      };
+      // queue the groups (row r, group g) of the lanes that hit, weigh when there are 4
+      auto add = [&](uint32_t hits, int entry) {
+        if (hits >> lane & 1u) queue[cnt + __popc(hits & ((1u << lane) - 1u))] = (uint16_t)entry;
+        cnt += __popc(hits);
+        while (cnt >= 4) weigh(4);
+      };
+      // four rows a step, from the block's own row outwards; eight groups of
+      // eight columns a row, a group per lane (a group past the window's
+      // columns may hit: its candidates count as the last column's)
+      const int g = lane & 7, down = (lane >> 3) & 1, odd = lane >> 4;
+      const int dx = min(max(max(8 * g - x0, x0 - 8 * g - 7), 0), SEARCH_R);
+      const int have = down ? nrow - 1 - y0 : y0 + 1;                 // rows on this lane's side
+      const int mine_n = 8 * g < cw - 1 ? (have - odd + 1) >> 1 : 0;  // steps in which it has one
+      const int r_0 = down ? y0 + 1 + odd : y0 - odd, r_s = down ? 2 : -2;
+      const int steps = (max(y0 + 1, nrow - 1 - y0) + 1) >> 1;
+      const uint32_t most_a = (uint32_t)__cvta_generic_to_shared(most) + 2 * (down + odd);
+      const int stride = r_s * 4 * kSiQuadStride, dx2 = 2 * (dx - down - odd);
+      // a lane without rows stays on the block's own row
+      uint32_t qa = (uint32_t)__cvta_generic_to_shared(quad + 8 * g + (mine_n > 0 ? r_0 : y0) * kSiQuadStride);
+      for (int s = 0; s < steps; s++) {
+        uint32_t q0, q1, q2, q3, q4, q5, q6, q7, far;
+        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(q0), "=r"(q1), "=r"(q2), "=r"(q3) : "r"(qa) : "memory");
+        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4 + 16];" : "=r"(q4), "=r"(q5), "=r"(q6), "=r"(q7) : "r"(qa) : "memory");
+        asm volatile("{\n\t.reg .u16 t;\n\tld.shared.u16 t, [%1];\n\tcvt.u32.u16 %0, t;\n\t}" : "=r"(far) : "r"(most_a + max(dx2, 4 * s)) : "memory");
+        const uint32_t a = __vimin3_u32(sad4_acc(q0, cq, 0u), sad4_acc(q1, cq, 0u), sad4_acc(q2, cq, 0u));
+        const uint32_t b = __vimin3_u32(sad4_acc(q3, cq, 0u), sad4_acc(q4, cq, 0u), sad4_acc(q5, cq, 0u));
+        const uint32_t d = min(__vimin3_u32(sad4_acc(q6, cq, 0u), sad4_acc(q7, cq, 0u), a), b);
+        const uint32_t hits = __ballot_sync(0xffffffffu, d <= far && s < mine_n);
+        if (hits) add(hits, (r_0 + r_s * s) << 4 | g);
+        if (s + 1 < mine_n) qa += stride;
+      }
+      for (int rr = 0; rr < nrow; rr += 32) {  // the last column
+        const int r = min(rr + lane, nrow - 1);
+        const uint32_t d = sad4_acc(quad[r * kSiQuadStride + cw - 1], cq, 0u);
+        const uint32_t hits = __ballot_sync(0xffffffffu, d <= most[max(cw - 1 - x0, abs(r - y0))] && rr + lane < nrow);
+        if (hits) add(hits, r << 4 | (cw - 1) >> 3);
+      }
+      while (cnt > 0) weigh(min(cnt, 4));
+      found[ref] = bi;
+    }
+    if (lane < 2) F.si_mv[2 * s_idx + lane] = lane ? found[1] : found[0];
+    // subPelRefine in the half-pel planes, no vector weight
+    // (sideInfoCreation.cpp:598-640): one lane per (reference, offset) SAD,
+    // then the strict-< scan over the offsets in the reference's (di, dj) order
+    const int which = lane >= 9, k = lane - 9 * which, mv = which ? found[1] : found[0];
+    int sad = 0x7fffffff;  // offset outside the half-pel plane: not a candidate
+    if (lane < 18) {
+      const int tt = ((st + (mv >> 8)) << 1) + k / 3 - 1, ll = ((sl + (mv & 255)) << 1) + k % 3 - 1;
+      if (tt >= 0 && tt <= h2 - 8 && ll >= 0 && ll <= w2 - 8) {
+        const uint8_t *p = (which ? F.future_ip : F.past_ip) + tt * w2 + ll;
+        sad = 0;
+#pragma unroll
+        for (int m = 0; m < 4; m++)
+#pragma unroll
+          for (int n = 0; n < 4; n++) sad += abs((int)(cur[m] >> (8 * n) & 255u) - (int)__ldg(p + 2 * m * w2 + 2 * n));
       }
     }
-    sbest[t][0] = nbx;
-    sbest[t][1] = nby;
-  }
-  __syncthreads();
-  if (t < 16) {
-    const int m = t >> 2, n = t & 3;
-    const double pv = (double)F.past_ip[(sbest[0][1] + 2 * m) * w2 + sbest[0][0] + 2 * n];
-    const double fv = (double)F.future_ip[(sbest[1][1] + 2 * m) * w2 + sbest[1][0] + 2 * n];
-    F.si[(top + m) * w + left + n] = (uint8_t)(int)(pv * F.ipc + fv * F.ifc);
+    int off[2];  // first offset with the lowest SAD, or 9: none (the integer position, as the reference leaves it)
+#pragma unroll
+    for (int ref = 0; ref < 2; ref++) {
+      const int v = (lane >= 9 * ref && lane < 9 * ref + 9) ? sad : 0x7fffffff;
+      const int least = __reduce_min_sync(0xffffffffu, v);
+      off[ref] = least == 0x7fffffff ? 9 : __ffs(__ballot_sync(0xffffffffu, v == least)) - 1 - 9 * ref;
+    }
+    if (lane < 16) {
+      const int m = lane >> 2, n = lane & 3;
+      double v[2];
+#pragma unroll
+      for (int ref = 0; ref < 2; ref++) {
+        const int y = st + (found[ref] >> 8), x = sl + (found[ref] & 255), o = off[ref];
+        const int yy = o < 9 ? (y << 1) + o / 3 - 1 : y, xx = o < 9 ? (x << 1) + o % 3 - 1 : x;
+        v[ref] = (double)(ref ? F.future_ip : F.past_ip)[(yy + 2 * m) * w2 + xx + 2 * n];
+      }
+      F.si[(top + m) * w + left + n] = (uint8_t)(int)(v[0] * F.ipc + v[1] * F.ifc);
+    }
   }
 }
 
@@ -1738,10 +1720,10 @@ static inline dim3 g2(int n, int tpb, int frames) { return dim3((n + tpb - 1) / 
 // threads per search block of the two motion searches (the candidate columns
 // or positions each thread walks follow from it); process-wide, set when a
 // context is created (dvc_b200.autotune picks them; the output never depends on them)
-static int g_si_threads = 64, g_fme_threads = 256;
+static int g_si_threads = 256, g_fme_threads = 256;
 
 void set_me_shapes(int si_threads, int fme_threads) {
-  g_si_threads = (si_threads == 128 || si_threads == 256) ? si_threads : 64;
+  g_si_threads = si_threads == 512 ? 512 : 256;
   g_fme_threads = (fme_threads == 128 || fme_threads == 512) ? fme_threads : 256;
 }
 
@@ -1797,16 +1779,30 @@ cudaError_t launch_cond_bit(FrameDev *fr, int nf, int w, int h, const XlmDev &xt
   return cudaGetLastError();
 }
 
+template <int NT>
+static cudaError_t launch_update_si(FrameDev *fr, dim3 tiles, int band, cudaStream_t s) {
+  // the attribute is per device: set it once for each device
+  static std::atomic<uint64_t> attr_set{0};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const uint64_t bit = 1ull << (dev & 63);
+  if (!(attr_set.load() & bit)) {
+    e = cudaFuncSetAttribute(update_si_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SiShared));
+    if (e != cudaSuccess) return e;
+    attr_set.fetch_or(bit);
+  }
+  update_si_kernel<NT><<<tiles, NT, sizeof(SiShared), s>>>(fr, band);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_band_end(FrameDev *fr, int nf, int w, int h, int max_nsir, int band, const XlmDev &xt,
                             cudaStream_t s) {
   if (max_nsir <= 0) return cudaSuccess;
   recon_kernel<<<g2(max_nsir, 128, nf), 128, 0, s>>>(fr, band);
-  if (g_si_threads == 64)
-    update_si_kernel<64><<<dim3(max_nsir, nf), 64, 0, s>>>(fr, band);
-  else if (g_si_threads == 256)
-    update_si_kernel<256><<<dim3(max_nsir, nf), 256, 0, s>>>(fr, band);
-  else
-    update_si_kernel<128><<<dim3(max_nsir, nf), 128, 0, s>>>(fr, band);
+  const dim3 tiles((w / kSiTile) * (h / kSiTile), nf);
+  const cudaError_t e = g_si_threads == 256 ? launch_update_si<256>(fr, tiles, band, s) : launch_update_si<512>(fr, tiles, band, s);
+  if (e != cudaSuccess) return e;
   over_complete_kernel<<<dim3((w - 3 + 127) / 128, nf, h - 3), 128, 0, s>>>(fr, band);
   update_smf_kernel<<<g2(max_nsir * 32, 128, nf), 128, 0, s>>>(fr, xt, band);
   update_ml_kernel<<<g2(max_nsir * 16, 128, nf), 128, 0, s>>>(fr, band);

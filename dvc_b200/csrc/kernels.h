@@ -27,8 +27,8 @@ cudaError_t launch_ldpca_spec(const LadderDev &L, const LdpcaJob *jobs_dev, int 
 // threads per codeword block of the ladder kernel: CIF 1024 or 512, QCIF 1024,
 // 512 or 256 (other values select the defaults, 1024 for both)
 void set_ldpca_threads(int nt, int nt_qcif);
-// threads per search block of updateSI (64, 128 or 256) and of the forward
-// motion search (128, 256 or 512); other values select 128 and 256
+// threads per updateSI tile (256 or 512) and per forward motion search block
+// (128, 256 or 512); other values select 256
 void set_me_shapes(int si_threads, int fme_threads);
 // L2 persisting access window of the LDPCA kernels' table reads (num_bytes 0: none)
 void set_phi_window(const void *base, size_t num_bytes, float hit_ratio);
