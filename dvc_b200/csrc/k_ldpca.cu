@@ -75,7 +75,11 @@ __global__ void __launch_bounds__(NT, MINB)
   // a slot that starts after its codeword has been decoded by a lower code
   // than its own has nothing to do
   bool late = false;
-  if (spec && kk > 0 && kk < K - 1) {  // the last slot reports the bound
+  // the slot that reports the bound: an early one, which has an SM from the
+  // start even when there are more slots than SMs (the last one held up every
+  // bitplane step of a lone CIF frame by 13 us)
+  const int reporter = min(K - 1, 3);
+  if (spec && kk > 0 && kk != reporter) {
     int l = 0;
     if (lead) {
       const int best = *(volatile int *)(sp.best + j);
@@ -92,17 +96,18 @@ __global__ void __launch_bounds__(NT, MINB)
   float llr[MAXC], part = 0.0f;
   ld_llr(g, n, J.lr, xt, xs, llr, S.msg, (J.llr_out && kk == 0) ? J.llr_out : nullptr, J.llr_in, J.term_in, &part);
   ld_stage_acc(g, J.acc, n, S.accs);
-  // The bound itself is only needed where it is reported (by the slot with the
-  // least likely code, whose delay matters least) and when the parallel sum
-  // leaves the start code open.
+  // The bound itself is only needed where it is reported and when the parallel
+  // sum leaves the start code open.
   start = J.use_given_entropy ? ld_start_code(L, J.given_entropy) : ld_start_near(g, L, part, s_ured, &s_ctl);
-  if (start < 0 || kk == K - 1) {
+  if (J.use_given_entropy) {
+    if (lead && kk == reporter && J.entropy) *J.entropy = J.given_entropy;
+  } else if (start < 0 || kk == reporter) {
     g.sync_all();
     int exact = start;
     if (lead) {
       const float h = ld_entropy_sum(S.msg, n);
       if (exact < 0) exact = ld_start_code(L, h);
-      if (J.entropy && kk == K - 1) *J.entropy = J.use_given_entropy ? J.given_entropy : h;
+      if (J.entropy && kk == reporter) *J.entropy = h;
     }
     start = g.bcast(exact, &s_word[1]);
   }
