@@ -62,6 +62,10 @@ extern "C" void dvc_destroy(dvc_ctx *ctx) {
 
 extern "C" const char *dvc_last_error(dvc_ctx *ctx) { return ctx ? ctx->c.err.c_str() : "null context"; }
 
+static int ldpca_batch_run(Context &c, int count, const int *n, const float *lr, const uint8_t *acc, const uint8_t *crc,
+                           const int *start, uint8_t *decoded, int *results, float *entropy, int max_iter,
+                           long long *bp_iterations, double *kernel_ms);
+
 static int ldpca_run(Context &c, int n, int count, const float *lr, const uint8_t *acc, const uint8_t *crc,
                      uint8_t *decoded, int *results, float *entropy, int max_iter, const float *given_entropy,
                      float *llr_back) {
@@ -73,6 +77,23 @@ static int ldpca_run(Context &c, int n, int count, const float *lr, const uint8_
   if (count <= 0 || !lr || !acc || !crc || !results || max_iter <= 0) {
     c.err = "dvc_ldpca_decode: bad arguments";
     return DVC_E_ARG;
+  }
+  int sms = 148, st;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
+  // Two codewords and more per SM go through the batched form's work queue: no
+  // last wave of half-empty SMs, and four QCIF codewords share a block.  Slots
+  // -> queue, ms: QCIF 200 codewords 3.9 -> 4.0, 300 5.7 -> 5.3, 592 10.5 ->
+  // 9.0; CIF 203 13.4 -> 13.3, 400 24.4 -> 23.3, 592 34.8 -> 33.2.  Against a
+  // block per ladder: QCIF 600 13.0 -> 8.9, 2400 39.2 -> 30.8; CIF 600 38.4 ->
+  // 34.1, 1000 60.1 -> 56.1.  Without memory for the queue, the forms below.
+  const bool queue = count >= 2 * sms && !given_entropy && !llr_back;
+  if (queue) {
+    const std::vector<int> ns(count, n);
+    st = ldpca_batch_run(c, count, ns.data(), lr, acc, crc, nullptr, decoded, results, entropy, max_iter, nullptr,
+                         nullptr);
+    if (st == DVC_OK || st == DVC_E_CUDA) return st;
+    for (auto *b : {&c.bt_lr, &c.bt_acc, &c.bt_dec, &c.bt_res, &c.bt_ent, &c.bt_cw, &c.bt_state}) b->release();
+    cudaGetLastError();  // the failed allocation's, or the next launch would report it
   }
   const size_t nb = (size_t)n / 8;
   if (!c.ld_lr.ensure((size_t)count * n * 4) || !c.ld_acc.ensure((size_t)count * nb) ||
@@ -100,20 +121,17 @@ static int ldpca_run(Context &c, int n, int count, const float *lr, const uint8_
     if (llr_back) j.llr_out = c.ld_llr.as<float>() + (size_t)i * n;  // apart from lr, which other slots read
   }
   cudaStream_t s = c.stream;
-  int st;
   // Codewords that leave SMs idle are decoded with speculative slots (and
-  // clusters); beyond four per SM a block walks each ladder alone, without
-  // scratch.  One codeword alone, sequential -> so: QCIF 2.2
+  // clusters), others by a block per ladder, without scratch.  One codeword alone, sequential -> so: QCIF 2.2
   // -> 0.26 ms, CIF 7.9 -> 0.43 ms; 33 QCIF codewords 4.5 -> 0.89 ms, 203 CIF
   // ones 19.8 -> 13.2 ms.
-  int sms = 148, K = 1, C = 1;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
+  int K = 1, C = 1;
   dvc::LdpcaSpec sp;
-  if (count <= 4 * sms) {
+  if (count < 2 * sms) {
     dvc::ldpca_spec_shape(n, count, sms, K, C);
-    // once for every count (at most 4 * sms slots of either length by default)
+    // once for every count (by default fewer than 2 * sms codewords of either length)
     const size_t had = c.ld_spec.bytes;
-    if (!c.ld_spec.ensure(std::max(dvc::ldpca_spec_scratch_bytes(6336, 4 * sms, 4),
+    if (!c.ld_spec.ensure(std::max(dvc::ldpca_spec_scratch_bytes(6336, 2 * sms, 4),
                                    dvc::ldpca_spec_scratch_bytes(n, count, K)))) {
       c.err = "device allocation failed";
       return DVC_E_NOMEM;
@@ -165,11 +183,9 @@ extern "C" int dvc_ldpca_decode(dvc_ctx *ctx, int n, int count, const float *lr,
   return ldpca_run(ctx->c, n, count, lr, acc, crc, decoded, results, entropy, max_iter, nullptr, nullptr);
 }
 
-extern "C" int dvc_ldpca_decode_batch(dvc_ctx *ctx, int count, const int *n, const float *lr, const uint8_t *acc,
-                                      const uint8_t *crc, const int *start, uint8_t *decoded, int *results,
-                                      float *entropy, int max_iter, long long *bp_iterations, double *kernel_ms) {
-  if (!ctx) return DVC_E_ARG;
-  Context &c = ctx->c;
+static int ldpca_batch_run(Context &c, int count, const int *n, const float *lr, const uint8_t *acc, const uint8_t *crc,
+                           const int *start, uint8_t *decoded, int *results, float *entropy, int max_iter,
+                           long long *bp_iterations, double *kernel_ms) {
   if (count <= 0 || count > (1 << 22) || !n || !lr || !acc || !crc || !results || max_iter <= 0) {
     c.err = "dvc_ldpca_decode_batch: bad arguments";
     return DVC_E_ARG;
@@ -277,6 +293,14 @@ extern "C" int dvc_ldpca_decode_batch(dvc_ctx *ctx, int count, const int *n, con
   if (e1) cudaEventDestroy(e1);
   if (!st && bp_iterations) *bp_iterations = (long long)work;
   return st;
+}
+
+extern "C" int dvc_ldpca_decode_batch(dvc_ctx *ctx, int count, const int *n, const float *lr, const uint8_t *acc,
+                                      const uint8_t *crc, const int *start, uint8_t *decoded, int *results,
+                                      float *entropy, int max_iter, long long *bp_iterations, double *kernel_ms) {
+  if (!ctx) return DVC_E_ARG;
+  return ldpca_batch_run(ctx->c, count, n, lr, acc, crc, start, decoded, results, entropy, max_iter, bp_iterations,
+                         kernel_ms);
 }
 
 extern "C" int dvc_ldpca_encode(dvc_ctx *ctx, int n, int count, const uint8_t *bits, uint8_t *acc, uint8_t *crc) {

@@ -57,3 +57,21 @@ def test_shapes_match_the_oracle(gpu_ctx):
                                                            int(crc[i]), float(ent[i]))
             assert (res[i, 0], res[i, 1], res[i, 2]) == (orate, ostart, oacc)
             assert np.array_equal(dec[i], odec)
+
+
+@pytest.mark.parametrize("n,per_sm,more", [(1584, 2, -1), (1584, 2, 0), (1584, 4, 1), (6336, 2, -1), (6336, 2, 0)])
+def test_queue_from_two_codewords_per_sm(gpu_ctx, n, per_sm, more):
+    """Either side of the count from which a call goes through the work queue,
+    against the same codewords in calls of a few (slots), with a full-rate and an
+    all-zero-information codeword among them and without the optional outputs."""
+    import torch
+    from dvc_b200 import ldpca_bench as lb
+    count = per_sm * torch.cuda.get_device_properties(0).multi_processor_count + more
+    lr, acc, crc, x = lb.make_codewords(n, count, 1000 + count)
+    lr[0] = 1.0              # no information: the bound asks for the full rate
+    crc[count - 1] ^= 0x5A   # no code's bits match: the ladder's end
+    dec, res, ent = gpu_ctx.ldpca_decode(lr, acc, crc)
+    for i in sorted({0, count // 2, count - 1} | set(range(0, count, 37))):
+        d, r, e = gpu_ctx.ldpca_decode(lr[i:i + 1], acc[i:i + 1], crc[i:i + 1])
+        assert np.array_equal(res[i], r[0]) and np.array_equal(dec[i], d[0])
+        assert ent[i:i + 1].view(np.uint32)[0] == e.view(np.uint32)[0]
