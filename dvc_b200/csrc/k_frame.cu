@@ -1443,79 +1443,92 @@ __device__ __forceinline__ uint32_t load4_u8(const uint8_t *a) {
   return __funnelshift_r(lo, hi, sh);
 }
 
-// updateSMF, motionLearning.cpp:70-127: one warp per WZ block.  The block's
-// float sum of squared pixel differences only ever holds integers below 2^24
-// (16 terms of at most 255^2), so every float step of it is exact and it
-// equals the integer sum, taken here four pixels at a time (vabsdiffu4, dp4a).
-__global__ void update_smf_kernel(FrameDev *frames, XlmDev xt, int band) {
+// updateSMF, motionLearning.cpp:70-127, and update_si_ML, :129-160: a block's
+// candidate probabilities, and with them the ML side coefficients of the bands
+// above `band`.  The block's float sum of squared pixel differences only ever
+// holds integers below 2^24 (16 terms of at most 255^2), so every float step of
+// it is exact and it equals the integer sum, taken here four pixels at a time
+// (vabsdiffu4, dp4a).  Both sums run in candidate order, so a block is a chain
+// of 81 adds and then one of 81 multiply-adds per coefficient; what bounds the
+// kernel is their latency and the window loads'.  Sixteen lanes take a block: they
+// share its candidates, three loads of a window in flight, all walk the (same)
+// sum, and each then owns one coefficient, two rows of nine candidates in
+// flight; the probabilities stay in shared memory between the two parts.  As two
+// kernels of a warp a block and a thread a coefficient, with one load of a chain
+// in flight, 16.7 + 18.4 us a band for one CIF frame; now 22.7 (eight lanes a
+// block and a coefficient pair each: 28.7).  A lone CIF frame 5.52 -> 5.40 ms,
+// eleven at QIndex 8 67.2 -> 66.3, one QCIF frame 2.51 -> 2.48.
+__global__ void __launch_bounds__(128) update_ml_kernel(FrameDev *frames, XlmDev xt, int band) {
+  __shared__ float s_p[8][ML_N];  // ML_N is odd: the two blocks of a warp read two banks
   FrameDev &F = frames[blockIdx.y];
   if (!F.active || !in_step(F, band, 0)) return;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (warp >= F.nsir) return;
-  const int w = F.w, h = F.h, b4w = w / 4;
-  const int blk = F.sir[warp];
-  const int top = (blk / b4w) << 2, left = (blk % b4w) << 2;
-  const Win wn = ml_window(top, left, w, h);
-  const int cw = wn.sr - wn.sl + 1, nc = cw * (wn.sb - wn.st + 1);
-  const XlSmall xs = xl_small_global(xt);
-  float *p = F.smf + (size_t)warp * ML_N;
-  uint32_t cb[4];
-#pragma unroll
-  for (int ii = 0; ii < 4; ii++) cb[ii] = load4_u8(F.recon + (size_t)(top + ii) * w + left);
-  float pr[3];
-  for (int r = 0; r < 3; r++) {
-    const int q = lane + 32 * r;
-    pr[r] = 0.0f;
-    if (q < nc) {
-      const int m = wn.st + q / cw, n = wn.sl + q % cw;
-      uint32_t sse = 0;
-#pragma unroll
-      for (int ii = 0; ii < 4; ii++) {
-        const uint32_t d = __vabsdiffu4(cb[ii], load4_u8(F.si + (size_t)(m + ii) * w + n));
-        sse = __dp4a(d, d, sse);
-      }
-      pr[r] = xl_expf(xt, xs, (float)-0.01f * (float)sse);
-    }
-  }
-  // sequential sum in candidate order
-  float sum = 0.0f;
-  for (int q = 0; q < nc; q++) {
-    const float v = __shfl_sync(0xffffffffu, pr[q >> 5], q & 31);
-    sum += v;
-  }
-  int center = 0;
-  {
-    const int cm = top - wn.st, cn = left - wn.sl;
-    center = cm * cw + cn;
-  }
-  for (int r = 0; r < 3; r++) {
-    const int q = lane + 32 * r;
-    if (q < nc) p[q] = sum > 0.0 ? pr[r] / sum : (q == center ? 1.0f : pr[r]);
-  }
-}
-
-// update_si_ML, motionLearning.cpp:129-160: ML side coefficients of bands >= first_band
-__global__ void update_ml_kernel(FrameDev *frames, int band) {
-  FrameDev &F = frames[blockIdx.y];
-  if (!F.active || !in_step(F, band, 0)) return;
-  const int first_band = band + 1;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int s_idx = t >> 4, c = t & 15;
-  if (s_idx >= F.nsir || c < first_band) return;
+  const int lane = threadIdx.x & 15;
+  const int s_idx = (blockIdx.x * blockDim.x + threadIdx.x) >> 4;
+  const bool live = s_idx < F.nsir;
   const int w = F.w, h = F.h, b4w = w / 4, srw = w - 3;
-  const int index = c_zigzag[c];
-  const int blk = F.sir[s_idx];
+  const int blk = live ? F.sir[s_idx] : 0;
   const int top = (blk / b4w) << 2, left = (blk % b4w) << 2;
   const Win wn = ml_window(top, left, w, h);
-  const float *p = F.smf + (size_t)s_idx * ML_N;
-  float acc = 0.0f;
-  int q = 0;
-  for (int m = wn.st; m <= wn.sb; m++)
-    for (int n = wn.sl; n <= wn.sr; n++) {
-      acc += p[q] * (float)(F.oct[((size_t)m * srw + n) * 16 + index]);
-      q++;
+  const int cw = wn.sr - wn.sl + 1, nc = live ? cw * (wn.sb - wn.st + 1) : 0;
+  const XlSmall xs = xl_small_global(xt);
+  float *pr = s_p[threadIdx.x >> 4];
+  if (live) {
+    uint32_t cb[4];
+#pragma unroll
+    for (int ii = 0; ii < 4; ii++) cb[ii] = load4_u8(F.recon + (size_t)(top + ii) * w + left);
+    // three rounds of loads in flight; past the last candidate it is read again
+    const int inv = 65536 / cw + 1;  // q / cw for q < 81, cw < 10
+    for (int q0 = lane; q0 < nc; q0 += 48) {
+      uint32_t sse[3] = {0, 0, 0};
+#pragma unroll
+      for (int r = 0; r < 3; r++) {
+        const int q = min(q0 + 16 * r, nc - 1), qm = (q * inv) >> 16;
+        const uint8_t *c = F.si + (size_t)(wn.st + qm) * w + wn.sl + q - qm * cw;
+#pragma unroll
+        for (int ii = 0; ii < 4; ii++) {
+          const uint32_t d = __vabsdiffu4(cb[ii], load4_u8(c + (size_t)ii * w));
+          sse[r] = __dp4a(d, d, sse[r]);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 3; r++) {
+        const float e = xl_expf(xt, xs, (float)-0.01f * (float)sse[r]);
+        if (q0 + 16 * r < nc) pr[q0 + 16 * r] = e;
+      }
     }
-  F.side_trans[(top + (index >> 2)) * w + left + (index & 3)] = (int)acc;
+  }
+  __syncwarp();
+  float sum = 0.0f;
+#pragma unroll 9
+  for (int q = 0; q < nc; q++) sum += pr[q];
+  __syncwarp();
+  if (live) {
+    const int center = (top - wn.st) * cw + left - wn.sl;
+    float *p = F.smf + (size_t)s_idx * ML_N;
+#pragma unroll 3
+    for (int q = lane; q < nc; q += 16) {
+      const float v = sum > 0.0 ? pr[q] / sum : (q == center ? 1.0f : pr[q]);
+      pr[q] = v;
+      p[q] = v;
+    }
+  }
+  __syncwarp();
+  bool want = false;  // the lane's raster position belongs to a band above `band`
+  for (int c = band + 1; c < 16; c++) want |= c_zigzag[c] == lane;
+  if (!live || !want) return;
+  float acc = 0.0f;
+  const int16_t *o = F.oct + lane;
+#pragma unroll 2
+  for (int m = wn.st; m <= wn.sb; m++, pr += cw) {
+    const int16_t *row = o + ((size_t)m * srw + wn.sl) * 16;
+    int v[2 * LEARN_R + 1];
+#pragma unroll
+    for (int j = 0; j <= 2 * LEARN_R; j++) v[j] = j < cw ? row[j * 16] : 0;
+#pragma unroll
+    for (int j = 0; j <= 2 * LEARN_R; j++)
+      if (j < cw) acc += pr[j] * (float)v[j];
+  }
+  F.side_trans[(top + (lane >> 2)) * w + left + (lane & 3)] = (int)acc;
 }
 
 // ------------------------------------------------------------- launchers
@@ -1804,8 +1817,7 @@ cudaError_t launch_band_end(FrameDev *fr, int nf, int w, int h, int max_nsir, in
   const cudaError_t e = g_si_threads == 256 ? launch_update_si<256>(fr, tiles, band, s) : launch_update_si<512>(fr, tiles, band, s);
   if (e != cudaSuccess) return e;
   over_complete_kernel<<<dim3((w - 3 + 127) / 128, nf, h - 3), 128, 0, s>>>(fr, band);
-  update_smf_kernel<<<g2(max_nsir * 32, 128, nf), 128, 0, s>>>(fr, xt, band);
-  update_ml_kernel<<<g2(max_nsir * 16, 128, nf), 128, 0, s>>>(fr, band);
+  update_ml_kernel<<<g2(max_nsir * 16, 128, nf), 128, 0, s>>>(fr, xt, band);
   return cudaGetLastError();
 }
 

@@ -12,7 +12,10 @@ pytestmark = pytest.mark.gpu
 def _map(kind, hb, wb):
     """8x8 blocks that stay Wyner-Ziv coded."""
     wz = np.zeros((hb, wb), bool)
-    if kind == "corners":
+    if kind.startswith("block "):  # the motion learning's smallest launches, windows of 25 to 81 candidates
+        for b in kind.split()[1:]:
+            wz.reshape(-1)[int(b)] = True
+    elif kind == "corners":
         wz[0, 0] = wz[0, -1] = wz[-1, 0] = wz[-1, -1] = True
     elif kind == "one per tile":
         wz[::2, 1::2] = True
@@ -24,6 +27,15 @@ def _map(kind, hb, wb):
 @pytest.mark.parametrize("threads", ["256", "512"])
 @pytest.mark.parametrize("kind", ["corners", "one per tile", "scattered"])
 def test_sparse_tiles_match_the_oracle(kind, threads, monkeypatch):
+    _compare(kind, threads, monkeypatch)
+
+
+@pytest.mark.parametrize("kind", ["block 0", "block 395", "block 21 22 200"])
+def test_a_few_blocks_match_the_oracle(kind, monkeypatch):
+    _compare(kind, "256", monkeypatch)
+
+
+def _compare(kind, threads, monkeypatch):
     from dvc_b200 import bitstream as bs, decoder, encoder, native, synth
     from oracle import pyoracle as po
     monkeypatch.setenv("DVC_SI_THREADS", threads)
