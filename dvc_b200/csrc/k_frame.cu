@@ -974,103 +974,94 @@ __global__ void __launch_bounds__(NT) noise_dist_kernel(FrameDev *frames, XlmDev
   }
 }
 
-// p[lo0..hi0) and p[lo1..hi1), each summed in ascending order (the float sums
-// of condBitProb).  Each lane walks its own row, so the reads wait on memory:
-// once aligned they are 16 bytes each, and up to four of either chain are in
-// flight before their additions (one of either: 20 us for a lone CIF frame).
-__device__ __forceinline__ void interval_sums(const float *p, int lo0, int hi0, int lo1, int hi1, float &s0,
-                                              float &s1) {
-  float a = 0.0f, b = 0.0f;
-  int q0 = lo0, q1 = lo1;
-  for (; q0 < hi0 && (reinterpret_cast<uintptr_t>(p + q0) & 15); q0++) a += __ldg(p + q0);
-  for (; q1 < hi1 && (reinterpret_cast<uintptr_t>(p + q1) & 15); q1++) b += __ldg(p + q1);
-  auto add4 = [](float &s, const float4 &v) {
-    s += v.x;
-    s += v.y;
-    s += v.z;
-    s += v.w;
-  };
-  constexpr int U = 4;
-  while (q0 + 4 <= hi0 || q1 + 4 <= hi1) {
-    float4 u[U], v[U];
+// p[lo..hi) summed in ascending order (a float sum of condBitProb).  Each lane
+// walks its own row, so the reads wait on memory: once aligned they are 16 bytes
+// each, and up to eight are in flight before their additions.
+__device__ __forceinline__ float interval_sum(const float *p, int lo, int hi) {
+  float a = 0.0f;
+  int q = lo;
+  for (; q < hi && (reinterpret_cast<uintptr_t>(p + q) & 15); q++) a += __ldg(p + q);
+  constexpr int U = 8;
+  for (; q + 4 <= hi; q = min(q + 4 * U, q + ((hi - q) & ~3))) {
+    float4 u[U];
+    // past the last whole quad +0 is added to a sum that is not negative
+#pragma unroll
+    for (int i = 0; i < U; i++)
+      u[i] = q + 4 * i + 4 <= hi ? __ldg(reinterpret_cast<const float4 *>(p + q) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int i = 0; i < U; i++) {
-      // a chain past its last whole quad adds +0 to a sum that is not negative
-      u[i] = q0 + 4 * i + 4 <= hi0 ? __ldg(reinterpret_cast<const float4 *>(p + q0) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-      v[i] = q1 + 4 * i + 4 <= hi1 ? __ldg(reinterpret_cast<const float4 *>(p + q1) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      a += u[i].x;
+      a += u[i].y;
+      a += u[i].z;
+      a += u[i].w;
     }
-#pragma unroll
-    for (int i = 0; i < U; i++) {
-      add4(a, u[i]);
-      add4(b, v[i]);
-    }
-    q0 = max(q0, min(q0 + 4 * U, q0 + ((hi0 - q0) & ~3)));
-    q1 = max(q1, min(q1 + 4 * U, q1 + ((hi1 - q1) & ~3)));
   }
-  for (; q0 < hi0; q0++) a += __ldg(p + q0);
-  for (; q1 < hi1; q1++) b += __ldg(p + q1);
-  s0 = a;
-  s1 = b;
+  for (; q < hi; q++) a += __ldg(p + q);
+  return a;
 }
 
 // condBitProb, noiseModel.cpp:191-310: LR = p0/p1 from sequential interval
-// sums of the pdf, one thread per 4x4 block.  Non-WZ blocks get the
-// reference's certain-zero ratio when the frame has skip or intra blocks.
-// Beside each ratio go its logarithm and its term of the entropy bound, which
-// every speculative block of the ladder would otherwise compute again.
-__global__ void cond_bit_kernel(FrameDev *frames, XlmDev xt, int band, int bit) {
+// sums of the pdf.  Non-WZ blocks get the reference's certain-zero ratio when
+// the frame has skip or intra blocks.  Beside each ratio go its logarithm and
+// its term of the entropy bound, which every speculative block of the ladder
+// would otherwise compute again.  The two sums are latency-bound chains, so two
+// lanes take a 4x4 block: the even one sums p0 and writes the ratio and its
+// logarithm, the odd one sums p1 and writes the entropy term.  Blocks of 64
+// threads, so that the rows of one CIF frame (6336) spread over all SMs.
+// With a thread for both sums, four quads of each in flight, and blocks of 128
+// threads (50 of 148 SMs for a lone CIF frame) 20.7 us a step, now 18.2; sixteen
+// CIF frames 26.2 -> 20.5.  One QCIF frame 2.46 -> 2.40 ms, one CIF frame 5.40 ->
+// 5.31, eleven at QIndex 8 66.2 -> 65.6.
+__global__ void __launch_bounds__(64) cond_bit_kernel(FrameDev *frames, XlmDev xt, int band, int bit) {
   FrameDev &F = frames[blockIdx.y];
   if (!F.active || !in_step(F, band, bit)) return;
   const int w = F.w, b4w = w / 4, b4n = b4w * (F.h / 4);
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, k = t >> 1, odd = t & 1;
+  const int s_idx = k < b4n ? F.sir_of_blk[k] : -1;
+  float sum = 0.0f;
+  if (s_idx >= 0) {
+    const int index = c_zigzag[band], step = F.step[index], range = F.crange[index];
+    const int i = k / b4w, j = k % b4w;
+    const int rc = F.recons_trans[(4 * i + (index >> 2)) * w + 4 * j + (index & 3)];
+    const float *p = F.pdf + (size_t)s_idx * F.pdf_stride;
+    const int iq = (1 << (bit - 1)) - 1;
+    // interval ends are clamped to the pdf row; consistent bitstreams never reach the clamp
+    if (index == 0) {
+      const int bl = odd ? ((rc << 1) + 1) << (bit - 1) : rc << bit, bu = bl + iq;
+      sum = interval_sum(p, max(bl * step, 0), min((bu + 1) * step, range));
+    } else {
+      const int ls = F.level_shift[index];
+      const int bl = (odd ? ((rc << 1) + 1) << (bit - 1) : rc << bit) - ls;
+      int bu = bl + iq;
+      if (odd && bu > ls) bu = ls;
+      const int vl = (bl <= 0) ? (bl - 1) * step + 1 : bl * step;
+      const int vu = ((bu < 0) ? bu * step + 1 : (bu + 1) * step) + range;
+      sum = interval_sum(p, max(vl + range, 0), min(vu, 2 * range + 1));
+    }
+  }
+  const float other = __shfl_xor_sync(0xffffffffu, sum, 1);
   if (k >= b4n) return;
   const XlSmall xs = xl_small_global(xt);
-  const int s_idx = F.sir_of_blk[k];
-  if (s_idx < 0) {
-    if (F.skip_mode == 1 || F.intra_mode == 1) F.lr[k] = 0.9999f / 0.0001f;
-    const float lr = F.lr[k];
-    F.llr[k] = xl_logf(xt, xs, lr);
-    F.term[k] = ld_entropy_term(lr, xt, xs);
-    return;
-  }
-  const int index = c_zigzag[band], step = F.step[index], range = F.crange[index];
-  const int i = k / b4w, j = k % b4w;
-  const int rc = F.recons_trans[(4 * i + (index >> 2)) * w + 4 * j + (index & 3)];
-  const float *p = F.pdf + (size_t)s_idx * F.pdf_stride;
-  const int iq = (1 << (bit - 1)) - 1;
-  float p0 = 0.0f, p1 = 0.0f;
-  // interval ends are clamped to the pdf row; consistent bitstreams never reach the clamp
-  if (index == 0) {
-    const int b0l = rc << bit, b1l = ((rc << 1) + 1) << (bit - 1);
-    const int b0u = b0l + iq, b1u = b1l + iq;
-    const int v0l = b0l * step, v1l = b1l * step, v0u = (b0u + 1) * step, v1u = (b1u + 1) * step;
-    interval_sums(p, max(v0l, 0), min(v0u, range), max(v1l, 0), min(v1u, range), p0, p1);
-  } else {
-    const int ls = F.level_shift[index];
-    const int b0l = (rc << bit) - ls;
-    const int b1l = (((rc << 1) + 1) << (bit - 1)) - ls;
-    const int b0u = b0l + iq;
-    int b1u = b1l + iq;
-    if (b1u > ls) b1u = ls;
-    const int v0l = (b0l <= 0) ? (b0l - 1) * step + 1 : b0l * step;
-    const int v1l = (b1l <= 0) ? (b1l - 1) * step + 1 : b1l * step;
-    const int v0u = ((b0u < 0) ? b0u * step + 1 : (b0u + 1) * step) + range;
-    const int v1u = ((b1u < 0) ? b1u * step + 1 : (b1u + 1) * step) + range;
-    const int len = 2 * range + 1;
-    interval_sums(p, max(v0l + range, 0), min(v0u, len), max(v1l + range, 0), min(v1u, len), p0, p1);
-  }
-  p0 = p0 / (p0 + p1);
-  p1 = 1 - p0;
   float lr;
-  if (p0 <= 0.0001)
-    lr = (float)(0.0001 / 0.9999);
-  else if (p0 >= 0.9999)
-    lr = (float)(0.9999 / 0.0001);
-  else
-    lr = p0 / p1;
-  F.lr[k] = lr;
-  F.llr[k] = xl_logf(xt, xs, lr);
-  F.term[k] = ld_entropy_term(lr, xt, xs);
+  if (s_idx < 0) {
+    lr = F.skip_mode == 1 || F.intra_mode == 1 ? 0.9999f / 0.0001f : F.lr[k];
+  } else {
+    float p0 = odd ? other : sum, p1 = odd ? sum : other;
+    p0 = p0 / (p0 + p1);
+    p1 = 1 - p0;
+    if (p0 <= 0.0001)
+      lr = (float)(0.0001 / 0.9999);
+    else if (p0 >= 0.9999)
+      lr = (float)(0.9999 / 0.0001);
+    else
+      lr = p0 / p1;
+  }
+  if (odd) {
+    F.term[k] = ld_entropy_term(lr, xt, xs);
+  } else {
+    F.lr[k] = lr;
+    F.llr[k] = xl_logf(xt, xs, lr);
+  }
 }
 
 // ------------------------------------------------------- reconstruction
@@ -1788,7 +1779,7 @@ cudaError_t launch_noise_dist(FrameDev *fr, int nf, int max_nsir, const XlmDev &
 }
 
 cudaError_t launch_cond_bit(FrameDev *fr, int nf, int w, int h, const XlmDev &xt, int band, int bit, cudaStream_t s) {
-  cond_bit_kernel<<<g2((w / 4) * (h / 4), 128, nf), 128, 0, s>>>(fr, xt, band, bit);
+  cond_bit_kernel<<<g2((w / 4) * (h / 4) * 2, 64, nf), 64, 0, s>>>(fr, xt, band, bit);
   return cudaGetLastError();
 }
 
