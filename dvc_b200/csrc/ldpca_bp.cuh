@@ -36,7 +36,12 @@
 // What bounds it: each magnitude phi(y) = -logf(tanhf(y)) is one 16-byte record
 // gathered from the packed table (dvc_common.cuh), two per edge and iteration,
 // and an SM takes one random 32-byte sector per cycle from L2 (measured: 1.0
-// cycle per gather for tables up to 64 MB): 38,016 cycles for a CIF codeword.
+// cycle per gather for hot tables up to 64 MB and at least about 90 KB of L1,
+// half that rate with a small L1): 38,016 cycles for a CIF codeword.  An
+// iteration takes 46.9 K (41 K in the edge pass, 5.4 K in the row pass); three
+// passes with separate sign and decision bytes took 65 K, this form with a
+// 72 MB hot table (36 MB now) 50.7 K.  Two columns of a thread in flight at once
+// change nothing at 1024 threads, three at 704 threads take 54 K.
 // Rows are stored transposed in groups of 32 of similar degree (LadderDev), so
 // the row pass reads without bank conflicts and spends its time on the sums.
 //
