@@ -652,9 +652,9 @@ def main():
                                               "the path is bound by its gathers and compute, not by moving "
                                               "these bytes"},
                          "note": "4-byte phi values gathered at random, one 16-byte record each through the "
-                                 "texture path, from a packed 166 MB table whose hot part mostly stays in L2 (84% "
-                                 "L2 hits, ~125 KB of DRAM traffic per block-iteration in ncu); the kernel is bound "
-                                 "by the latency of those gathers, not by DRAM bandwidth.  Launches of 16 streams "
+                                 "texture path, from a packed 101 MB table whose hot 36 MB stay in L2 (2 KB of "
+                                 "DRAM traffic per block-iteration in ncu); the kernel is bound by the rate of those "
+                                 "gathers (one per cycle and SM), not by DRAM bandwidth.  Launches of 16 streams "
                                  "overlap, so the per-launch figure understates the device-wide rate "
                                  "(aggregate_achieved: all launches of a step over the step time)"},
             "cpu_baseline": cpu,

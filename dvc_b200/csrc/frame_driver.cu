@@ -464,8 +464,8 @@ long long FrameBatcher::launches_per_execute() const {
     long long bands = 0;
     for (size_t i = 0; i < G.steps.size(); i++)
       if (i == 0 || G.steps[i].band != G.steps[i - 1].band) bands++;
-    // side info 8, prep 6, per band 1 + 5, per step condBitProb + ladder, final 1, deblocking 5
-    total += 8 + 6 + bands * 6 + (long long)G.steps.size() * 2 + 1 + (G.deblock ? 5 : 0);
+    // side info 8, prep 6, per band 1 + 4, per step condBitProb + ladder, final 1, deblocking 5
+    total += 8 + 6 + bands * 5 + (long long)G.steps.size() * 2 + 1 + (G.deblock ? 5 : 0);
   }
   return total;
 }
