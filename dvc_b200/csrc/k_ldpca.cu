@@ -32,7 +32,6 @@
 #include <stdlib.h>
 
 #include <algorithm>
-#include <atomic>
 
 #include "dvc_common.cuh"
 #include "dvc_types.h"
@@ -238,25 +237,10 @@ static cudaError_t launch_nt(const LadderDev &L, const LdpcaJob *jobs, int num_j
   if (L.n > LDPCA_MAX_N || LDPCA_COLS(L.n, NT * C) > MAXC) return cudaErrorInvalidValue;
   auto kernel = ldpca_ladder_kernel<NT, MAXC, MINB, C>;
   const size_t smem = ldpca_smem_bytes(L.n, L.pos_max);
-  // the attributes are per device: set them once for each device
-  static std::atomic<uint64_t> attr_set{0};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
+  // the rest of the SM's 256 KB is L1 for the phi records, which BP iterations re-read
+  static SmemLimit limit;
+  const cudaError_t e = limit.raise(kernel, smem, MINB);
   if (e != cudaSuccess) return e;
-  const uint64_t bit = 1ull << (dev & 63);
-  if (!(attr_set.load() & bit)) {
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    // the smallest shared-memory split that holds the blocks an SM runs (MINB
-    // of them), so that the rest of the SM's 256 KB is L1 for the
-    // phi records, which BP iterations re-read (percent of the 228 KB maximum;
-    // the driver rounds up to a supported split)
-    const size_t need = (size_t)MINB * (smem + 12 * 1024);  // with the descriptors and the block's own
-    const int pct = (int)((need * 100 + 228 * 1024 - 1) / (228 * 1024));
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct > 100 ? 100 : pct);
-    if (e != cudaSuccess) return e;
-    attr_set.fetch_or(bit);
-  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(num_jobs * K * C);
   cfg.blockDim = dim3(NT);

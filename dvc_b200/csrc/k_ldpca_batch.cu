@@ -28,8 +28,6 @@
 // decodes the accepted code again (BP is deterministic).
 #include <cuda_runtime.h>
 
-#include <atomic>
-
 #include "dvc_common.cuh"
 #include "dvc_types.h"
 #include "kernels.h"
@@ -285,19 +283,9 @@ static size_t batch_smem_bytes(const LdpcaBatch &A) {
 cudaError_t launch_ldpca_batch(LdpcaBatch A, int count, int grid, cudaStream_t s) {
   if (A.L_cif.n != 6336 || A.L_qcif.n != 1584) return cudaErrorInvalidValue;
   const size_t smem = batch_smem_bytes(A);
-  static std::atomic<uint64_t> attr_set{0};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
+  static SmemLimit limit;
+  cudaError_t e = limit.raise(ldpca_batch_kernel, smem, 1);
   if (e != cudaSuccess) return e;
-  const uint64_t bit = 1ull << (dev & 63);
-  if (!(attr_set.load() & bit)) {
-    e = cudaFuncSetAttribute(ldpca_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    const int pct = (int)(((smem + 12 * 1024) * 100 + 228 * 1024 - 1) / (228 * 1024));
-    e = cudaFuncSetAttribute(ldpca_batch_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
-    if (e != cudaSuccess) return e;
-    attr_set.fetch_or(bit);
-  }
   if ((e = cudaMemsetAsync(A.ctr, 0, 2 * sizeof(int), s)) != cudaSuccess) return e;
   if ((e = cudaMemsetAsync(A.work, 0, sizeof(unsigned long long), s)) != cudaSuccess) return e;
   // the entropy terms (n floats), later the full-rate syndrome, its words and the decoded bits

@@ -3,10 +3,44 @@
 #include <cuda_runtime.h>
 #include <stddef.h>
 
+#include <algorithm>
+#include <atomic>
+#include <mutex>
+
 #include "dvc_types.h"
 #include "libm_tables.h"
 
 namespace dvc {
+
+// A kernel's dynamic shared memory limit and preferred carveout, set per device
+// and raised when a launch needs more than every one before it: what a ladder
+// kernel needs depends on the ladder file of the context (the padding of its
+// rows), and a process may hold contexts on several.
+struct SmemLimit {
+  std::mutex mu;
+  std::atomic<size_t> most[64] = {};
+  // for the current device; blocks: those of `smem` dynamic bytes, and 12 KB of
+  // its own, that an SM is to hold (the carveout is the smallest split that
+  // does, so that the rest is L1; percent of the 228 KB maximum, the driver
+  // rounds up to a supported split)
+  template <class Kernel>
+  cudaError_t raise(Kernel kernel, size_t smem, int blocks) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::atomic<size_t> &m = most[dev & 63];
+    if (smem <= m.load()) return cudaSuccess;
+    std::lock_guard<std::mutex> lk(mu);
+    if (smem <= m.load()) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    const size_t need = (size_t)blocks * (smem + 12 * 1024);
+    const int pct = (int)std::min<size_t>(100, (need * 100 + 228 * 1024 - 1) / (228 * 1024));
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
+    if (e == cudaSuccess) m.store(smem);
+    return e;
+  }
+};
 
 // direct form: one block per codeword, no scratch
 cudaError_t launch_ldpca(const LadderDev &L, const LdpcaJob *jobs_dev, int num_jobs, const XlmDev &xt,

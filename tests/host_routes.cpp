@@ -1,0 +1,245 @@
+// Test driver: the library's host code (dispatch, buffers, streams) linked with
+// a CUDA runtime that runs no kernel.  Device memory is host memory, a launch is
+// checked as the runtime checks it (a function's dynamic shared memory against
+// the attribute set for it) and written down, and allocations can be made to
+// fail by size.  tests/test_host_routes.py builds it from the library's object
+// files and reads what it prints.  The C-library table sweeps are left out (the
+// kernels that read the tables do not run).
+#include <cuda_runtime.h>
+
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <map>
+#include <string>
+#include <vector>
+
+#include "dvc_b200.h"
+#include "libm_tables.h"
+
+// ------------------------------------------------------------ the runtime
+namespace {
+std::map<const void *, std::string> g_name;   // host stub -> kernel
+std::map<const void *, size_t> g_smem;        // largest dynamic shared memory allowed
+std::map<void *, size_t> g_mem;               // device allocations
+size_t g_live = 0, g_fail_from = ~(size_t)0;  // bytes held; allocations of this size and more fail
+int g_streams = 0, g_events = 0;              // alive
+bool g_record = false;
+
+cudaError_t take(void **p, size_t bytes) {
+  *p = nullptr;
+  if (bytes >= g_fail_from || bytes > ((size_t)1 << 36)) return cudaErrorMemoryAllocation;
+  *p = aligned_alloc(256, (bytes + 255) & ~(size_t)255);
+  memset(*p, 0, bytes);
+  g_mem[*p] = bytes;
+  g_live += bytes;
+  return cudaSuccess;
+}
+cudaError_t give(void *p) {
+  if (!p) return cudaSuccess;
+  auto it = g_mem.find(p);
+  if (it == g_mem.end()) return cudaErrorInvalidValue;
+  g_live -= it->second;
+  g_mem.erase(it);
+  free(p);
+  return cudaSuccess;
+}
+cudaError_t launch(const void *f, dim3 grid, dim3 block, unsigned cluster, size_t smem) {
+  const size_t most = g_smem.count(f) ? g_smem[f] : 48 * 1024;
+  const bool bad = smem > most || grid.x % cluster != 0 || block.x > 1024;
+  if (g_record)
+    printf("launch %s grid %u block %u cluster %u smem %zu%s\n", g_name[f].c_str(), grid.x, block.x, cluster, smem,
+           bad ? " refused" : "");
+  return bad ? cudaErrorInvalidValue : cudaSuccess;
+}
+struct {
+  dim3 grid, block;
+  size_t smem;
+  cudaStream_t stream;
+} g_call;
+}  // namespace
+
+extern "C" {
+void **__cudaRegisterFatBinary(void *) { return (void **)&g_call; }
+void __cudaRegisterFatBinaryEnd(void **) {}
+void __cudaUnregisterFatBinary(void **) {}
+void __cudaRegisterFunction(void **, const char *host, char *, const char *name, int, uint3 *, uint3 *, dim3 *, dim3 *,
+                            int *) {
+  g_name[host] = name;
+}
+void __cudaRegisterVar(void **, char *, char *, const char *, int, size_t, int, int) {}
+unsigned __cudaPushCallConfiguration(dim3 g, dim3 b, size_t s, cudaStream_t st) {
+  g_call = {g, b, s, st};
+  return 0;
+}
+cudaError_t __cudaPopCallConfiguration(dim3 *g, dim3 *b, size_t *s, void *st) {
+  *g = g_call.grid;
+  *b = g_call.block;
+  *s = g_call.smem;
+  *(cudaStream_t *)st = g_call.stream;
+  return cudaSuccess;
+}
+cudaError_t cudaLaunchKernel(const void *f, dim3 g, dim3 b, void **, size_t smem, cudaStream_t) {
+  return launch(f, g, b, 1, smem);
+}
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void **) {
+  unsigned cluster = 1;
+  for (unsigned i = 0; i < c->numAttrs; i++)
+    if (c->attrs[i].id == cudaLaunchAttributeClusterDimension) cluster = c->attrs[i].val.clusterDim.x;
+  return launch(f, c->gridDim, c->blockDim, cluster, c->dynamicSmemBytes);
+}
+cudaError_t cudaFuncSetAttribute(const void *f, cudaFuncAttribute a, int v) {
+  if (a == cudaFuncAttributeMaxDynamicSharedMemorySize) {
+    if (v > 227 * 1024) return cudaErrorInvalidValue;
+    g_smem[f] = (size_t)v;
+  }
+  return cudaSuccess;
+}
+cudaError_t cudaMalloc(void **p, size_t n) { return take(p, n); }
+cudaError_t cudaMallocAsync(void **p, size_t n, cudaStream_t) { return take(p, n); }
+cudaError_t cudaFree(void *p) { return give(p); }
+cudaError_t cudaFreeAsync(void *p, cudaStream_t) { return give(p); }
+cudaError_t cudaMallocHost(void **p, size_t n) { return (*p = calloc(n, 1)) ? cudaSuccess : cudaErrorMemoryAllocation; }
+cudaError_t cudaFreeHost(void *p) {
+  free(p);
+  return cudaSuccess;
+}
+cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) {
+  memcpy(d, s, n);
+  return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t) {
+  memcpy(d, s, n);
+  return cudaSuccess;
+}
+cudaError_t cudaMemset(void *p, int v, size_t n) {
+  memset(p, v, n);
+  return cudaSuccess;
+}
+cudaError_t cudaMemsetAsync(void *p, int v, size_t n, cudaStream_t) { return cudaMemset(p, v, n); }
+cudaError_t cudaMemcpyToSymbol(const void *, const void *, size_t, size_t, cudaMemcpyKind) { return cudaSuccess; }
+cudaError_t cudaGetSymbolAddress(void **p, const void *) {
+  static char room[1 << 20];
+  *p = room;
+  return cudaSuccess;
+}
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) {
+  *s = (cudaStream_t) new int(0);
+  g_streams++;
+  return cudaSuccess;
+}
+cudaError_t cudaStreamDestroy(cudaStream_t s) {
+  delete (int *)s;
+  g_streams--;
+  return cudaSuccess;
+}
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) {
+  *e = (cudaEvent_t) new int(0);
+  g_events++;
+  return cudaSuccess;
+}
+cudaError_t cudaEventCreate(cudaEvent_t *e) { return cudaEventCreateWithFlags(e, 0); }
+cudaError_t cudaEventDestroy(cudaEvent_t e) {
+  delete (int *)e;
+  g_events--;
+  return cudaSuccess;
+}
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventQuery(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) {
+  *ms = 1.0f;
+  return cudaSuccess;
+}
+cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaErrorNotSupported; }
+cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t *) { return cudaErrorNotSupported; }
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t *, cudaGraph_t, unsigned long long) { return cudaErrorNotSupported; }
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaErrorNotSupported; }
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
+cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
+cudaError_t cudaGetDevice(int *d) {
+  *d = 0;
+  return cudaSuccess;
+}
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr a, int) {
+  *v = a == cudaDevAttrMultiProcessorCount ? 148 : 1 << 27;
+  return cudaSuccess;
+}
+cudaError_t cudaDeviceSetLimit(cudaLimit, size_t) { return cudaSuccess; }
+cudaError_t cudaDeviceGetDefaultMemPool(cudaMemPool_t *p, int) {
+  *p = nullptr;
+  return cudaSuccess;
+}
+cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void *) { return cudaSuccess; }
+cudaError_t cudaCreateTextureObject(cudaTextureObject_t *t, const cudaResourceDesc *, const cudaTextureDesc *,
+                                    const cudaResourceViewDesc *) {
+  *t = 1;
+  return cudaSuccess;
+}
+cudaError_t cudaDestroyTextureObject(cudaTextureObject_t) { return cudaSuccess; }
+cudaChannelFormatDesc cudaCreateChannelDesc(int x, int y, int z, int w, cudaChannelFormatKind f) {
+  return {x, y, z, w, f};
+}
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+const char *cudaGetErrorString(cudaError_t e) { return e == cudaErrorMemoryAllocation ? "out of memory" : "CUDA error"; }
+
+int dvc_libm_build(const char *, int, char *, int) { return 0; }
+}
+
+int dvc_libm_load(const char *, XlmHost *out, char *, int) {
+  out->log_tab.assign(4, 0);
+  out->exp_tab.assign(4, 0);
+  memset(&out->hdr, 0, sizeof out->hdr);
+  out->hdr.log_cap = out->hdr.exp_cap = 2;
+  out->hdr.tanh_y1 = 16;
+  return 0;
+}
+void dvc_phi_build(float *, uint32_t, uint32_t, int) {}
+bool dvc_phi_pack(const float *, uint32_t, uint32_t, int, PhiPacked &out, char *, int) {
+  out.desc.assign(4, 0);
+  out.rec.assign(4, 0);
+  return true;
+}
+
+// ---------------------------------------------------------------- the modes
+static dvc_ctx *context(const char *data, const char *tables) {
+  dvc_ctx *c = nullptr;
+  const int rc = dvc_create(data, tables, 0, &c);
+  if (rc != DVC_OK) {
+    printf("create %d %s\n", rc, dvc_last_error(c));
+    exit(0);
+  }
+  return c;
+}
+
+// one dvc_ldpca_decode of `count` codewords of zeros
+static int decode_zeros(dvc_ctx *c, int n, int count) {
+  std::vector<float> lr((size_t)count * n, 1.0f), ent(count);
+  std::vector<uint8_t> acc((size_t)count * n / 8), crc(count), dec((size_t)count * n);
+  std::vector<int> res((size_t)count * 4);
+  return dvc_ldpca_decode(c, n, count, lr.data(), acc.data(), crc.data(), dec.data(), res.data(), ent.data(), 50);
+}
+
+// files DATA TABLES DATA2: codewords of both lengths and a batch of them with one
+// ladder file after another
+static void files(char **a) {
+  for (const char *data : {a[0], a[2]}) {
+    dvc_ctx *c = context(data, a[1]);
+    g_record = true;
+    for (int n : {1584, 6336})
+      for (int count : {1, 200, 600}) printf("rc %d\n", decode_zeros(c, n, count));
+    g_record = false;
+    dvc_destroy(c);
+  }
+}
+
+int main(int argc, char **argv) {
+  const std::string mode = argc > 1 ? argv[1] : "";
+  if (mode == "files" && argc == 5) files(argv + 2);
+  else return 2;
+  printf("left bytes %zu streams %d events %d\n", g_live, g_streams, g_events);
+  return 0;
+}

@@ -1,0 +1,56 @@
+"""The library's host code on the CPU, linked with a CUDA runtime that runs no
+kernel (tests/host_routes.cpp): which launches a call makes, what it does when
+memory is refused, what it holds and gives back."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+from ladder_files import data_dir, lad
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CUDA = "/usr/local/cuda"
+
+
+@pytest.fixture(scope="module")
+def routes(tmp_path_factory):
+    """run(mode, *args) -> the lines the driver prints; its tables are cached for the module."""
+    gxx = shutil.which("g++")
+    if gxx is None or not os.path.exists(os.path.join(CUDA, "include", "cuda_runtime.h")):
+        pytest.skip("g++ or the CUDA headers not available")
+    from dvc_b200 import build
+    build.build()
+    tmp = tmp_path_factory.mktemp("routes")
+    objs = [os.path.join(build.OBJDIR, os.path.basename(s) + ".o") for s in build.sources()]
+    objs = [o for o in objs if "libm_tables" not in o]  # the driver's own, which sweep nothing
+    out = str(tmp / "host_routes")
+    r = subprocess.run([gxx, "-O1", "-std=c++17", "-w", "-I", os.path.join(CUDA, "include"), "-I",
+                        os.path.join(ROOT, "include"), "-I", build.CSRC, "-o", out,
+                        os.path.join(ROOT, "tests", "host_routes.cpp")] + objs + ["-lpthread"],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-3000:]
+
+    def run(mode, data, *args, env=None):
+        r = subprocess.run([out, mode, str(data), str(tmp)] + [str(a) for a in args], capture_output=True, text=True,
+                           timeout=300, env=dict(os.environ, **(env or {})))
+        assert r.returncode == 0, (r.returncode, r.stdout[-1000:], r.stderr[-1000:])
+        return r.stdout.splitlines()
+
+    run.tmp = tmp
+    return run
+
+
+def launches(lines):
+    return [x.split() for x in lines if x.startswith("launch ")]
+
+
+def test_a_ladder_file_after_one_that_needs_less_memory(routes):
+    """Codes of the same length take more or less shared memory by the degrees of
+    their rows: a second context's launches must not be held to the first's."""
+    shipped = lad.read_compact(os.path.join(ROOT, "dvc_b200", "ladders", "ldpca_ladders.bin"))
+    few = [dict(L, bpp=L["bpp"][-2:], idx=L["idx"][-2:]) for L in shipped]  # the highest codes: rows of equal degree
+    lines = routes("files", data_dir(routes.tmp / "few", few), data_dir(routes.tmp / "all", shipped))
+    smem = [int(x[9]) for x in launches(lines) if "ladder_kernel" in x[1] or "ldpca_batch_kernel" in x[1]]
+    assert len(smem) == 12 and any(b > a for a, b in zip(smem[:6], smem[6:])), lines
+    assert [x for x in lines if x.startswith("rc")] == ["rc 0"] * 12, lines
