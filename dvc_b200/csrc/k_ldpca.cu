@@ -45,7 +45,9 @@ namespace dvc {
 // blocks per SM.  Alone NT = 1024 for both lengths (CIF: one block per SM, 105
 // KB of shared memory; QCIF: 27 KB); QCIF codewords can also run with 256 or
 // 512 threads, four or two blocks per SM (the autotuner measures which is faster).
-template <int NT, int MAXC, int MINB, int C>
+// ANY: a codeword of any length up to NT * MAXC; without it of a length that
+// needs all MAXC rounds, which spares the edge pass a bound.
+template <int NT, int MAXC, int MINB, int C, bool ANY>
 __global__ void __launch_bounds__(NT, MINB)
     ldpca_ladder_kernel(LadderDev L, const LdpcaJob *__restrict__ jobs, XlmDev xt, int max_iter, int K,
                         LdpcaSpec sp) {
@@ -57,7 +59,7 @@ __global__ void __launch_bounds__(NT, MINB)
   const LdpcaJob J = jobs[j];
   if (!J.active) return;
   const bool spec = sp.best != nullptr;
-  using G = LdGroup<NT, true, C>;
+  using G = LdGroup<NT, true, C, ANY>;
   const G g{(int)threadIdx.x, 0, C > 1 ? (int)blockIdx.x - unit * C : 0};
   const int n = L.n, tid = threadIdx.x;
   const bool lead = tid == 0 && g.rank == 0;
@@ -231,11 +233,12 @@ unsigned phi_window_attr(cudaLaunchAttribute &a) {
   return 1;
 }
 
-template <int NT, int MAXC, int MINB, int C = 1>
+template <int NT, int MAXC, int MINB, int C = 1, bool ANY = false>
 static cudaError_t launch_nt(const LadderDev &L, const LdpcaJob *jobs, int num_jobs, const XlmDev &xt, int max_iter,
                              int K, const LdpcaSpec &sp, cudaStream_t stream) {
-  if (L.n > LDPCA_MAX_N || LDPCA_COLS(L.n, NT * C) > MAXC) return cudaErrorInvalidValue;
-  auto kernel = ldpca_ladder_kernel<NT, MAXC, MINB, C>;
+  const int rounds = LDPCA_COLS(L.n, NT * C);
+  if (L.n > LDPCA_MAX_N || (ANY ? rounds > MAXC : rounds != MAXC)) return cudaErrorInvalidValue;
+  auto kernel = ldpca_ladder_kernel<NT, MAXC, MINB, C, ANY>;
   const size_t smem = ldpca_smem_bytes(L.n, L.pos_max);
   // the rest of the SM's 256 KB is L1 for the phi records, which BP iterations re-read
   static SmemLimit limit;
@@ -273,6 +276,7 @@ static cudaError_t launch_shape(const LadderDev &L, const LdpcaJob *jobs_dev, in
     if (g_ldpca_threads_qcif == 512) return launch_nt<512, 4, 2>(L, jobs_dev, num_jobs, xt, max_iter, K, sp, stream);
     return launch_nt<256, 7, 4>(L, jobs_dev, num_jobs, xt, max_iter, K, sp, stream);
   }
+  if (L.n != LDPCA_MAX_N) return launch_nt<1024, 7, 1, 1, true>(L, jobs_dev, num_jobs, xt, max_iter, K, sp, stream);
   if (g_ldpca_threads == 512) return launch_nt<512, 13, 1>(L, jobs_dev, num_jobs, xt, max_iter, K, sp, stream);
   return launch_nt<1024, 7, 1>(L, jobs_dev, num_jobs, xt, max_iter, K, sp, stream);
 }
@@ -298,13 +302,15 @@ cudaError_t launch_ldpca(const LadderDev &L, const LdpcaJob *jobs_dev, int num_j
 // eleven at QIndex 8 80 -> 73 ms at C = 2; six or three slots instead of four:
 // four frames 14.6 or 12.3 ms), and QCIF, which gains less, sixteen (a lone
 // frame 3.45 -> 3.04 ms at C = 4; with eight, the three QCIF streams lose 5%).
+// A codeword of another length (a ladder file may hold any up to LDPCA_MAX_N)
+// keeps one block per slot: the cluster shapes are cut for these two.
 // DVC_LDPCA_SPEC_FLOOR replaces the least number of slots (the autotuner's
 // setting), DVC_LDPCA_SPEC fixes it outright.
 void ldpca_spec_shape(int n, int active, int sms, int &K, int &C) {
   const int N = std::max(1, active);
   const bool small = n < LDPCA_MAX_N;
   const int resident = small ? 16 : 4;
-  C = small ? 4 : 8;
+  C = n == 1584 ? 4 : n == LDPCA_MAX_N ? 8 : 1;
   while (C > 1 && N * C * resident > sms) C /= 2;
   int least = 4;
   if (const char *e = getenv("DVC_LDPCA_SPEC_FLOOR")) least = std::max(1, std::min(32, atoi(e)));

@@ -115,8 +115,9 @@ __device__ __forceinline__ uint32_t ld_edge(const uint32_t *p) {
 // each block); `t` is the thread's index in its block's part.  BLOCK: the group
 // is the whole thread block and synchronises with the block's barrier
 // (__syncthreads); otherwise on the hardware barrier `bar` (1-15), which only
-// its NT threads use.
-template <int NT_, bool BLOCK, int C_ = 1>
+// its NT threads use.  ANY: codewords of any length, whose rounds may be fewer
+// than the caller's loops; otherwise of one that fills them all.
+template <int NT_, bool BLOCK, int C_ = 1, bool ANY_ = false>
 struct LdGroup {
   static constexpr int NT = NT_, C = C_, STRIDE = NT_ * C_;
   static_assert(C_ == 1 || BLOCK, "a cluster group takes whole blocks");
@@ -135,8 +136,10 @@ struct LdGroup {
     return l < share && r < rest ? n - rest + r : n;  // n: none in this round
   }
   __device__ __forceinline__ int colf() const { return C_ == 1 ? t : rank * NT_ + t; }
-  // column of round c > 0
+  // column of round c > 0; with ANY, n past the codeword's rounds (otherwise the
+  // first round's columns would be taken a second time)
   __device__ __forceinline__ int col(int n, int c) const {
+    if (ANY_ && c >= LDPCA_COLS(n, STRIDE)) return n;
     return c == 0 ? col0(n) : colf() + (c - (n % STRIDE != 0)) * STRIDE;
   }
   // barrier over the block's part

@@ -236,9 +236,19 @@ static void files(char **a) {
   }
 }
 
+// decode DATA TABLES n count
+static void decode(char **a) {
+  dvc_ctx *c = context(a[0], a[1]);
+  g_record = true;
+  printf("rc %d\n", decode_zeros(c, atoi(a[2]), atoi(a[3])));
+  g_record = false;
+  dvc_destroy(c);
+}
+
 int main(int argc, char **argv) {
   const std::string mode = argc > 1 ? argv[1] : "";
   if (mode == "files" && argc == 5) files(argv + 2);
+  else if (mode == "decode" && argc == 6) decode(argv + 2);
   else return 2;
   printf("left bytes %zu streams %d events %d\n", g_live, g_streams, g_events);
   return 0;

@@ -7,7 +7,7 @@ import subprocess
 
 import pytest
 
-from ladder_files import data_dir, lad
+from ladder_files import circulant, data_dir, lad
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CUDA = "/usr/local/cuda"
@@ -54,3 +54,14 @@ def test_a_ladder_file_after_one_that_needs_less_memory(routes):
     smem = [int(x[9]) for x in launches(lines) if "ladder_kernel" in x[1] or "ldpca_batch_kernel" in x[1]]
     assert len(smem) == 12 and any(b > a for a, b in zip(smem[:6], smem[6:])), lines
     assert [x for x in lines if x.startswith("rc")] == ["rc 0"] * 12, lines
+
+
+@pytest.mark.parametrize("n,count", [(256, 1), (256, 3), (1024, 40)])
+def test_other_codeword_lengths_reach_the_ladder(routes, n, count):
+    """A ladder file may hold other lengths than the two of the codec's sizes:
+    the cluster shapes, cut for those two, are not for them."""
+    d = data_dir(routes.tmp / ("n%d" % n), [circulant(n, 32, range(4, 33, 4))])
+    lines = routes("decode", d, n, count)
+    assert "rc 0" in lines, lines
+    ladder = [x for x in launches(lines) if "ldpca_ladder_kernel" in x[1]]
+    assert len(ladder) == 1 and ladder[0][7] == "1", lines
