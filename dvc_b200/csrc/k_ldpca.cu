@@ -95,8 +95,10 @@ __global__ void __launch_bounds__(NT, MINB)
   // accumulated syndrome bits (ByteToBit, LdpcaDecoder.cpp:81-107), log LR and
   // the entropy terms (ComputeCE), the bound as a sequential sum in block order
   float llr[MAXC], part = 0.0f;
-  ld_llr(g, n, J.lr, xt, xs, llr, S.msg, (J.llr_out && kk == 0) ? J.llr_out : nullptr, J.llr_in, J.term_in, &part);
+  ld_llr(g, n, J.lr, xt, xs, llr, J.use_given_entropy ? nullptr : S.msg, (J.llr_out && kk == 0) ? J.llr_out : nullptr,
+         J.llr_in, J.term_in, &part);
   ld_stage_acc(g, J.acc, n, S.accs);
+  if (J.use_given_entropy) g.sync_all();  // the staged syndrome; otherwise ld_start_near's barriers
   // The bound itself is only needed where it is reported and when the parallel
   // sum leaves the start code open.
   start = J.use_given_entropy ? ld_start_code(L, J.given_entropy) : ld_start_near(g, L, part, s_ured, &s_ctl);
