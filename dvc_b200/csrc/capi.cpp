@@ -86,7 +86,10 @@ static int ldpca_run(Context &c, int n, int count, const float *lr, const uint8_
   // 9.0; CIF 203 13.4 -> 13.3, 400 24.4 -> 23.3, 592 34.8 -> 33.2.  Against a
   // block per ladder: QCIF 600 13.0 -> 8.9, 2400 39.2 -> 30.8; CIF 600 38.4 ->
   // 34.1, 1000 60.1 -> 56.1.  Without memory for the queue, the forms below.
-  const bool queue = count >= 2 * sms && !given_entropy && !llr_back;
+  // A ladder of more codes than the queue and the slots count (a file may hold
+  // any number) takes a block per codeword, which counts nothing.
+  const bool counted = L->num_codes - 1 <= LDPCA_TRIED;
+  const bool queue = counted && count >= 2 * sms && !given_entropy && !llr_back;
   if (queue) {
     const std::vector<int> ns(count, n);
     st = ldpca_batch_run(c, count, ns.data(), lr, acc, crc, nullptr, decoded, results, entropy, max_iter, nullptr,
@@ -127,7 +130,7 @@ static int ldpca_run(Context &c, int n, int count, const float *lr, const uint8_
   // ones 19.8 -> 13.2 ms.
   int K = 1, C = 1;
   dvc::LdpcaSpec sp;
-  if (count < 2 * sms) {
+  if (counted && count < 2 * sms) {
     dvc::ldpca_spec_shape(n, count, sms, K, C);
     // once for every count (by default fewer than 2 * sms codewords of either length)
     const size_t had = c.ld_spec.bytes;

@@ -55,10 +55,14 @@ struct LdpcaJob {
   int w, index_in_blk;
 };
 
+// codes below full rate that a codeword's iteration counts (LdpcaSpec,
+// LdpcaBatchState) and the queue's masks hold; the shipped ladders have 64
+#define LDPCA_TRIED 64
+
 // Scratch of the speculative ladder form (k_ldpca.cu): per codeword the lowest
 // successful code, summed BP iterations and first code; per (codeword, slot)
 // the code it succeeded with and its decoded bits; when wanted, the BP
-// iterations of every code tried ([64] per codeword, from the first code).
+// iterations of every code tried ([LDPCA_TRIED] per codeword, from the first code).
 struct LdpcaSpec {
   int *best = nullptr, *iters = nullptr, *start = nullptr, *done = nullptr, *slot_code = nullptr;
   int *code_iters = nullptr;
@@ -81,7 +85,7 @@ struct LdpcaBatchState {
   int nsucc;                 // successes so far (each takes the next slot)
   unsigned long long mask;   // bit c - start: code c has finished
   int succ_code[4];          // code that filled each slot
-  int iters[64];             // BP iterations of code start + k
+  int iters[LDPCA_TRIED];    // BP iterations of code start + k
 };
 
 // Arguments of the batched launch (all device pointers).

@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(NT, MINB)
     uint32_t dm = 0;
     const int ok = ld_try_code(g, L, code, llr, J.crc, xt, s_pdesc, max_iter, bestp, S, s_ured, &s_ctl, it, dm);
     total_iters += it;
-    if (spec && sp.code_iters && lead) sp.code_iters[j * 64 + code - start] = it;
+    if (spec && sp.code_iters && lead) sp.code_iters[j * LDPCA_TRIED + code - start] = it;
     if (ok) {
       accepted = code;
       if (spec) {
@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(NT, MINB)
       // accepted one ran to its end), or those of every code tried
       int iters = 0;
       if (sp.code_iters)
-        for (int c = start; c <= min(acc, last - 1); c++) iters += __ldcg(sp.code_iters + j * 64 + c - start);
+        for (int c = start; c <= min(acc, last - 1); c++) iters += __ldcg(sp.code_iters + j * LDPCA_TRIED + c - start);
       else
         iters = __ldcg(sp.iters + j);
       s_iters = iters;
@@ -322,7 +322,8 @@ void ldpca_spec_shape(int n, int active, int sms, int &K, int &C) {
 }
 
 size_t ldpca_spec_scratch_bytes(int n, int num_jobs, int K) {
-  return (size_t)num_jobs * 16 + (size_t)num_jobs * K * 4 + (size_t)num_jobs * K * n + (size_t)num_jobs * 256 + 64;
+  return (size_t)num_jobs * 16 + (size_t)num_jobs * K * 4 + (size_t)num_jobs * K * n +
+         (size_t)num_jobs * LDPCA_TRIED * 4 + 64;
 }
 
 LdpcaSpec ldpca_spec_carve(void *base, int num_jobs, int K, bool code_iters) {
@@ -339,7 +340,7 @@ LdpcaSpec ldpca_spec_carve(void *base, int num_jobs, int K, bool code_iters) {
   sp.slot_code = (int *)p;
   p += (size_t)num_jobs * K * 4;
   if (code_iters) sp.code_iters = (int *)p;
-  p += (size_t)num_jobs * 256;
+  p += (size_t)num_jobs * LDPCA_TRIED * 4;
   sp.slot_dec = p;
   return sp;
 }

@@ -39,6 +39,7 @@ unsigned phi_window_attr(cudaLaunchAttribute &a);
 
 namespace {
 
+static_assert(LDPCA_TRIED <= 64, "one bit of a 64-bit mask per code tried");
 constexpr int kSlots = 4;
 constexpr int kWords = (LDPCA_MAX_N + 31) / 32;  // packed decoded bits per slot
 
@@ -168,7 +169,7 @@ __device__ int pop_item(const LdpcaBatch &A, int which) {
   int *ctr = A.ctr + which;
   for (;;) {
     const long long q = atomicAdd(ctr, 1);
-    if (q >= (long long)count * 64) return -1;
+    if (q >= (long long)count * LDPCA_TRIED) return -1;
     const int k = (int)(q / count), j = list[q % count];
     const LdpcaBatchState &st = A.state[j];
     const int code = st.start + k;

@@ -20,6 +20,13 @@ def circulant(n, period, bpp):
     return dict(N=n, E=3 * n, period=period, jc=3 * np.arange(n + 1), ir_full=ir, bpp=list(bpp), idx=idx)
 
 
+def many_codes(num):
+    """The shipped ladders with every code but the last repeated, `num` codes in all."""
+    shipped = lad.read_compact(os.path.join(ROOT, "dvc_b200", "ladders", "ldpca_ladders.bin"))
+    at = [i // 2 for i in range(2 * 64)][-(num - 1):] + [64]
+    return [dict(L, bpp=[L["bpp"][i] for i in at], idx=[L["idx"][i] for i in at]) for L in shipped]
+
+
 def data_dir(path, ladders):
     os.makedirs(path, exist_ok=True)
     lad.write_compact(os.path.join(path, "ldpca_ladders.bin"), ladders)

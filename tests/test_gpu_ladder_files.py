@@ -1,9 +1,9 @@
 """GPU: ladder files of other codeword lengths than the codec's two (shorter than a
-block's threads, as long, with and without a partial round of columns) against
-the oracle, in the forms a call may take: speculative slots, one block per ladder
-(the call that owns its memory, and one with two codewords per SM, whose queue
-holds the codec's lengths only).  Bits, rates, codes and the bound's bits are
-compared exactly."""
+block's threads, as long, with and without a partial round of columns) and of
+more codes than the shipped ones against the oracle, in the forms a call may
+take: speculative slots, one block per ladder (the call that owns its memory, and
+one with two codewords per SM, whose queue holds the codec's lengths only).
+Bits, rates, codes and the bound's bits are compared exactly."""
 import os
 import shutil
 
@@ -62,3 +62,26 @@ def test_other_lengths_match_the_oracle(context, n):
             assert (res[i, 0], res[i, 1], res[i, 2]) == (orate, ostart, oacc)
             assert np.array_equal(dec[i], odec)
         assert np.array_equal(res, got[0][1])
+
+
+@pytest.mark.parametrize("num", [65, 66, 129])
+def test_many_codes_match_the_oracle(context, num):
+    from oracle import pyoracle as po
+    from dvc_b200 import ldpca_bench as lb
+    ladders = lf.many_codes(num)
+    L = lf.lad.ladder_for(ladders, 1584)
+    ctx, o = context(ladders), lf.oracle(L)
+    lr, acc, crc, x = lb.make_codewords(1584, 4, 70 + num)
+    crc[3] ^= 0x5A  # no code's bits match: every code is tried, up to the full rate
+    lr[3] = np.where(lr[3] > 1, np.float32(20), np.float32(0.05))  # ... from one of the first
+    many = [np.repeat(a, 80, axis=0) for a in (lr, acc, crc)]
+    got = [ctx.ldpca_decode(lr, acc, crc), noalloc(ctx, lr, acc, crc), [a[::80] for a in ctx.ldpca_decode(*many)]]
+    for i in range(4):
+        odec, orate, ostart, oacc, _ = po.ldpca_decode(o, lr[i], np.unpackbits(acc[i]), int(crc[i]),
+                                                       po.compute_ce(lr[i]))
+        assert i < 3 or (oacc == num - 1 and num - 1 - ostart > (64 if num > 66 else 0))
+        for dec, res, ent in got:
+            assert (res[i, 0], res[i, 1], res[i, 2]) == (orate, ostart, oacc)
+            assert np.array_equal(dec[i], odec) and np.array_equal(res[i], got[0][1][i])
+        dec, rate, llr = ctx.LdpcaDecoder(lr[i], np.unpackbits(acc[i]), int(crc[i]), float(got[0][2][i]))
+        assert rate == orate and np.array_equal(dec, odec)

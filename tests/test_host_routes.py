@@ -7,7 +7,7 @@ import subprocess
 
 import pytest
 
-from ladder_files import circulant, data_dir, lad
+from ladder_files import circulant, data_dir, lad, many_codes
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CUDA = "/usr/local/cuda"
@@ -65,3 +65,17 @@ def test_other_codeword_lengths_reach_the_ladder(routes, n, count):
     assert "rc 0" in lines, lines
     ladder = [x for x in launches(lines) if "ldpca_ladder_kernel" in x[1]]
     assert len(ladder) == 1 and ladder[0][7] == "1", lines
+
+
+@pytest.mark.parametrize("num,own_block", [(65, False), (66, True), (129, True)])
+@pytest.mark.parametrize("count", [1, 40, 600])
+def test_ladders_of_many_codes_take_a_block_each(routes, num, own_block, count):
+    """The slots' iteration counts and the queue's masks hold 64 codes a codeword:
+    a file with more keeps the form without either."""
+    d = data_dir(routes.tmp / ("codes%d" % num), many_codes(num))
+    lines = routes("decode", d, 1584, count)
+    assert "rc 0" in lines, lines
+    ladder = [x for x in launches(lines) if "ldpca_ladder_kernel" in x[1]]
+    queue = [x for x in launches(lines) if "ldpca_batch_kernel" in x[1]]
+    alone = [(int(x[3]), int(x[7])) for x in ladder] == [(count, 1)] and not queue
+    assert alone == own_block and len(ladder) + len(queue) == 1, lines
