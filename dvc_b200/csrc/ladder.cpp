@@ -81,6 +81,12 @@ bool load_ladders(const std::string &path, std::vector<LadderHost> &out, std::st
         err = "ladder with a column degree other than 3";
         return false;
       }
+    // (e = 3 n: the codewords' syndromes and decoded bits are whole bytes)
+    if (L.e % 8 != 0 || L.e > 65535) {
+      fclose(f);
+      err = "ladder edge count not a multiple of 8 or above 65535";
+      return false;
+    }
     // expand the per-code rows: row of edge e in code c is the first kept
     // accumulated-syndrome position >= its full-rate row; then the BP layout
     const int gmax = (L.n + 31) / 32;

@@ -79,3 +79,14 @@ def test_ladders_of_many_codes_take_a_block_each(routes, num, own_block, count):
     queue = [x for x in launches(lines) if "ldpca_batch_kernel" in x[1]]
     alone = [(int(x[3]), int(x[7])) for x in ladder] == [(count, 1)] and not queue
     assert alone == own_block and len(ladder) + len(queue) == 1, lines
+
+
+@pytest.mark.parametrize("n,accepted", [(96, True), (100, False), (260, False)])
+def test_lengths_that_are_no_whole_bytes_are_refused(routes, n, accepted):
+    """Syndromes are stored eight bits to a byte, n / 8 bytes a codeword: with
+    another length the last bits of one would be read past its end."""
+    lines = routes("decode", data_dir(routes.tmp / ("n%d" % n), [circulant(n, 4, range(1, 5))]), n, 1)
+    if accepted:
+        assert "rc 0" in lines, lines
+    else:
+        assert lines[0] == "create -4 ladder edge count not a multiple of 8 or above 65535", lines
