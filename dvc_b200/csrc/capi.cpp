@@ -101,11 +101,37 @@ static int ldpca_run(Context &c, int n, int count, const float *lr, const uint8_
   const size_t nb = (size_t)n / 8;
   if (!c.ld_lr.ensure((size_t)count * n * 4) || !c.ld_acc.ensure((size_t)count * nb) ||
       !c.ld_dec.ensure((size_t)count * n) || !c.ld_res.ensure((size_t)count * 16) ||
-      !c.ld_ent.ensure((size_t)count * 4) || !c.ld_jobs.ensure((size_t)count * sizeof(dvc::LdpcaJob)) ||
-      (llr_back && !c.ld_llr.ensure((size_t)count * n * 4))) {
+      !c.ld_ent.ensure((size_t)count * 4) || !c.ld_jobs.ensure((size_t)count * sizeof(dvc::LdpcaJob))) {
     c.err = "device allocation failed";
     return DVC_E_NOMEM;
   }
+  // Codewords that leave SMs idle are decoded with speculative slots (and
+  // clusters), others by a block per ladder, without scratch.  One codeword
+  // alone, sequential -> so: QCIF 2.2 -> 0.26 ms, CIF 7.9 -> 0.43 ms; 33 QCIF
+  // codewords 4.5 -> 0.89 ms, 203 CIF ones 19.8 -> 13.2 ms.  Without memory for
+  // the slots a block per ladder, too.
+  cudaStream_t s = c.stream;
+  int K = 1, C = 1;
+  dvc::LdpcaSpec sp;
+  if (counted && count < 2 * sms) {
+    dvc::ldpca_spec_shape(n, count, sms, K, C);
+    // once for every count (by default fewer than 2 * sms codewords of either length)
+    const size_t had = c.ld_spec.bytes;
+    const bool room = (!llr_back || c.ld_llr.ensure((size_t)count * n * 4)) &&
+                      c.ld_spec.ensure(std::max(dvc::ldpca_spec_scratch_bytes(6336, 2 * sms, 4),
+                                                dvc::ldpca_spec_scratch_bytes(n, count, K)));
+    if (!room) cudaGetLastError();  // the failed allocation's, or the next launch would report it
+    if (c.ld_spec.bytes != had) c.ld_spec_jobs = 0;
+    if (room) {
+      sp = dvc::ldpca_spec_carve(c.ld_spec.p, count, K, true);
+      if (c.ld_spec_jobs != count || c.ld_spec_k != K) {
+        c.ld_spec_jobs = 0;
+        if ((st = cuda_status(c, dvc::ldpca_spec_reset(sp, count, K, s), "LDPCA scratch"))) return st;
+      }
+    }
+  }
+  // the log ratios: apart from lr where other slots read it
+  float *llr_dev = !llr_back ? nullptr : sp.best ? c.ld_llr.as<float>() : c.ld_lr.as<float>();
   std::vector<dvc::LdpcaJob> jobs(count);
   for (int i = 0; i < count; i++) {
     dvc::LdpcaJob &j = jobs[i];
@@ -121,30 +147,7 @@ static int ldpca_run(Context &c, int n, int count, const float *lr, const uint8_
       j.use_given_entropy = 1;
       j.given_entropy = given_entropy[i];
     }
-    if (llr_back) j.llr_out = c.ld_llr.as<float>() + (size_t)i * n;  // apart from lr, which other slots read
-  }
-  cudaStream_t s = c.stream;
-  // Codewords that leave SMs idle are decoded with speculative slots (and
-  // clusters), others by a block per ladder, without scratch.  One codeword alone, sequential -> so: QCIF 2.2
-  // -> 0.26 ms, CIF 7.9 -> 0.43 ms; 33 QCIF codewords 4.5 -> 0.89 ms, 203 CIF
-  // ones 19.8 -> 13.2 ms.
-  int K = 1, C = 1;
-  dvc::LdpcaSpec sp;
-  if (counted && count < 2 * sms) {
-    dvc::ldpca_spec_shape(n, count, sms, K, C);
-    // once for every count (by default fewer than 2 * sms codewords of either length)
-    const size_t had = c.ld_spec.bytes;
-    if (!c.ld_spec.ensure(std::max(dvc::ldpca_spec_scratch_bytes(6336, 2 * sms, 4),
-                                   dvc::ldpca_spec_scratch_bytes(n, count, K)))) {
-      c.err = "device allocation failed";
-      return DVC_E_NOMEM;
-    }
-    if (c.ld_spec.bytes != had) c.ld_spec_jobs = 0;
-    sp = dvc::ldpca_spec_carve(c.ld_spec.p, count, K, true);
-    if (c.ld_spec_jobs != count || c.ld_spec_k != K) {
-      c.ld_spec_jobs = 0;
-      if ((st = cuda_status(c, dvc::ldpca_spec_reset(sp, count, K, s), "LDPCA scratch"))) return st;
-    }
+    if (llr_back) j.llr_out = llr_dev + (size_t)i * n;
   }
   if ((st = cuda_status(c, cudaMemcpyAsync(c.ld_lr.p, lr, (size_t)count * n * 4, cudaMemcpyHostToDevice, s), "H2D lr")))
     return st;
@@ -169,7 +172,7 @@ static int ldpca_run(Context &c, int n, int count, const float *lr, const uint8_
       (st = cuda_status(c, cudaMemcpyAsync(entropy, c.ld_ent.p, (size_t)count * 4, cudaMemcpyDeviceToHost, s), "D2H ent")))
     return st;
   if (llr_back &&
-      (st = cuda_status(c, cudaMemcpyAsync(llr_back, c.ld_llr.p, (size_t)count * n * 4, cudaMemcpyDeviceToHost, s),
+      (st = cuda_status(c, cudaMemcpyAsync(llr_back, llr_dev, (size_t)count * n * 4, cudaMemcpyDeviceToHost, s),
                         "D2H llr")))
     return st;
   if ((st = cuda_status(c, cudaStreamSynchronize(s), "ldpca sync"))) return st;

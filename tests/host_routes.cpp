@@ -23,12 +23,14 @@ std::map<const void *, std::string> g_name;   // host stub -> kernel
 std::map<const void *, size_t> g_smem;        // largest dynamic shared memory allowed
 std::map<void *, size_t> g_mem;               // device allocations
 size_t g_live = 0, g_fail_from = ~(size_t)0;  // bytes held; allocations of this size and more fail
+int g_fail_after = 0;                         // ... but for the first few
 int g_streams = 0, g_events = 0;              // alive
 bool g_record = false;
+cudaError_t g_last = cudaSuccess;
 
 cudaError_t take(void **p, size_t bytes) {
   *p = nullptr;
-  if (bytes >= g_fail_from || bytes > ((size_t)1 << 36)) return cudaErrorMemoryAllocation;
+  if ((bytes >= g_fail_from && g_fail_after-- <= 0) || bytes > ((size_t)1 << 36)) return g_last = cudaErrorMemoryAllocation;
   *p = aligned_alloc(256, (bytes + 255) & ~(size_t)255);
   memset(*p, 0, bytes);
   g_mem[*p] = bytes;
@@ -183,7 +185,11 @@ cudaError_t cudaDestroyTextureObject(cudaTextureObject_t) { return cudaSuccess; 
 cudaChannelFormatDesc cudaCreateChannelDesc(int x, int y, int z, int w, cudaChannelFormatKind f) {
   return {x, y, z, w, f};
 }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError() {
+  const cudaError_t e = g_last;
+  g_last = cudaSuccess;
+  return e;
+}
 const char *cudaGetErrorString(cudaError_t e) { return e == cudaErrorMemoryAllocation ? "out of memory" : "CUDA error"; }
 
 int dvc_libm_build(const char *, int, char *, int) { return 0; }
@@ -236,6 +242,14 @@ static void files(char **a) {
   }
 }
 
+// the reference-shaped call on zeros
+static int decoder_zeros(dvc_ctx *c, int n) {
+  std::vector<float> lr(n, 1.0f);
+  std::vector<uint8_t> acc(n), dec(n);
+  int rate = 0;
+  return dvc_LdpcaDecoder(c, n, lr.data(), acc.data(), dec.data(), &rate, 0, 0.5f);
+}
+
 // decode DATA TABLES n count
 static void decode(char **a) {
   dvc_ctx *c = context(a[0], a[1]);
@@ -245,10 +259,27 @@ static void decode(char **a) {
   dvc_destroy(c);
 }
 
+// scarce DATA TABLES n count from after: the two LDPCA calls while allocations
+// of `from` bytes and more, but for the first `after`, are refused, then with memory
+static void scarce(char **a) {
+  dvc_ctx *c = context(a[0], a[1]);
+  const int n = atoi(a[2]), count = atoi(a[3]);
+  g_record = true;
+  for (int turn = 0; turn < 2; turn++) {
+    g_fail_from = turn == 0 ? strtoull(a[4], nullptr, 0) : ~(size_t)0;
+    g_fail_after = atoi(a[5]);
+    const int rc = count > 0 ? decode_zeros(c, n, count) : decoder_zeros(c, n);
+    printf("rc %d last %d\n", rc, (int)cudaGetLastError());
+  }
+  g_record = false;
+  dvc_destroy(c);
+}
+
 int main(int argc, char **argv) {
   const std::string mode = argc > 1 ? argv[1] : "";
   if (mode == "files" && argc == 5) files(argv + 2);
   else if (mode == "decode" && argc == 6) decode(argv + 2);
+  else if (mode == "scarce" && argc == 8) scarce(argv + 2);
   else return 2;
   printf("left bytes %zu streams %d events %d\n", g_live, g_streams, g_events);
   return 0;

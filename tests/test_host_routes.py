@@ -90,3 +90,16 @@ def test_lengths_that_are_no_whole_bytes_are_refused(routes, n, accepted):
         assert "rc 0" in lines, lines
     else:
         assert lines[0] == "create -4 ladder edge count not a multiple of 8 or above 65535", lines
+
+
+SHIPPED = os.path.join(ROOT, "dvc_b200", "ladders")
+
+
+@pytest.mark.parametrize("n,count,size,after", [
+    (1584, 1, 1 << 20, 0), (6336, 7, 1 << 20, 0), (6336, 295, 7500000, 0),  # no room for the slots
+    (1584, 0, 1 << 20, 0), (6336, 0, 6336 * 4, 1)])                          # count 0: dvc_LdpcaDecoder
+def test_calls_without_memory_for_slots_decode_a_block_each(routes, n, count, size, after):
+    lines = routes("scarce", SHIPPED, n, count, size, after)
+    assert [x for x in lines if x.startswith("rc")] == ["rc 0 last 0"] * 2, lines
+    poor, rich = [(int(x[3]), int(x[7])) for x in launches(lines) if "ldpca_ladder_kernel" in x[1]]
+    assert poor == (max(count, 1), 1) and rich[0] > poor[0], lines
