@@ -62,9 +62,11 @@ extern "C" void dvc_destroy(dvc_ctx *ctx) {
 
 extern "C" const char *dvc_last_error(dvc_ctx *ctx) { return ctx ? ctx->c.err.c_str() : "null context"; }
 
-static int ldpca_batch_run(Context &c, int count, const int *n, const float *lr, const uint8_t *acc, const uint8_t *crc,
-                           const int *start, uint8_t *decoded, int *results, float *entropy, int max_iter,
-                           long long *bp_iterations, double *kernel_ms);
+// codewords of lengths n[], or all of length same_n without n
+static int ldpca_batch_run(Context &c, int count, const int *n, int same_n, const float *lr, const uint8_t *acc,
+                           const uint8_t *crc, const int *start, uint8_t *decoded, int *results, float *entropy,
+                           int max_iter, long long *bp_iterations, double *kernel_ms);
+static const int kBatchMost = 1 << 22;  // codewords of one batch
 
 static int ldpca_run(Context &c, int n, int count, const float *lr, const uint8_t *acc, const uint8_t *crc,
                      uint8_t *decoded, int *results, float *entropy, int max_iter, const float *given_entropy,
@@ -89,10 +91,9 @@ static int ldpca_run(Context &c, int n, int count, const float *lr, const uint8_
   // A ladder of more codes than the queue and the slots count (a file may hold
   // any number) takes a block per codeword, which counts nothing.
   const bool counted = L->num_codes - 1 <= LDPCA_TRIED;
-  const bool queue = counted && count >= 2 * sms && !given_entropy && !llr_back;
+  const bool queue = counted && count >= 2 * sms && count <= kBatchMost && !given_entropy && !llr_back;
   if (queue) {
-    const std::vector<int> ns(count, n);
-    st = ldpca_batch_run(c, count, ns.data(), lr, acc, crc, nullptr, decoded, results, entropy, max_iter, nullptr,
+    st = ldpca_batch_run(c, count, nullptr, n, lr, acc, crc, nullptr, decoded, results, entropy, max_iter, nullptr,
                          nullptr);
     if (st == DVC_OK || st == DVC_E_CUDA) return st;
     for (auto *b : {&c.bt_lr, &c.bt_acc, &c.bt_dec, &c.bt_res, &c.bt_ent, &c.bt_cw, &c.bt_state}) b->release();
@@ -189,10 +190,10 @@ extern "C" int dvc_ldpca_decode(dvc_ctx *ctx, int n, int count, const float *lr,
   return ldpca_run(ctx->c, n, count, lr, acc, crc, decoded, results, entropy, max_iter, nullptr, nullptr);
 }
 
-static int ldpca_batch_run(Context &c, int count, const int *n, const float *lr, const uint8_t *acc, const uint8_t *crc,
-                           const int *start, uint8_t *decoded, int *results, float *entropy, int max_iter,
-                           long long *bp_iterations, double *kernel_ms) {
-  if (count <= 0 || count > (1 << 22) || !n || !lr || !acc || !crc || !results || max_iter <= 0) {
+static int ldpca_batch_run(Context &c, int count, const int *n, int same_n, const float *lr, const uint8_t *acc,
+                           const uint8_t *crc, const int *start, uint8_t *decoded, int *results, float *entropy,
+                           int max_iter, long long *bp_iterations, double *kernel_ms) {
+  if (count <= 0 || count > kBatchMost || (!n && !same_n) || !lr || !acc || !crc || !results || max_iter <= 0) {
     c.err = "dvc_ldpca_decode_batch: bad arguments";
     return DVC_E_ARG;
   }
@@ -206,12 +207,13 @@ static int ldpca_batch_run(Context &c, int count, const int *n, const float *lr,
   lists.reserve(count);
   long long lr_off = 0, byte_off = 0;
   for (int i = 0; i < count; i++) {
-    if (n[i] != 1584 && n[i] != 6336) {
-      c.err = "dvc_ldpca_decode_batch: codeword " + std::to_string(i) + " has length " + std::to_string(n[i]) +
+    const int ni = n ? n[i] : same_n;
+    if (ni != 1584 && ni != 6336) {
+      c.err = "dvc_ldpca_decode_batch: codeword " + std::to_string(i) + " has length " + std::to_string(ni) +
               " (1584 or 6336)";
       return DVC_E_ARG;
     }
-    cw[i].cif = n[i] == 6336;
+    cw[i].cif = ni == 6336;
     cw[i].crc = crc[i];
     cw[i].given_start = start ? start[i] : -1;
     if (start && (start[i] < 0 || start[i] > 64)) {
@@ -221,8 +223,8 @@ static int ldpca_batch_run(Context &c, int count, const int *n, const float *lr,
     cw[i].lr_off = lr_off;
     cw[i].acc_off = byte_off / 8;
     cw[i].dec_off = byte_off;
-    lr_off += n[i];
-    byte_off += n[i];
+    lr_off += ni;
+    byte_off += ni;
   }
   for (int i = 0; i < count; i++)
     if (cw[i].cif) lists.push_back(i);
@@ -305,7 +307,7 @@ extern "C" int dvc_ldpca_decode_batch(dvc_ctx *ctx, int count, const int *n, con
                                       const uint8_t *crc, const int *start, uint8_t *decoded, int *results,
                                       float *entropy, int max_iter, long long *bp_iterations, double *kernel_ms) {
   if (!ctx) return DVC_E_ARG;
-  return ldpca_batch_run(ctx->c, count, n, lr, acc, crc, start, decoded, results, entropy, max_iter, bp_iterations,
+  return ldpca_batch_run(ctx->c, count, n, 0, lr, acc, crc, start, decoded, results, entropy, max_iter, bp_iterations,
                          kernel_ms);
 }
 

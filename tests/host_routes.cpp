@@ -6,6 +6,7 @@
 // files and reads what it prints.  The C-library table sweeps are left out (the
 // kernels that read the tables do not run).
 #include <cuda_runtime.h>
+#include <sys/resource.h>
 
 #include <cstdio>
 #include <cstdlib>
@@ -275,11 +276,26 @@ static void scarce(char **a) {
   dvc_destroy(c);
 }
 
+// huge DATA TABLES n count: a count that no device holds (the inputs are not read)
+static void huge(char **a) {
+  dvc_ctx *c = context(a[0], a[1]);
+  const int n = atoi(a[2]), count = atoi(a[3]);
+  const rlimit most = {(rlim_t)3 << 30, (rlim_t)3 << 30};
+  setrlimit(RLIMIT_AS, &most);
+  g_fail_from = (size_t)1 << 30;
+  float lr = 1.0f;
+  uint8_t acc = 0, crc = 0;
+  int res[4] = {0};
+  printf("rc %d\n", dvc_ldpca_decode(c, n, count, &lr, &acc, &crc, nullptr, res, nullptr, 50));
+  dvc_destroy(c);
+}
+
 int main(int argc, char **argv) {
   const std::string mode = argc > 1 ? argv[1] : "";
   if (mode == "files" && argc == 5) files(argv + 2);
   else if (mode == "decode" && argc == 6) decode(argv + 2);
   else if (mode == "scarce" && argc == 8) scarce(argv + 2);
+  else if (mode == "huge" && argc == 6) huge(argv + 2);
   else return 2;
   printf("left bytes %zu streams %d events %d\n", g_live, g_streams, g_events);
   return 0;

@@ -103,3 +103,9 @@ def test_calls_without_memory_for_slots_decode_a_block_each(routes, n, count, si
     assert [x for x in lines if x.startswith("rc")] == ["rc 0 last 0"] * 2, lines
     poor, rich = [(int(x[3]), int(x[7])) for x in launches(lines) if "ldpca_ladder_kernel" in x[1]]
     assert poor == (max(count, 1), 1) and rich[0] > poor[0], lines
+
+
+@pytest.mark.parametrize("n,count", [(1584, 2**31 - 1), (6336, 2**22 + 1)])
+def test_a_count_that_no_device_holds_is_refused(routes, n, count):
+    """... with a status, and without host memory for so many codewords."""
+    assert "rc -3" in routes("huge", SHIPPED, n, count)
