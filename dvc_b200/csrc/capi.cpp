@@ -532,6 +532,7 @@ struct dvc_session {
   std::vector<int> batch_stream;
   std::vector<cudaEvent_t> batch_done;
   std::vector<cudaStream_t> streams;
+  std::vector<dvc::SideStreams> side;          // of each stream, shared by its batches
   std::vector<std::vector<dvc::FrameResult>> results;
   cudaEvent_t t0 = nullptr, t1 = nullptr;
   std::vector<cudaEvent_t> done;
@@ -548,6 +549,7 @@ static void session_release(dvc_session *S) {
   for (auto &b : S->batches) b.release();
   for (auto *v : {&S->ref, &S->lp, &S->ip, &S->out, &S->olp, &S->oip, &S->init})
     for (auto &b : *v) b.release();
+  for (auto &sd : S->side) sd.release();
   for (cudaStream_t st : S->streams) cudaStreamDestroy(st);
   for (cudaEvent_t e : S->done) cudaEventDestroy(e);
   for (cudaEvent_t e : S->batch_done) cudaEventDestroy(e);
@@ -701,6 +703,7 @@ extern "C" int dvc_session_create(dvc_ctx *ctx, int count, const dvc_wz_frame *f
   const int nb = (int)S->batch_frames.size();
   S->batches.resize(nb);
   S->results.resize(nb);
+  S->side.resize(nstreams);
   for (int b = 0; b < nb; b++) {
     cudaEvent_t e;
     if ((st = cuda_status(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event"))) return bail(st);
@@ -747,6 +750,7 @@ extern "C" int dvc_session_create(dvc_ctx *ctx, int count, const dvc_wz_frame *f
     cudaStream_t sb = S->streams[S->batch_stream[b]];
     // frames decoding at once: those of the batch's level, one batch per stream
     const int concurrent = std::min(level_frames[level[S->batch_frames[b][0]]], nstreams * max_batch);
+    S->batches[b].set_side_streams(&S->side[S->batch_stream[b]]);
     if (!S->batches[b].prepare(c, specs, sb, concurrent)) return bail(DVC_E_CUDA);
     if ((st = cuda_status(c, cudaStreamSynchronize(sb), "session prepare"))) return bail(st);
   }

@@ -116,15 +116,34 @@ bool FrameBatcher::ensure_pinned(size_t b) {
   return true;
 }
 
+bool SideStreams::ensure(Context &ctx, size_t n) {
+  if (n && !fork && !ctx.cuda_ok(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming), "event")) return false;
+  while (done.size() < n) {
+    cudaEvent_t e;
+    if (!ctx.cuda_ok(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event")) return false;
+    done.push_back(e);
+  }
+  while (streams.size() < n) {
+    cudaStream_t st;
+    if (!ctx.cuda_ok(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "stream")) return false;
+    streams.push_back(st);
+  }
+  return true;
+}
+
+void SideStreams::release() {
+  for (cudaStream_t st : streams) cudaStreamDestroy(st);
+  streams.clear();
+  for (cudaEvent_t e : done) cudaEventDestroy(e);
+  done.clear();
+  if (fork) cudaEventDestroy(fork);
+  fork = nullptr;
+}
+
 void FrameBatcher::release() {
   for (cudaEvent_t e : ev_) cudaEventDestroy(e);
   ev_.clear();
-  for (cudaStream_t st : side_) cudaStreamDestroy(st);
-  side_.clear();
-  for (cudaEvent_t e : side_done_) cudaEventDestroy(e);
-  side_done_.clear();
-  if (fork_) cudaEventDestroy(fork_);
-  fork_ = nullptr;
+  own_side_.release();
   for (auto &s : slots_) s.release();
   slots_.clear();
   frames_dev_.release();
@@ -435,16 +454,7 @@ bool FrameBatcher::prepare(Context &ctx, const std::vector<FrameSpec> &frames, c
     if (!ctx.cuda_ok(ldpca_spec_reset(ldpca_spec_carve(spec_.as<uint8_t>() + G.spec_off, G.nf, G.spec_k), G.nf, G.spec_k, s),
                      "LDPCA scratch"))
       return false;
-  while (side_.size() + 1 < groups.size()) {
-    cudaStream_t st;
-    if (!ctx.cuda_ok(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "stream")) return false;
-    side_.push_back(st);
-    cudaEvent_t e;
-    if (!ctx.cuda_ok(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event")) return false;
-    side_done_.push_back(e);
-  }
-  if (groups.size() > 1 && !fork_ && !ctx.cuda_ok(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming), "event"))
-    return false;
+  if (!side().ensure(ctx, groups.size() - 1)) return false;
   groups_ = std::move(groups);
   fd_ = fd;
   qb_ = qb;
@@ -564,12 +574,13 @@ bool FrameBatcher::execute(Context &ctx, cudaStream_t s, int max_iter, ProfileSt
     }
   }
   const size_t ng = groups_.size();
+  SideStreams &sd = side();
   if (ng > 1) {
-    if (!ctx.cuda_ok(cudaEventRecord(fork_, s), "event")) return false;
+    if (!ctx.cuda_ok(cudaEventRecord(sd.fork, s), "event")) return false;
     for (size_t g = 1; g < ng; g++)
-      if (!ctx.cuda_ok(cudaStreamWaitEvent(side_[g - 1], fork_, 0), "wait")) return false;
+      if (!ctx.cuda_ok(cudaStreamWaitEvent(sd.streams[g - 1], sd.fork, 0), "wait")) return false;
   }
-  auto stream_of = [&](size_t g) { return g == 0 ? s : side_[g - 1]; };
+  auto stream_of = [&](size_t g) { return g == 0 ? s : sd.streams[g - 1]; };
   bool ok = true;
   for (size_t g = 0; g < ng && ok; g++) {
     groups_[g].next = 0;
@@ -587,8 +598,8 @@ bool FrameBatcher::execute(Context &ctx, cudaStream_t s, int max_iter, ProfileSt
   for (size_t g = 0; g < ng && ok; g++) ok = launch_end(ctx, groups_[g], stream_of(g));
   // the batch's stream joins the others even after a failure
   for (size_t g = 1; g < ng; g++)
-    if (!ctx.cuda_ok(cudaEventRecord(side_done_[g - 1], side_[g - 1]), "event") ||
-        !ctx.cuda_ok(cudaStreamWaitEvent(s, side_done_[g - 1], 0), "wait"))
+    if (!ctx.cuda_ok(cudaEventRecord(sd.done[g - 1], sd.streams[g - 1]), "event") ||
+        !ctx.cuda_ok(cudaStreamWaitEvent(s, sd.done[g - 1], 0), "wait"))
       return false;
   if (ok && prof) prof->kernel_launches += launches_per_execute();
   return ok;

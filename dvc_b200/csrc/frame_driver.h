@@ -64,6 +64,16 @@ struct ProfileStats {
   long long kernel_launches = 0;  // every kernel this library launched
 };
 
+// The streams a batch's groups beyond the first decode on, with the events that
+// fork them from the batch's stream and join them to it.
+struct SideStreams {
+  std::vector<cudaStream_t> streams;
+  std::vector<cudaEvent_t> done;  // the end of each
+  cudaEvent_t fork = nullptr;
+  bool ensure(Context &ctx, size_t n);  // at least n of them
+  void release();
+};
+
 class FrameBatcher {
  public:
   // prepare: per-frame constants, block lists, packed inputs, descriptors and
@@ -92,6 +102,10 @@ class FrameBatcher {
   // grow device buffers in the order of this stream (the batcher is only used
   // on it), so that a growth does not wait for other streams' work
   void set_alloc_stream(cudaStream_t s) { alloc_stream_ = s; }
+  // decode the groups on streams that outlive the batcher and that it shares with
+  // others: those whose batches run before and after its own on one stream
+  // (batches side by side would wait for each other)
+  void set_side_streams(SideStreams *side) { shared_side_ = side; }
   int frames() const { return nf_; }
   // launches execute() issues (for the launch counter)
   long long launches_per_execute() const;
@@ -122,9 +136,8 @@ class FrameBatcher {
     size_t next = 0;            // execute(): next step to launch
   };
   std::vector<Group> groups_;
-  std::vector<cudaStream_t> side_;      // streams of groups 1, 2, ...
-  std::vector<cudaEvent_t> side_done_;  // their ends, and the batch's start
-  cudaEvent_t fork_ = nullptr;
+  SideStreams own_side_, *shared_side_ = nullptr;  // streams of groups 1, 2, ...
+  SideStreams &side() { return shared_side_ ? *shared_side_ : own_side_; }
   bool launch_start(Context &ctx, const Group &G, cudaStream_t s);
   bool launch_band(Context &ctx, Group &G, cudaStream_t s, int max_iter, ProfileStats *prof);
   bool launch_end(Context &ctx, const Group &G, cudaStream_t s);

@@ -290,12 +290,56 @@ static void huge(char **a) {
   dvc_destroy(c);
 }
 
+// a frame of zeros between two references
+struct Frame {
+  std::vector<uint8_t> past, future, crc, acc, recon;
+  int range[16];
+  dvc_wz_frame f;
+  Frame(int w, int h, int q) : past(w * h), future(w * h), crc(64), acc(64 * w * h / 128), recon(w * h) {
+    for (int &r : range) r = 100;
+    memset(&f, 0, sizeof f);
+    f.width = w;
+    f.height = h;
+    f.qindex = q;
+    f.cur_idx = 1;
+    f.future_idx = 2;
+    f.past = past.data();
+    f.future = future.data();
+    f.crc = crc.data();
+    f.acc_synd = acc.data();
+    f.recon = recon.data();
+    f.ac_range = range;
+  }
+};
+
+// session DATA TABLES frames max_batch streams: what a session of independent
+// QCIF frames holds, and two runs of it
+static void session(char **a) {
+  dvc_ctx *c = context(a[0], a[1]);
+  const int count = atoi(a[2]), s0 = g_streams;
+  std::vector<Frame> frames;
+  std::vector<dvc_wz_frame> list;
+  frames.reserve(count);
+  for (int i = 0; i < count; i++) {
+    frames.emplace_back(176, 144, 1);
+    list.push_back(frames.back().f);
+  }
+  dvc_session *s = nullptr;
+  int rc = dvc_session_create(c, count, list.data(), atoi(a[3]), atoi(a[4]), &s);
+  printf("rc %d\nstreams %d\n", rc, g_streams - s0);
+  double ms = 0;
+  for (int run = 0; run < 2; run++) printf("rc %d\n", dvc_session_run(s, 0, &ms));
+  dvc_session_destroy(s);
+  dvc_destroy(c);
+}
+
 int main(int argc, char **argv) {
   const std::string mode = argc > 1 ? argv[1] : "";
   if (mode == "files" && argc == 5) files(argv + 2);
   else if (mode == "decode" && argc == 6) decode(argv + 2);
   else if (mode == "scarce" && argc == 8) scarce(argv + 2);
   else if (mode == "huge" && argc == 6) huge(argv + 2);
+  else if (mode == "session" && argc == 7) session(argv + 2);
   else return 2;
   printf("left bytes %zu streams %d events %d\n", g_live, g_streams, g_events);
   return 0;

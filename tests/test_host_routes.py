@@ -109,3 +109,14 @@ def test_calls_without_memory_for_slots_decode_a_block_each(routes, n, count, si
 def test_a_count_that_no_device_holds_is_refused(routes, n, count):
     """... with a status, and without host memory for so many codewords."""
     assert "rc -3" in routes("huge", SHIPPED, n, count)
+
+
+@pytest.mark.parametrize("frames,max_batch,streams,side", [
+    (64, 4, 2, 6), (40, 8, 4, 28), (9, 16, 1, 4), (33, 16, 4, 14), (66, 33, 2, 0)])
+def test_a_sessions_batches_share_their_streams(routes, frames, max_batch, streams, side):
+    """Batches on one of the session's streams run one after another: the streams
+    their groups decode on (up to seven) are the stream's, however many they are."""
+    lines = routes("session", SHIPPED, frames, max_batch, streams)
+    assert [x for x in lines if x.startswith("rc")] == ["rc 0"] * 3, lines
+    assert "streams %d" % (streams + side) in lines, lines
+    assert lines[-1] == "left bytes 0 streams 0 events 0"
