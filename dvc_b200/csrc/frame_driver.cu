@@ -78,26 +78,78 @@ static cudaError_t ensure_scales() {
   return e;
 }
 
+// the buffers of a slot and their sizes for a frame
+struct SlotBuf {
+  DevBuf Slot::*buf;
+  size_t bytes;
+};
+static std::vector<SlotBuf> slot_buffers(int w, int h, size_t pdf_floats, size_t in_bytes, size_t out_bytes) {
+  const size_t fs = (size_t)w * h, n = fs / 16;
+  const size_t b16n = fs / 256, b8n = fs / 64, octn = (size_t)(w - 3) * (h - 3) * 16;
+  return {{&Slot::si, fs},
+          {&Slot::dbf, fs},
+          {&Slot::residue, fs * 4},
+          {&Slot::side_trans, fs * 4},
+          {&Slot::recons_trans, fs * 4},
+          {&Slot::alpha, fs * 4},
+          {&Slot::lr, 3 * n * 4},
+          {&Slot::oct, octn * 2},
+          {&Slot::smf, n * 81 * 4},
+          {&Slot::pdf, pdf_floats * 4},
+          {&Slot::mb_mv, b16n * sizeof(MVd)},
+          {&Slot::fmv, b16n * sizeof(MVd)},
+          {&Slot::blk_mv, b8n * sizeof(MVd)},
+          {&Slot::blk_mv2, b8n * sizeof(MVd)},
+          {&Slot::holes, b16n * 16},
+          {&Slot::mse, b8n * 8},
+          {&Slot::stats, 32 * 4},
+          {&Slot::in, in_bytes},
+          {&Slot::out, out_bytes},
+          {&Slot::db_img, fs},
+          {&Slot::db_mode, 2 * n},
+          {&Slot::db_bs, 2 * n * 8},
+          {&Slot::si_mv, 2 * n * 4}};
+}
+
 bool Slot::ensure(int w_, int h_, size_t pdf_floats, size_t in_bytes, size_t out_bytes, cudaStream_t a) {
-  const size_t fs = (size_t)w_ * h_, n = fs / 16;
-  const size_t b16n = fs / 256, b8n = fs / 64, octn = (size_t)(w_ - 3) * (h_ - 3) * 16;
-  bool ok = si.ensure(fs, a) && dbf.ensure(fs, a) && residue.ensure(fs * 4, a) && side_trans.ensure(fs * 4, a) &&
-            recons_trans.ensure(fs * 4, a) && alpha.ensure(fs * 4, a) && lr.ensure(3 * n * 4, a) &&
-            oct.ensure(octn * 2, a) && smf.ensure(n * 81 * 4, a) && pdf.ensure(pdf_floats * 4, a) &&
-            mb_mv.ensure(b16n * sizeof(MVd), a) && fmv.ensure(b16n * sizeof(MVd), a) &&
-            blk_mv.ensure(b8n * sizeof(MVd), a) && blk_mv2.ensure(b8n * sizeof(MVd), a) && holes.ensure(b16n * 16, a) &&
-            mse.ensure(b8n * 8, a) && stats.ensure(32 * 4, a) && in.ensure(in_bytes, a) && out.ensure(out_bytes, a) &&
-            db_img.ensure(fs, a) && db_mode.ensure(2 * n, a) && db_bs.ensure(2 * n * 8, a) && si_mv.ensure(2 * n * 4, a);
+  bool ok = true;
+  for (const SlotBuf &b : slot_buffers(w_, h_, pdf_floats, in_bytes, out_bytes)) ok = ok && (this->*b.buf).ensure(b.bytes, a);
   w = w_;
   h = h_;
   return ok;
 }
 
 void Slot::release() {
-  DevBuf *all[] = {&si, &dbf, &residue, &side_trans, &recons_trans, &alpha, &lr, &oct, &smf, &pdf,
-                   &mb_mv, &fmv, &blk_mv, &blk_mv2, &holes, &mse, &stats, &in, &out, &db_img, &db_mode, &db_bs,
-                   &si_mv};
-  for (DevBuf *b : all) b->release();
+  for (const SlotBuf &b : slot_buffers(16, 16, 0, 0, 0)) (this->*b.buf).release();
+}
+
+static size_t align16(size_t v) { return (v + 15) & ~(size_t)15; }
+
+// a frame's packed inputs: mode map, WZ block list, block -> list position,
+// CRCs, syndromes, the past reference's mode map
+struct Packed {
+  size_t mode, sir, sob, crc, acc, pmode, total;
+  Packed(int w, int h, int qb) {
+    const size_t n = (size_t)w * h / 16, nb = n / 8, b8n = n / 4;
+    mode = 0;
+    sir = align16(mode + b8n);
+    sob = align16(sir + n * 4);
+    crc = align16(sob + n * 4);
+    acc = align16(crc + (size_t)qb);
+    pmode = align16(acc + (size_t)qb * nb);
+    total = align16(pmode + b8n);
+  }
+};
+
+// a slot's results: four words and the bound of every bitplane
+static size_t slot_out_bytes(int qb) { return (size_t)qb * 20 + 64; }
+
+size_t frame_device_bytes(int w, int h, int q, size_t pdf_floats) {
+  const int n = w * h / 16, qb = qbits_per_block(q), most_steps = qbits_per_block(8);
+  size_t sum = 0;
+  for (const SlotBuf &b : slot_buffers(w, h, pdf_floats, Packed(w, h, qb).total, slot_out_bytes(qb))) sum += b.bytes;
+  // the frame's descriptor, its jobs (of every step of the batch), its part of the ladder's scratch
+  return sum + sizeof(FrameDev) + most_steps * sizeof(LdpcaJob) + ldpca_spec_scratch_bytes(n, 1, 32) + 256;
 }
 
 bool FrameBatcher::ensure_pinned(size_t b) {
@@ -156,8 +208,6 @@ void FrameBatcher::release() {
   pinned_bytes_ = 0;
 }
 
-static size_t align16(size_t v) { return (v + 15) & ~(size_t)15; }
-
 bool FrameBatcher::prepare(Context &ctx, const std::vector<FrameSpec> &frames, cudaStream_t s, int concurrent,
                            int max_groups) {
   const int nf = (int)frames.size();
@@ -184,24 +234,14 @@ bool FrameBatcher::prepare(Context &ctx, const std::vector<FrameSpec> &frames, c
   // ---- host-side per-frame constants, WZ block lists and upload packing
   std::vector<FrameDev> fd(nf);
   std::vector<std::vector<int>> plane_base(nf);
-  struct Packed {
-    size_t mode, sir, sob, crc, acc, pmode, total;
-  };
-  std::vector<Packed> pk(nf);
+  std::vector<Packed> pk;
   std::vector<int> qb(nf);
   size_t pinned_need = 0;
   for (int f = 0; f < nf; f++) {
     const FrameSpec &F = frames[f];
     qb[f] = qbits_per_block(F.qindex);
-    Packed &p = pk[f];
-    p.mode = 0;
-    p.sir = align16(p.mode + b8n);
-    p.sob = align16(p.sir + (size_t)n * 4);
-    p.crc = align16(p.sob + (size_t)n * 4);
-    p.acc = align16(p.crc + (size_t)qb[f]);
-    p.pmode = align16(p.acc + (size_t)qb[f] * nb);
-    p.total = align16(p.pmode + b8n);
-    pinned_need += p.total;
+    pk.emplace_back(w, h, qb[f]);
+    pinned_need += pk[f].total;
   }
   const size_t fd_off = pinned_need;
   pinned_need += align16(sizeof(FrameDev) * nf);
@@ -326,7 +366,7 @@ bool FrameBatcher::prepare(Context &ctx, const std::vector<FrameSpec> &frames, c
       memset(P + p.pmode, 0, b8n);
     memcpy(P + p.acc, F.acc, (size_t)qb[f] * nb);
     Slot &S = slots_[f];
-    if (!S.ensure(w, h, (size_t)std::max(nsir, 1) * pdf_stride, p.total, (size_t)qb[f] * 20 + 64, alloc_stream_))
+    if (!S.ensure(w, h, (size_t)std::max(nsir, 1) * pdf_stride, p.total, slot_out_bytes(qb[f]), alloc_stream_))
       return ctx.fail("device allocation for frame slot failed");
     uint8_t *in = S.in.as<uint8_t>();
     D.mode = in + p.mode;
@@ -641,12 +681,8 @@ void FrameBatcher::read_results(std::vector<FrameResult> &results) {
 
 size_t FrameBatcher::device_bytes() const {
   size_t b = frames_dev_.bytes + jobs_dev_.bytes + spec_.bytes;
-  for (const Slot &S : slots_) {
-    const DevBuf *all[] = {&S.si, &S.dbf, &S.residue, &S.side_trans, &S.recons_trans, &S.alpha, &S.lr, &S.oct,
-                           &S.smf, &S.pdf, &S.mb_mv, &S.fmv, &S.blk_mv, &S.blk_mv2, &S.holes, &S.mse, &S.stats,
-                           &S.in, &S.out};
-    for (const DevBuf *d : all) b += d->bytes;
-  }
+  for (const Slot &S : slots_)
+    for (const SlotBuf &d : slot_buffers(16, 16, 0, 0, 0)) b += (S.*d.buf).bytes;
   return b;
 }
 

@@ -57,6 +57,10 @@ struct Slot {
   void release();
 };
 
+// device bytes a batch holds for one frame with the given floats of noise pdf
+// (its references and output aside), at the widest speculation
+size_t frame_device_bytes(int w, int h, int q, size_t pdf_floats);
+
 // Kernel-level measurements, filled while Context-level profiling is on.
 struct ProfileStats {
   double ldpca_ms = 0;      // summed CUDA-event time of LDPCA ladder launches

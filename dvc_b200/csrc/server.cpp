@@ -77,11 +77,8 @@ size_t frame_bytes(int w, int h, int q, const int *ac_range) {
     const int ls = (dvc::kQTable[q][i] - 2) / 2;
     stride = std::max(stride, (size_t)(2 * ((ls + 1) * step - 1) + 1));
   }
-  const size_t slot = fs * 18 + n * 4 + (size_t)(w - 3) * (h - 3) * 32 + n * 81 * 4 + n * stride * 4 +
-                      fs / 256 * 48 * 2 + fs / 64 * 56 * 2 + (size_t)dvc::qbits_per_block(q) * (n / 8 + 24);
   const size_t refs = 2 * fs * 6 + fs;  // two references with low-pass and half-pel planes, output
-  const size_t spec = (size_t)32 * n;   // speculative ladder slots
-  return slot + refs + spec + (1 << 16);
+  return dvc::frame_device_bytes(w, h, q, n * stride) + refs + (1 << 16);
 }
 
 }  // namespace

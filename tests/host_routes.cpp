@@ -333,6 +333,29 @@ static void session(char **a) {
   dvc_destroy(c);
 }
 
+// server DATA TABLES w h q range count: the bytes a server charges for requests in
+// flight, and those its cohort of them holds on the device
+static void server(char **a) {
+  dvc_ctx *c = context(a[0], a[1]);
+  const int w = atoi(a[2]), h = atoi(a[3]), q = atoi(a[4]), count = atoi(a[6]);
+  dvc_server *s = nullptr;
+  printf("rc %d\n", dvc_server_create(c, (size_t)64 << 30, 1, count, &s));
+  const size_t before = g_live;
+  long long ticket, pending, in_flight;
+  size_t charged = 0;
+  int done = 0;
+  for (int i = 0; i < count; i++) {
+    Frame f(w, h, q);
+    for (int &r : f.range) r = atoi(a[5]);
+    printf("rc %d\n", dvc_server_submit(s, &f.f, &ticket));
+  }
+  printf("rc %d\n", dvc_server_poll(s, &done));
+  dvc_server_stats(s, &pending, &in_flight, &charged);
+  printf("in flight %lld charged %zu held %zu\n", in_flight, charged, g_live - before);
+  dvc_server_destroy(s);
+  dvc_destroy(c);
+}
+
 int main(int argc, char **argv) {
   const std::string mode = argc > 1 ? argv[1] : "";
   if (mode == "files" && argc == 5) files(argv + 2);
@@ -340,6 +363,7 @@ int main(int argc, char **argv) {
   else if (mode == "scarce" && argc == 8) scarce(argv + 2);
   else if (mode == "huge" && argc == 6) huge(argv + 2);
   else if (mode == "session" && argc == 7) session(argv + 2);
+  else if (mode == "server" && argc == 9) server(argv + 2);
   else return 2;
   printf("left bytes %zu streams %d events %d\n", g_live, g_streams, g_events);
   return 0;

@@ -120,3 +120,18 @@ def test_a_sessions_batches_share_their_streams(routes, frames, max_batch, strea
     assert [x for x in lines if x.startswith("rc")] == ["rc 0"] * 3, lines
     assert "streams %d" % (streams + side) in lines, lines
     assert lines[-1] == "left bytes 0 streams 0 events 0"
+
+
+@pytest.mark.parametrize("w,h", [(176, 144), (352, 288)])
+@pytest.mark.parametrize("q", [1, 4, 8])
+@pytest.mark.parametrize("range_,count", [(1, 1), (200, 1), (2000, 1), (200, 16)])
+def test_the_server_charges_what_a_request_holds(routes, w, h, q, range_, count):
+    """The budget is one on device memory: a request counts at least for the bytes
+    that are allocated for it, and beyond them for no more than the widest
+    speculation (32 slots of a codeword's bits), every step's job and 64 KB."""
+    lines = routes("server", SHIPPED, w, h, q, range_, count)
+    got = [x.split() for x in lines if x.startswith("in flight")][0]
+    flight, charged, held = int(got[2]), int(got[4]), int(got[6])
+    assert flight == count
+    more = 32 * (w * h // 16 + 4) + 63 * 112 + 65536 + 1024
+    assert held <= charged <= held + count * more, (charged, held)
