@@ -3,15 +3,18 @@
     python -m dvc_b200.autotune [--out tuning.json] [--streams 4] [--frames 33] [--runs 5] [--bench-workload]
 
 Five launch parameters are chosen by measurement on the device the tuner runs on:
-  - threads per CIF codeword block of the LDPCA ladder, 512 or 1024 (edges per
-    thread = 19,008 / threads: 38 or 19; columns per thread 13 or 7);
-  - threads per QCIF codeword block, 1024, 256 or 512 (edges per thread 5, 19
-    or 10; one, four or two codewords per SM);
+  - threads per CIF codeword block of the LDPCA ladder, 512 or 1024 (columns per
+    thread 13 or 7), where a codeword takes one block;
+  - threads per QCIF codeword block, 1024, 256 or 512 (columns per thread 2, 7 or
+    4; one, four or two codewords per SM), where a codeword takes one block;
   - the floor of the speculative ladder width: every codeword of a bitplane step
-    is decoded by max(floor, SMs / codewords in flight) blocks, each starting at
-    another code of the ladder (1 turns speculation off);
-  - threads per updateSI search block, 64, 128 or 256 (one block per WZ 4x4
-    block: 2 x 65 candidate columns, two adjacent ones per thread);
+    is tried by max(floor, 4 SMs / (codewords in flight * C)) slots, at most 32,
+    each starting at another code of the ladder; a slot is a block, or a cluster
+    of C = 2, 4 or 8 blocks while few codewords are in flight (1 turns
+    speculation off where there are many);
+  - threads per updateSI tile, 256 ("64", the name this default had when a block
+    took a single 4x4 block, and still has in saved files) or 512 (one thread
+    block per 16x16 tile, a warp per WZ 4x4 block of it: two in turn, or one);
   - threads per forward-search block, 128, 256 or 512 (one block per 16x16
     macroblock: 65 x 65 candidate positions over the threads).
 The search is coordinate-wise: starting from the library's defaults, each
@@ -37,7 +40,7 @@ import numpy as np
 ENV_THREADS, ENV_THREADS_QCIF, ENV_FLOOR = "DVC_LDPCA_THREADS", "DVC_LDPCA_THREADS_QCIF", "DVC_LDPCA_SPEC_FLOOR"
 ENV_SI, ENV_FME = "DVC_SI_THREADS", "DVC_FME_THREADS"
 KNOBS = [(ENV_THREADS, ("1024", "512")), (ENV_THREADS_QCIF, ("1024", "256", "512")),
-         (ENV_FLOOR, ("4", "1", "2", "8", "12", "16", "24", "32")), (ENV_SI, ("64", "128", "256")),
+         (ENV_FLOOR, ("4", "1", "2", "8", "12", "16", "24", "32")), (ENV_SI, ("64", "512")),  # every value but 512 is 256 threads
          (ENV_FME, ("256", "128", "512"))]
 ENV_ALL = tuple(k for k, _ in KNOBS)
 THREADS = ("1024", "512")

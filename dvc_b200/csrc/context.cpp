@@ -65,10 +65,10 @@ bool Context::init(const char *data, const char *tables, int dev) {
   const char *nt = getenv("DVC_LDPCA_THREADS");
   const char *ntq = getenv("DVC_LDPCA_THREADS_QCIF");
   set_ldpca_threads(nt ? atoi(nt) : 1024, ntq ? atoi(ntq) : 1024);
-  // the same for the motion searches: threads per updateSI and forward-search block
+  // the same for the motion searches: threads per updateSI tile and forward-search block
   const char *si = getenv("DVC_SI_THREADS");
   const char *fme = getenv("DVC_FME_THREADS");
-  set_me_shapes(si ? atoi(si) : 64, fme ? atoi(fme) : 256);
+  set_me_shapes(si ? atoi(si) : 256, fme ? atoi(fme) : 256);
 
   // library-exact math tables: load, or sweep the C library once and cache
   const std::string xpath = table_dir + "/xlm_tables.bin";

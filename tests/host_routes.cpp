@@ -356,6 +356,22 @@ static void server(char **a) {
   dvc_destroy(c);
 }
 
+// shapes DATA TABLES: a frame, and codewords of both lengths a block each
+static void shapes(char **a) {
+  dvc_ctx *c = context(a[0], a[1]);
+  Frame f(176, 144, 1);
+  g_record = true;
+  printf("rc %d\n", dvc_decode_wz_frames(c, 1, &f.f));
+  void *room = nullptr;  // no kernel reads it
+  cudaMalloc(&room, 1 << 16);
+  for (int n : {1584, 6336})
+    printf("rc %d\n", dvc_ldpca_decode_noalloc(c, n, 1, (float *)room, (uint8_t *)room, (uint8_t *)room, nullptr,
+                                               (int *)room, nullptr, 50, nullptr));
+  g_record = false;
+  cudaFree(room);
+  dvc_destroy(c);
+}
+
 int main(int argc, char **argv) {
   const std::string mode = argc > 1 ? argv[1] : "";
   if (mode == "files" && argc == 5) files(argv + 2);
@@ -364,6 +380,7 @@ int main(int argc, char **argv) {
   else if (mode == "huge" && argc == 6) huge(argv + 2);
   else if (mode == "session" && argc == 7) session(argv + 2);
   else if (mode == "server" && argc == 9) server(argv + 2);
+  else if (mode == "shapes" && argc == 4) shapes(argv + 2);
   else return 2;
   printf("left bytes %zu streams %d events %d\n", g_live, g_streams, g_events);
   return 0;

@@ -135,3 +135,21 @@ def test_the_server_charges_what_a_request_holds(routes, w, h, q, range_, count)
     assert flight == count
     more = 32 * (w * h // 16 + 4) + 63 * 112 + 65536 + 1024
     assert held <= charged <= held + count * more, (charged, held)
+
+
+def test_every_value_of_a_tuned_parameter_is_another_launch_shape(routes):
+    """The autotuner times each value of a thread count once: two that launch the
+    same kernels would be chosen between by noise, and the default setting is the
+    one a process without the variables runs."""
+    from dvc_b200 import autotune as at
+    unset = dict.fromkeys(at.ENV_ALL, "")
+
+    def shape(**env):
+        return tuple(x for x in routes("shapes", SHIPPED, env=dict(unset, **env)) if x.startswith("launch"))
+
+    plain = tuple(x for x in routes("shapes", SHIPPED) if x.startswith("launch"))
+    for name, values in at.KNOBS:
+        if name != at.ENV_FLOOR:
+            got = [shape(**{name: v}) for v in values]
+            assert len(set(got)) == len(values), name
+            assert got[0] == plain, name
