@@ -39,7 +39,7 @@ struct LadderDev {
 struct LdpcaJob {
   int active;            // 0: the block returns at once (frame not in this step)
   const float *lr;       // [n] p0/p1 per 4x4 block (condBitProb output)
-  const float *llr_in;   // [n] log(p0/p1) and [n] entropy terms (ld_bit_terms) of lr,
+  const float *llr_in;   // [n] log(p0/p1) and [n] entropy terms (ld_entropy_term) of lr,
   const float *term_in;  //     when the caller has them; null: computed from lr
   const uint8_t *acc;    // [n/8] accumulated syndrome bytes, MSB first
   int crc;               // CRC-8 of the source bitplane
@@ -48,7 +48,8 @@ struct LdpcaJob {
   float *entropy;        // conditional entropy bound (may be null)
   int use_given_entropy; // 1: take the bound from given_entropy instead of computing it
   float given_entropy;
-  float *llr_out;        // [n] log(p0/p1) written back (may alias lr), or null
+  float *llr_out;        // [n] log(p0/p1) written back, or null; lr itself only where one block decodes
+                         // the codeword (other slots still read the ratios)
   // optional fused putBitplaneToCoeff (bitplane.cpp:4-22)
   int *recons_trans;     // [w*h] quantisation indices, or null
   const uint8_t *mode;   // [w*h/64] block modes

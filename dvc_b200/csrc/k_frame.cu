@@ -1010,8 +1010,7 @@ __device__ __forceinline__ float interval_sum(const float *p, int lo, int hi) {
 // threads, so that the rows of one CIF frame (6336) spread over all SMs.
 // With a thread for both sums, four quads of each in flight, and blocks of 128
 // threads (50 of 148 SMs for a lone CIF frame) 20.7 us a step, now 18.2; sixteen
-// CIF frames 26.2 -> 20.5.  One QCIF frame 2.46 -> 2.40 ms, one CIF frame 5.40 ->
-// 5.31, eleven at QIndex 8 66.2 -> 65.6.
+// CIF frames 26.2 -> 20.5.
 __global__ void __launch_bounds__(64) cond_bit_kernel(FrameDev *frames, XlmDev xt, int band, int bit) {
   FrameDev &F = frames[blockIdx.y];
   if (!F.active || !in_step(F, band, bit)) return;
@@ -1447,8 +1446,7 @@ __device__ __forceinline__ uint32_t load4_u8(const uint8_t *a) {
 // flight; the probabilities stay in shared memory between the two parts.  As two
 // kernels of a warp a block and a thread a coefficient, with one load of a chain
 // in flight, 16.7 + 18.4 us a band for one CIF frame; now 22.7 (eight lanes a
-// block and a coefficient pair each: 28.7).  A lone CIF frame 5.52 -> 5.40 ms,
-// eleven at QIndex 8 67.2 -> 66.3, one QCIF frame 2.51 -> 2.48.
+// block and a coefficient pair each: 28.7).
 __global__ void __launch_bounds__(128) update_ml_kernel(FrameDev *frames, XlmDev xt, int band) {
   __shared__ float s_p[8][ML_N];  // ML_N is odd: the two blocks of a warp read two banks
   FrameDev &F = frames[blockIdx.y];

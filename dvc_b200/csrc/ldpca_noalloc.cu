@@ -10,7 +10,7 @@
 // The only scratch this decode needs beyond its inputs and outputs is the
 // array of per-codeword job descriptors the LDPCA kernel reads.  Here it lives
 // in a file-scope __device__ array of fixed size (kMaxCodewords descriptors,
-// about 100 KB), which every GPU that loads this library holds until the
+// 112 KB), which every GPU that loads this library holds until the
 // process exits.  Host code cannot use the array's name as a device address,
 // so the first call on each device looks the address up with
 // cudaGetSymbolAddress (with that device current) and keeps it; make that first
@@ -30,7 +30,8 @@
 
 namespace {
 
-constexpr int kMaxCodewords = DVC_NOALLOC_MAX_CODEWORDS;  // sizeof(LdpcaJob) is 96 bytes
+constexpr int kMaxCodewords = DVC_NOALLOC_MAX_CODEWORDS;
+static_assert(sizeof(dvc::LdpcaJob) * kMaxCodewords == 112 * 1024, "the size given above and in dvc_b200.h");
 constexpr int kMaxDevices = 64;
 
 static __device__ __align__(256) dvc::LdpcaJob g_jobs[kMaxCodewords];

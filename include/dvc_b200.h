@@ -41,9 +41,9 @@ typedef struct dvc_ctx dvc_ctx;
  * codeword block (default 1024), DVC_SI_THREADS = 256 or 512 threads per
  * updateSI tile (default 256, as for any other value) and DVC_FME_THREADS = 128, 256 or 512
  * per forward-search block (default 256), read here; DVC_LDPCA_SPEC_FLOOR = 1..32, the least number of
- * speculative blocks per codeword in a frame batch (default 4), and
- * DVC_LDPCA_SPEC = 1..32, a fixed number instead, both read when a batch is
- * prepared. */
+ * speculative slots per codeword (default 4), and DVC_LDPCA_SPEC = 1..32, a
+ * fixed number instead, both read when a batch of frames is prepared and by
+ * dvc_ldpca_decode and dvc_LdpcaDecoder. */
 int dvc_create(const char *data_dir, const char *table_dir, int device, dvc_ctx **out);
 
 /* Release everything the context owns.  Replaces LDPCA_CUDA_Free_Variable and
@@ -238,7 +238,7 @@ int dvc_ldpca_decode_batch(dvc_ctx *ctx, int count, const int *n, const float *l
  * and the call only enqueues work on `stream` (a cudaStream_t; NULL is the
  * legacy default stream), returning before the device is done.  The
  * per-codeword descriptors the kernel reads are kept in a fixed array in the
- * library's device memory (DVC_NOALLOC_MAX_CODEWORDS entries, about 100 KB,
+ * library's device memory (DVC_NOALLOC_MAX_CODEWORDS entries, 112 KB,
  * held on every GPU that loads the library until the process exits); more
  * codewords per call are rejected with DVC_E_ARG.  The first call on each
  * device sets that device up: it looks the array's address up, sets the LDPCA
