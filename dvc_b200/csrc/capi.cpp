@@ -532,7 +532,7 @@ struct dvc_session {
   std::vector<int> batch_stream;
   std::vector<cudaEvent_t> batch_done;
   std::vector<cudaStream_t> streams;
-  std::vector<dvc::SideStreams> side;          // of each stream, shared by its batches
+  std::vector<dvc::SideStreams> side;          // shared by batches that run one after another
   std::vector<std::vector<dvc::FrameResult>> results;
   cudaEvent_t t0 = nullptr, t1 = nullptr;
   std::vector<cudaEvent_t> done;
@@ -667,14 +667,6 @@ extern "C" int dvc_session_create(dvc_ctx *ctx, int count, const dvc_wz_frame *f
       return bail(st);
   }
   if ((st = cuda_status(c, cudaStreamSynchronize(s0), "session upload"))) return bail(st);
-  for (int k = 0; k < nstreams; k++) {
-    cudaStream_t sk;
-    if ((st = cuda_status(c, cudaStreamCreateWithFlags(&sk, cudaStreamNonBlocking), "stream"))) return bail(st);
-    S->streams.push_back(sk);
-    cudaEvent_t e;
-    if ((st = cuda_status(c, cudaEventCreate(&e), "event"))) return bail(st);
-    S->done.push_back(e);
-  }
   if ((st = cuda_status(c, cudaEventCreate(&S->t0), "event")) || (st = cuda_status(c, cudaEventCreate(&S->t1), "event")))
     return bail(st);
   // batches: level by level, frames of a level in the caller's order, at most
@@ -701,9 +693,36 @@ extern "C" int dvc_session_create(dvc_ctx *ctx, int count, const dvc_wz_frame *f
     }
   }
   const int nb = (int)S->batch_frames.size();
+  // streams without a batch are not made (a stream takes 60 to 400 us)
+  for (int k = 0; k < std::min(nstreams, nb); k++) {
+    cudaStream_t sk;
+    if ((st = cuda_status(c, cudaStreamCreateWithFlags(&sk, cudaStreamNonBlocking), "stream"))) return bail(st);
+    S->streams.push_back(sk);
+    cudaEvent_t e;
+    if ((st = cuda_status(c, cudaEventCreate(&e), "event"))) return bail(st);
+    S->done.push_back(e);
+  }
+  // The side streams of a batch are those of one it runs after, the last on its
+  // stream or one whose output it reads, if no other batch took them since; so
+  // there are no more sets than streams, and no batch waits for another's groups.
+  std::vector<int> last_user;  // of each set
+  std::vector<int> side_of(nb, -1);
+  for (int b = 0; b < nb; b++) {
+    const auto &deps = S->batch_deps[b];
+    for (int own = 1; own >= 0 && side_of[b] < 0; own--)
+      for (int k = 0; k < (int)last_user.size() && side_of[b] < 0; k++)
+        if (own ? S->batch_stream[last_user[k]] == S->batch_stream[b]
+                : std::find(deps.begin(), deps.end(), last_user[k]) != deps.end())
+          side_of[b] = k;
+    if (side_of[b] < 0) {
+      side_of[b] = (int)last_user.size();
+      last_user.push_back(b);
+    }
+    last_user[side_of[b]] = b;
+  }
   S->batches.resize(nb);
   S->results.resize(nb);
-  S->side.resize(nstreams);
+  S->side.resize(last_user.size());
   for (int b = 0; b < nb; b++) {
     cudaEvent_t e;
     if ((st = cuda_status(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event"))) return bail(st);
@@ -750,7 +769,7 @@ extern "C" int dvc_session_create(dvc_ctx *ctx, int count, const dvc_wz_frame *f
     cudaStream_t sb = S->streams[S->batch_stream[b]];
     // frames decoding at once: those of the batch's level, one batch per stream
     const int concurrent = std::min(level_frames[level[S->batch_frames[b][0]]], nstreams * max_batch);
-    S->batches[b].set_side_streams(&S->side[S->batch_stream[b]]);
+    S->batches[b].set_side_streams(&S->side[side_of[b]]);
     if (!S->batches[b].prepare(c, specs, sb, concurrent)) return bail(DVC_E_CUDA);
     if ((st = cuda_status(c, cudaStreamSynchronize(sb), "session prepare"))) return bail(st);
   }

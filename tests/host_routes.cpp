@@ -312,20 +312,26 @@ struct Frame {
   }
 };
 
-// session DATA TABLES frames max_batch streams: what a session of independent
-// QCIF frames holds, and two runs of it
+// session DATA TABLES sequences levels max_batch streams: what a session of QCIF
+// sequences holds, and two runs of it; a sequence is a GOP of 2^levels frames,
+// whose first level is the middle frame, the next those half way to its ends
 static void session(char **a) {
   dvc_ctx *c = context(a[0], a[1]);
-  const int count = atoi(a[2]), s0 = g_streams;
+  const int sequences = atoi(a[2]), levels = atoi(a[3]), gop = 1 << levels, count = sequences * (gop - 1);
+  const int s0 = g_streams;
   std::vector<Frame> frames;
   std::vector<dvc_wz_frame> list;
   frames.reserve(count);
+  for (int i = 0; i < count; i++) frames.emplace_back(176, 144, 1);
   for (int i = 0; i < count; i++) {
-    frames.emplace_back(176, 144, 1);
-    list.push_back(frames.back().f);
+    const int at = i % (gop - 1) + 1, half = at & -at;  // frame `at` lies between at - half and at + half
+    dvc_wz_frame f = frames[i].f;
+    if (at - half > 0) f.past = frames[i - half].recon.data();
+    if (at + half < gop) f.future = frames[i + half].recon.data();
+    list.push_back(f);
   }
   dvc_session *s = nullptr;
-  int rc = dvc_session_create(c, count, list.data(), atoi(a[3]), atoi(a[4]), &s);
+  int rc = dvc_session_create(c, count, list.data(), atoi(a[4]), atoi(a[5]), &s);
   printf("rc %d\nstreams %d\n", rc, g_streams - s0);
   double ms = 0;
   for (int run = 0; run < 2; run++) printf("rc %d\n", dvc_session_run(s, 0, &ms));
@@ -378,7 +384,7 @@ int main(int argc, char **argv) {
   else if (mode == "decode" && argc == 6) decode(argv + 2);
   else if (mode == "scarce" && argc == 8) scarce(argv + 2);
   else if (mode == "huge" && argc == 6) huge(argv + 2);
-  else if (mode == "session" && argc == 7) session(argv + 2);
+  else if (mode == "session" && argc == 8) session(argv + 2);
   else if (mode == "server" && argc == 9) server(argv + 2);
   else if (mode == "shapes" && argc == 4) shapes(argv + 2);
   else return 2;

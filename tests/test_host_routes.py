@@ -111,14 +111,16 @@ def test_a_count_that_no_device_holds_is_refused(routes, n, count):
     assert "rc -3" in routes("huge", SHIPPED, n, count)
 
 
-@pytest.mark.parametrize("frames,max_batch,streams,side", [
-    (64, 4, 2, 6), (40, 8, 4, 28), (9, 16, 1, 4), (33, 16, 4, 14), (66, 33, 2, 0)])
-def test_a_sessions_batches_share_their_streams(routes, frames, max_batch, streams, side):
-    """Batches on one of the session's streams run one after another: the streams
-    their groups decode on (up to seven) are the stream's, however many they are."""
-    lines = routes("session", SHIPPED, frames, max_batch, streams)
+@pytest.mark.parametrize("sequences,levels,max_batch,streams,own,side", [
+    (64, 1, 4, 2, 2, 6), (40, 1, 8, 4, 4, 28), (9, 1, 16, 1, 1, 4), (33, 1, 16, 4, 3, 14), (66, 1, 33, 2, 2, 0),
+    (6, 3, 16, 8, 4, 14),  # levels of 6, 12 and 16 + 8 frames: the first three batches follow one another
+    (6, 3, 16, 2, 2, 14), (6, 3, 4, 16, 11, 3 * 6), (1, 3, 16, 8, 3, 3)])
+def test_a_sessions_batches_share_their_streams(routes, sequences, levels, max_batch, streams, own, side):
+    """A session makes no stream that no batch is on, and a batch's groups (up to
+    eight) decode on the streams of one that it runs after where there is one."""
+    lines = routes("session", SHIPPED, sequences, levels, max_batch, streams)
     assert [x for x in lines if x.startswith("rc")] == ["rc 0"] * 3, lines
-    assert "streams %d" % (streams + side) in lines, lines
+    assert "streams %d" % (own + side) in lines, lines
     assert lines[-1] == "left bytes 0 streams 0 events 0"
 
 
