@@ -21,15 +21,17 @@ struct LadderDev {
   const int *synd_len;    // [num_codes]
   const float *code_rate; // [num_codes]
   // Rows of a code are decoded in slot order: sorted by degree, largest first
-  // (ties in row order), 32 slots to a group, one group to a warp.  The edge
-  // messages of group g are stored transposed: edge i (in increasing edge
-  // order) of the row in lane l at position base + i * width + l, width = the
-  // rows of the group (32 but for the last), so a warp reads its rows without
-  // bank conflicts.  Rows shorter than the group's first are padded.
+  // (ties in row order), up to 32 rows to a group, one group to a warp, the row in
+  // lane l of group g in slot 32 g + l.  The edge messages of a group are stored
+  // transposed: edge i (in increasing edge order) of the row in lane l at position
+  // base + i * width + l, width = the rows of the group, so a warp reads its rows
+  // without bank conflicts.  Rows shorter than the group's first are padded.
   int pos_max;               // positions of the largest code, padding included (multiple of 4)
+  int groups;                // groups of the code that has most
+  const int *ng;             // [num_codes] groups
   const uint32_t *edge;      // [num_codes*3*n] edge 3k + i of column k at [(3*code + i)*n + k]: position | slot << 16
-  const uint32_t *grp;       // [num_codes*ceil(n/32)] base | edges of its longest row << 16
-  const uint16_t *slot_row;  // [num_codes*n] row of each slot
+  const uint2 *grp;          // [num_codes*groups] base | edges of its longest row << 16, width
+  const uint16_t *slot_row;  // [num_codes*32*groups] row of each slot
   const uint16_t *ir_full;   // [e] row of edge e in the full-rate code (the encoder's matrix)
   const uint8_t *crc_tab;    // [n]
   const uint32_t *invh;      // [n*invh_words]
@@ -55,6 +57,8 @@ struct LdpcaJob {
   const uint8_t *mode;   // [w*h/64] block modes
   int w, index_in_blk;
 };
+
+#define LDPCA_MAX_N 6336  // longest codeword that decodes
 
 // codes below full rate that a codeword's iteration counts (LdpcaSpec,
 // LdpcaBatchState) and the queue's masks hold; the shipped ladders have 64

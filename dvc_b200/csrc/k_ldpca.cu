@@ -241,7 +241,7 @@ static cudaError_t launch_nt(const LadderDev &L, const LdpcaJob *jobs, int num_j
   const int rounds = LDPCA_COLS(L.n, NT * C);
   if (L.n > LDPCA_MAX_N || (ANY ? rounds > MAXC : rounds != MAXC)) return cudaErrorInvalidValue;
   auto kernel = ldpca_ladder_kernel<NT, MAXC, MINB, C, ANY>;
-  const size_t smem = ldpca_smem_bytes(L.n, L.pos_max);
+  const size_t smem = ldpca_smem_bytes(L);
   // the rest of the SM's 256 KB is L1 for the phi records, which BP iterations re-read
   static SmemLimit limit;
   const cudaError_t e = limit.raise(kernel, smem, MINB);

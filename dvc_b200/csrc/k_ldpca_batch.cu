@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(1024, 1) ldpca_batch_kernel(LdpcaBatch A) {
   {
     const int gi = threadIdx.x >> 8;
     const LdGroup<256, false> g{(int)threadIdx.x & 255, 1 + gi, 0};
-    const size_t quarter = ldpca_smem_bytes(A.L_qcif.n, A.L_qcif.pos_max);
+    const size_t quarter = ldpca_smem_bytes(A.L_qcif);
     const LdSmem S = ld_carve(smem + gi * quarter, A.L_qcif);
     for (;;) {
       if (g.t == 0) s_item[gi] = A.n_qcif ? pop_item(A, 1) : -1;
@@ -276,8 +276,8 @@ size_t ldpca_batch_state_bytes(int count) {
 
 // dynamic shared memory of a batch block: one CIF codeword, or four QCIF ones
 static size_t batch_smem_bytes(const LdpcaBatch &A) {
-  const size_t cif = ldpca_smem_bytes(A.L_cif.n, A.L_cif.pos_max);
-  const size_t qcif4 = 4 * ldpca_smem_bytes(A.L_qcif.n, A.L_qcif.pos_max);
+  const size_t cif = ldpca_smem_bytes(A.L_cif);
+  const size_t qcif4 = 4 * ldpca_smem_bytes(A.L_qcif);
   return cif > qcif4 ? cif : qcif4;
 }
 

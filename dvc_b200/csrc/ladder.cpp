@@ -89,12 +89,13 @@ bool load_ladders(const std::string &path, std::vector<LadderHost> &out, std::st
     }
     // expand the per-code rows: row of edge e in code c is the first kept
     // accumulated-syndrome position >= its full-rate row; then the BP layout
-    const int gmax = (L.n + 31) / 32;
     L.synd_len.resize(L.num_codes);
     L.code_rate.resize(L.num_codes);
+    L.ng.resize(L.num_codes);
     L.edge.assign((size_t)L.num_codes * L.e, 0u);
-    L.grp.assign((size_t)L.num_codes * gmax, 0u);
-    L.slot_row.assign((size_t)L.num_codes * L.n, 0);
+    L.groups = (L.n + 31) / 32;
+    std::vector<std::vector<uint2>> grp(L.num_codes);
+    std::vector<std::vector<uint16_t>> slot_row(L.num_codes);
     for (int c = 0; c < L.num_codes; c++) {
       const int b = L.bpp[c];
       const int m = (L.n / L.period) * b;
@@ -112,32 +113,51 @@ bool load_ladders(const std::string &path, std::vector<LadderHost> &out, std::st
         row[e] = r;
         deg[r]++;
       }
-      std::vector<int> order(m), slot(m), fill(m, 0);
+      std::vector<int> order(m), fill(m, 0), group(m), lane(m);
       for (int r = 0; r < m; r++) order[r] = r;
       std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return deg[x] > deg[y]; });
-      for (int s = 0; s < m; s++) {
-        slot[order[s]] = s;
-        L.slot_row[(size_t)c * L.n + s] = (uint16_t)order[s];
-      }
-      std::vector<int> base((m + 31) / 32);
+      // Groups of 32 rows.  A code whose rows differ so much in degree that the
+      // padding would exceed the edges (none of the shipped ones: 19,072
+      // positions for 19,008 edges) closes a group where the degree has halved,
+      // so that every code of a length that decodes fits its shared memory.
       int pos = 0;
-      for (int g = 0; g * 32 < m; g++) {
-        const int width = std::min(32, m - 32 * g), d = deg[order[32 * g]];
-        base[g] = pos;
-        L.grp[(size_t)c * gmax + g] = (uint32_t)pos | ((uint32_t)d << 16);
-        pos += width * d;
+      for (bool even : {false, true}) {
+        pos = 0;
+        grp[c].clear();
+        for (int r = 0, w; r < m; r += w) {
+          const int d = deg[order[r]];
+          for (w = 0; w < 32 && r + w < m && (!even || 2 * deg[order[r + w]] >= d); w++) {
+            group[order[r + w]] = (int)grp[c].size();
+            lane[order[r + w]] = w;
+          }
+          grp[c].push_back(make_uint2((uint32_t)pos | ((uint32_t)d << 16), (uint32_t)w));
+          pos += w * d;
+        }
+        if (pos <= 2 * L.e) break;
       }
-      if (pos > 65536 || m > 65536) {
+      L.ng[c] = (int)grp[c].size();
+      L.groups = std::max(L.groups, L.ng[c]);
+      if (L.n > LDPCA_MAX_N) continue;  // encodes only: no kernel decodes it
+      if (pos > 65536 || 32 * L.ng[c] > 65536) {
         fclose(f);
         err = "ladder code too large for 16-bit positions";
         return false;
       }
       L.pos_max = std::max(L.pos_max, (pos + 3) & ~3);
+      slot_row[c].assign((size_t)32 * L.ng[c], 0);
+      for (int r = 0; r < m; r++) slot_row[c][32 * group[r] + lane[r]] = (uint16_t)r;
       for (int e = 0; e < L.e; e++) {
-        const int r = row[e], s = slot[r], g = s >> 5, width = std::min(32, m - 32 * g);
-        const uint32_t p = (uint32_t)(base[g] + fill[r]++ * width + (s & 31));
-        L.edge[((size_t)c * 3 + e % 3) * L.n + e / 3] = p | ((uint32_t)s << 16);
+        const int r = row[e];
+        const uint2 place = grp[c][group[r]];
+        const uint32_t p = (place.x & 0xffffu) + (uint32_t)fill[r]++ * place.y + (uint32_t)lane[r];
+        L.edge[((size_t)c * 3 + e % 3) * L.n + e / 3] = p | ((uint32_t)(32 * group[r] + lane[r]) << 16);
       }
+    }
+    L.grp.assign((size_t)L.num_codes * L.groups, make_uint2(0, 0));
+    L.slot_row.assign((size_t)L.num_codes * 32 * L.groups, 0);
+    for (int c = 0; c < L.num_codes; c++) {
+      std::copy(grp[c].begin(), grp[c].end(), L.grp.begin() + (size_t)c * L.groups);
+      std::copy(slot_row[c].begin(), slot_row[c].end(), L.slot_row.begin() + (size_t)c * 32 * L.groups);
     }
     // CRC-8 is linear over GF(2) for a fixed message length (zero initial
     // value, no final xor), so the CRC of a bitplane is the xor of the CRCs
@@ -254,9 +274,10 @@ bool LadderGpu::upload(const LadderHost &L, std::string &err) {
   dev.num_codes = L.num_codes;
   dev.invh_words = L.invh_words;
   dev.pos_max = L.pos_max;
+  dev.groups = L.groups;
   return put(allocs, L.jc, &dev.jc, err) && put(allocs, L.bpp, &dev.bpp, err) && put(allocs, L.idx, &dev.idx, err) &&
          put(allocs, L.synd_len, &dev.synd_len, err) && put(allocs, L.code_rate, &dev.code_rate, err) &&
-         put(allocs, L.edge, &dev.edge, err) && put(allocs, L.grp, &dev.grp, err) &&
+         put(allocs, L.ng, &dev.ng, err) && put(allocs, L.edge, &dev.edge, err) && put(allocs, L.grp, &dev.grp, err) &&
          put(allocs, L.slot_row, &dev.slot_row, err) && put(allocs, L.ir_full16, &dev.ir_full, err) &&
          put(allocs, L.crc_tab, &dev.crc_tab, err) && put(allocs, L.invh, &dev.invh, err);
 }

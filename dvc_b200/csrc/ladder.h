@@ -12,11 +12,12 @@ namespace dvc {
 
 struct LadderHost {
   int n = 0, e = 0, period = 0, num_codes = 0, invh_words = 0;
-  int pos_max = 0;
-  std::vector<int> jc, bpp, idx, synd_len;
+  int pos_max = 0, groups = 0;
+  std::vector<int> jc, bpp, idx, synd_len, ng;
   std::vector<float> code_rate;
   // BP layout per code (dvc_types.h LadderDev)
-  std::vector<uint32_t> edge, grp;
+  std::vector<uint32_t> edge;
+  std::vector<uint2> grp;
   std::vector<uint16_t> slot_row;
   std::vector<uint8_t> crc_tab;
   std::vector<uint32_t> invh;

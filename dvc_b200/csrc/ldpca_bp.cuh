@@ -48,10 +48,10 @@
 // Shared memory per codeword (n bits, P = pos_max positions; CIF P = 19,072:
 // 102 KB; QCIF 27 KB):
 //   msg[P]    f32  edge messages
-//   rowt[n]   f32  row sums with the parity sign (after decoding: the decoded
-//                  bits, one byte each)
+//   rowt      f32  row sums by slot, with the parity sign (after decoding: the
+//                  decoded bits, one byte each)
 //   hdr       uint4 per row group: its place, the syndrome bits of its rows,
-//                  the rows whose check fails
+//                  the rows whose check fails, its width
 //   accs[n/8]      the packed accumulated syndrome, staged once per codeword
 #pragma once
 #include <cuda_runtime.h>
@@ -63,18 +63,15 @@ namespace dvc {
 
 #define LDPCA_LOG2 (0.693147181f)  // LdpcaDecoder.cpp:18
 #define LDPCA_NONE 0x7f7f7f7f      // "no success yet" (memset pattern 0x7f)
-#define LDPCA_MAX_N 6336           // largest codeword length
 
 // rounds (columns per thread) of a group of nt threads on codewords of n bits
 #define LDPCA_COLS(n, nt) (((n) + (nt) - 1) / (nt))
 
-__host__ __device__ inline int ldpca_groups(int n) { return (n + 31) / 32; }
-
-__host__ __device__ inline size_t ldpca_smem_bytes(int n, int pos_max) {
-  size_t b = (size_t)pos_max * 4;          // msg
-  b += (size_t)ldpca_groups(n) * 16;       // hdr
-  b += (size_t)n * 4;                      // rowt
-  b += (size_t)n / 8;                      // accs
+__host__ __device__ inline size_t ldpca_smem_bytes(const LadderDev &L) {
+  size_t b = (size_t)L.pos_max * 4;        // msg
+  b += (size_t)L.groups * 16;              // hdr
+  b += (size_t)L.groups * 32 * 4;          // rowt (n words or more: the full-rate code has n rows)
+  b += (size_t)L.n / 8;                    // accs
   return (b + 15) & ~(size_t)15;
 }
 
@@ -203,8 +200,8 @@ __device__ __forceinline__ LdSmem ld_carve(uint8_t *base, const LadderDev &L) {
   LdSmem S;
   S.msg = reinterpret_cast<float *>(base);
   S.hdr = reinterpret_cast<uint4 *>(S.msg + L.pos_max);  // pos_max is a multiple of 4
-  S.rowt = reinterpret_cast<float *>(S.hdr + ldpca_groups(L.n));
-  S.accs = reinterpret_cast<uint8_t *>(S.rowt + L.n);  // the codeword's packed accumulated syndrome
+  S.rowt = reinterpret_cast<float *>(S.hdr + L.groups);
+  S.accs = reinterpret_cast<uint8_t *>(S.rowt + 32 * L.groups);  // the codeword's packed accumulated syndrome
   S.dec = reinterpret_cast<uint8_t *>(S.rowt);       // decoded bits, once BP is over
   return S;
 }
@@ -431,7 +428,8 @@ __device__ __forceinline__ int ld_try_code(const G &g, const LadderDev &L, int c
   const int rank = C > 1 ? g.rank : 0;
   const bool lead = t == 0 && rank == 0;
   float *msg = S.msg, *rowt = S.rowt;
-  const int m = L.synd_len[code], ng = (m + 31) >> 5;
+  const uint2 *__restrict__ grp = L.grp + (size_t)code * L.groups;
+  const int ng = __ldg(L.ng + code);
   const uint32_t *__restrict__ edge = L.edge + (size_t)code * 3 * n;
   const uint32_t msg_a = (uint32_t)__cvta_generic_to_shared(msg);
   const uint32_t hdr_a = (uint32_t)__cvta_generic_to_shared(S.hdr);
@@ -454,14 +452,14 @@ __device__ __forceinline__ int ld_try_code(const G &g, const LadderDev &L, int c
   // padding positions add +0 to their row's sum, which leaves it unchanged
   for (int p = t; p < L.pos_max / 4; p += NT) reinterpret_cast<float4 *>(msg)[p] = make_float4(0.f, 0.f, 0.f, 0.f);
   {
-    const uint32_t *grp = L.grp + (size_t)code * ldpca_groups(n);
-    const uint16_t *srow = L.slot_row + (size_t)code * n;
+    const uint16_t *srow = L.slot_row + (size_t)code * 32 * L.groups;
     const int nb = L.bpp[code];
     const int *idx = L.idx + (size_t)code * L.period;
     for (int gr = rank + C * warp; gr < ng; gr += C * NW) {
-      const int s = 32 * gr + lane;
-      const uint32_t b = __ballot_sync(0xffffffffu, s < m && ld_synd_bit(L, idx, nb, S.accs, __ldg(srow + min(s, m - 1))));
-      if (lane == 0) S.hdr[gr] = make_uint4(__ldg(grp + gr), b, b, 0u);
+      const uint2 place = __ldg(grp + gr);
+      const uint32_t b = __ballot_sync(
+          0xffffffffu, lane < (int)place.y && ld_synd_bit(L, idx, nb, S.accs, __ldg(srow + 32 * gr + lane)));
+      if (lane == 0) S.hdr[gr] = make_uint4(place.x, b, b, place.y);
     }
   }
   if (t == 0) {
@@ -530,8 +528,8 @@ __device__ __forceinline__ int ld_try_code(const G &g, const LadderDev &L, int c
         }
         if (left & 1) add(p[0]);
       };
-      const int width = m - 32 * gr;
-      if (width >= 32)
+      const int width = (int)hd.w;
+      if (width == 32)
         row(32);
       else if (lane < width)
         row(width);

@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 #include <sys/resource.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -15,8 +16,13 @@
 #include <string>
 #include <vector>
 
+#include "context.h"
 #include "dvc_b200.h"
 #include "libm_tables.h"
+
+namespace dvc {
+Context *context_of(dvc_ctx *ctx);
+}
 
 // ------------------------------------------------------------ the runtime
 namespace {
@@ -378,6 +384,49 @@ static void shapes(char **a) {
   dvc_destroy(c);
 }
 
+// layout DATA TABLES: the BP layout of every code of a ladder file.  Every edge has
+// a position of its own inside its row's group, a row's edges follow one another
+// in edge order, and its slot names the row, found here from the file's data.
+static void layout(char **a) {
+  dvc_ctx *c = context(a[0], a[1]);
+  for (const dvc::LadderHost &L : dvc::context_of(c)->ladders_host) {
+    int bad = 0, most = 0;
+    for (int code = 0; code < L.num_codes; code++) {
+      const int b = L.bpp[code], m = L.synd_len[code];
+      std::vector<int> next(m, 0), used(L.pos_max, 0), rows(m, 0);
+      int positions = 0, held = 0;
+      for (int g = 0; g < L.ng[code]; g++) {
+        const uint2 p = L.grp[(size_t)code * L.groups + g];
+        bad += p.y < 1 || p.y > 32;
+        for (uint32_t l = 0; l < p.y; l++) rows[L.slot_row[((size_t)code * L.groups + g) * 32 + l]]++;
+        positions += (int)((p.x >> 16) * p.y);
+        held += (int)p.y;
+      }
+      for (int r = 0; r < m; r++) bad += rows[r] != 1;
+      bad += held != m || positions > L.pos_max;
+      most = std::max(most, positions);
+      for (int k = 0; k < L.n; k++)
+        for (int i = 0; i < 3; i++) {
+          int r = 0;  // the first kept position at or after the edge's full-rate row
+          const int at = L.ir_full[3 * k + i], q = at / L.period;
+          while (r < b && L.idx[(size_t)code * L.period + r] < at - q * L.period) r++;
+          r += q * b;
+          const uint32_t e = L.edge[((size_t)code * 3 + i) * L.n + k], p = e & 0xffffu, s = e >> 16;
+          if ((int)(s >> 5) >= L.ng[code] || (int)p >= L.pos_max) {
+            bad++;
+            continue;
+          }
+          const uint2 G = L.grp[(size_t)code * L.groups + (s >> 5)];
+          bad += (s & 31) >= G.y || L.slot_row[(size_t)code * L.groups * 32 + s] != r;
+          const int nth = next[r]++;
+          bad += p != (G.x & 0xffffu) + (uint32_t)nth * G.y + (s & 31) || nth >= (int)(G.x >> 16) || used[p]++;
+        }
+    }
+    printf("length %d codes %d positions %d groups %d bad %d\n", L.n, L.num_codes, most, L.groups, bad);
+  }
+  dvc_destroy(c);
+}
+
 int main(int argc, char **argv) {
   const std::string mode = argc > 1 ? argv[1] : "";
   if (mode == "files" && argc == 5) files(argv + 2);
@@ -387,6 +436,7 @@ int main(int argc, char **argv) {
   else if (mode == "session" && argc == 8) session(argv + 2);
   else if (mode == "server" && argc == 9) server(argv + 2);
   else if (mode == "shapes" && argc == 4) shapes(argv + 2);
+  else if (mode == "layout" && argc == 4) layout(argv + 2);
   else return 2;
   printf("left bytes %zu streams %d events %d\n", g_live, g_streams, g_events);
   return 0;

@@ -20,6 +20,17 @@ def circulant(n, period, bpp):
     return dict(N=n, E=3 * n, period=period, jc=3 * np.arange(n + 1), ir_full=ir, bpp=list(bpp), idx=idx)
 
 
+def merged(n):
+    """The circulant code with a period of its whole length, and codes that keep
+    the accumulated bits of one end only, all but one row in a hundred, and every
+    second: the first row of the first two gathers most or a part of the edges."""
+    ends = [np.arange(n * 3 // 5, n), np.r_[np.arange(0, n // 3, 100), np.arange(n // 3, n)], np.arange(n // 12, n),
+            np.arange(1, n, 2), np.arange(n)]
+    ends.sort(key=len)
+    L = circulant(n, 32, [32])
+    return dict(L, period=n, bpp=[len(i) for i in ends], idx=ends)
+
+
 def many_codes(num):
     """The shipped ladders with every code but the last repeated, `num` codes in all."""
     shipped = lad.read_compact(os.path.join(ROOT, "dvc_b200", "ladders", "ldpca_ladders.bin"))

@@ -85,3 +85,35 @@ def test_many_codes_match_the_oracle(context, num):
             assert np.array_equal(dec[i], odec) and np.array_equal(res[i], got[0][1][i])
         dec, rate, llr = ctx.LdpcaDecoder(lr[i], np.unpackbits(acc[i]), int(crc[i]), float(got[0][2][i]))
         assert rate == orate and np.array_equal(dec, odec)
+
+
+@pytest.mark.parametrize("n", [256, 1584, 6336])
+def test_rows_of_most_edges_match_the_oracle(context, n):
+    """Codes whose rows differ in degree by a thousand times (their groups of rows
+    are cut where the degree halves), in every form, entered at each code."""
+    from oracle import pyoracle as po
+    ladders = [lf.merged(m) for m in sorted({n, 1584, 6336})]
+    L = lf.lad.ladder_for(ladders, n)
+    ctx, o = context(ladders), lf.oracle(L)
+    lr, acc, crc, x = lf.codewords(L, 4, 7 * n)
+    # nearly every bit is sure, the others lean to the wrong side
+    doubt = np.random.default_rng(n).random(lr.shape) < [[0.0], [0.004], [0.02], [0.06]]
+    for_0 = np.where(doubt, np.float32(1 / 1.5), np.float32(3000))
+    lr = np.where(x == 0, for_0, 1 / for_0).astype(np.float32)
+    crc[3] ^= 0x5A
+    many = [np.repeat(a, 80, axis=0) for a in (lr, acc, crc)]
+    got = [ctx.ldpca_decode(lr, acc, crc), noalloc(ctx, lr, acc, crc), [a[::80] for a in ctx.ldpca_decode(*many)]]
+    accepted = set()
+    for i in range(4):
+        for start in range(5):
+            bound = np.float32(L["bpp"][start]) / np.float32(n)
+            odec, orate, ostart, oacc, _ = po.ldpca_decode(o, lr[i], np.unpackbits(acc[i]), int(crc[i]), float(bound))
+            dec, rate, llr = ctx.LdpcaDecoder(lr[i], np.unpackbits(acc[i]), int(crc[i]), float(bound))
+            assert rate == orate and np.array_equal(dec, odec), (i, start)
+            accepted.add(oacc)
+        odec, orate, ostart, oacc, _ = po.ldpca_decode(o, lr[i], np.unpackbits(acc[i]), int(crc[i]),
+                                                       po.compute_ce(lr[i]))
+        for dec, res, ent in got:
+            assert (res[i, 0], res[i, 1], res[i, 2]) == (orate, ostart, oacc)
+            assert np.array_equal(dec[i], odec) and np.array_equal(res[i], got[0][1][i])
+    assert len(accepted) >= 3, accepted  # codes with such rows decode, too

@@ -7,7 +7,7 @@ import subprocess
 
 import pytest
 
-from ladder_files import circulant, data_dir, lad, many_codes
+from ladder_files import circulant, data_dir, lad, many_codes, merged
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CUDA = "/usr/local/cuda"
@@ -155,3 +155,20 @@ def test_every_value_of_a_tuned_parameter_is_another_launch_shape(routes):
             got = [shape(**{name: v}) for v in values]
             assert len(set(got)) == len(values), name
             assert got[0] == plain, name
+
+
+@pytest.mark.parametrize("which", ["shipped", "129 codes", "a row of most edges"])
+def test_layout_of_every_code(routes, which):
+    """... of rows of any degrees: a code keeps within twice its edges' positions
+    (the shipped ones within a hundredth more than the edges), and a launch of any
+    form holds it."""
+    d = {"shipped": lambda: SHIPPED, "129 codes": lambda: data_dir(routes.tmp / "c129", many_codes(129)),
+         "a row of most edges": lambda: data_dir(routes.tmp / "merged", [merged(n) for n in (256, 1600, 6336)])}[which]()
+    seen = [x.split() for x in routes("layout", d) if x.startswith("length")]
+    assert seen and all(x[-1] == "0" for x in seen), seen
+    for x in seen:
+        n, positions = int(x[1]), int(x[5])
+        assert positions <= (2 if which[0] == "a" else 1.12) * 3 * n
+        for count in (1, 100, 700):
+            lines = routes("decode", d, n, count)
+            assert "rc 0" in lines and not any("refused" in t for t in lines), lines
