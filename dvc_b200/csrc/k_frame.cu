@@ -1155,8 +1155,8 @@ __device__ __forceinline__ uint32_t sad4_acc(uint32_t a, uint32_t b, uint32_t c)
 //
 // One thread block takes a 16x16 tile of a frame, whose (up to) 16 WZ blocks
 // search nearly the same 80x80 pixels of either reference; a warp takes a
-// block.  What bounds it is instruction issue, so candidates are ruled out
-// eight to a lane and step before their SADs are formed: the tile's window holds,
+// block.  Forming every SAD is bound by instruction issue, so candidates are ruled
+// out eight to a lane and step before their SADs are formed: the tile's window holds,
 // for every position, the floored means of the four 2x2 quadrants of the 4x4
 // block there, one word.  With d the sum of the four mean differences (one
 // packed instruction), SAD >= 4 d - 12; the weight of a candidate is at least
@@ -1166,6 +1166,9 @@ __device__ __forceinline__ uint32_t sad4_acc(uint32_t a, uint32_t b, uint32_t c)
 // previous band's best.  Those left are queued per warp (by groups of eight
 // columns) and weighed 32 at a time; the (cost, index) order makes the result
 // independent of the order in which candidates are weighed.
+// What bounds it now is shared memory: with many tiles in flight (65 QCIF frames)
+// L1 runs at 88% of its peak and 58% of the issue slots are used; a lone CIF
+// frame's 396 tiles are 0.9 of a wave and take as long as the last of them.
 // All SADs of a block by packed instructions took 93 us for a band of two CIF
 // frames (40 M warp instructions a frame) and 70 us for a lone one; so 72 and 43
 // us (20 M) with 256 threads, two blocks to a warp and three thread blocks an
